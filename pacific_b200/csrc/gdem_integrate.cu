@@ -49,6 +49,9 @@ namespace {
 
 __device__ __forceinline__ bool gatedOff(const int* gate) { return gate && !*gate; }
 
+// Most rounds of 32 pairs a warp of the contact filter takes per append.
+constexpr int kFilterRounds = 8;
+
 __global__ void k_decide(DevState S, cudaGraphConditionalHandle h, int use_handle) {
   if (threadIdx.x != 0 || blockIdx.x != 0) return;
   const int need = S.ctl[kCtlNeed];
@@ -56,6 +59,9 @@ __global__ void k_decide(DevState S, cudaGraphConditionalHandle h, int use_handl
   S.ctl[kCtlNeed] = 0;
   S.ctl[kCtlEpoch] += 1;
   S.ctl[kCtlWork] = 0;
+  // the filter's rounds per append, from the last evaluation's kept pairs
+  const long long kept = (long long)S.ctl[kCtlKept] + S.ctl[kCtlKeptCold];
+  S.ctl[kCtlRounds] = 8 * kept > S.ctl[kCtlPairs] ? kFilterRounds : 1;
   S.ctl[kCtlKept] = 0;
   S.ctl[kCtlKeptCold] = 0;
   S.ctl[kCtlKept2] = 0;
@@ -452,16 +458,16 @@ __global__ void __launch_bounds__(kMoveBlock<kFast, kBasis>(), (kFast && kBasis)
 // contacts; the kept pairs are listed for the pair kernel, which decides each
 // exactly, and both partners marked as candidates.  With walls, the first
 // pblocks blocks take one particle per thread and list (and mark) those near
-// a wall.  The pairs are taken in chunks of kFilterUnroll rounds of 32 per
-// warp with their loads issued together, in a grid-stride loop over chunks
-// (the count is known on the device only) on a grid of one block per 2,048
-// pairs at the leapfrog start (kFilterPairsPerBlock; the host resizes it
-// then).  Measured at 1M spheres: one round per chunk and that grid take
-// 21.3 us, four rounds on a grid of one block per 1,024 pairs 27.0 us (the
-// kernel is bound by the latency of its gathers: fewer registers, more warps).
-constexpr int kFilterUnroll = 1;
-constexpr int kFilterPairsPerBlock = 2048;
-
+// a wall.  A warp tests `rounds` rounds of 32 pairs, then appends all it kept
+// with one atomic: where the last evaluation kept more than an eighth of the
+// pairs (a packed bed, colliding convex bodies) up to kFilterRounds of them,
+// else one, whose append then overlaps the other warps' loads.  A grid-stride
+// loop covers any count (known on the device only).
+// What bounds it: in a gas (few pairs kept) the latency of the position
+// gathers (1M spheres: 20.9 us with 1 round, 23.1 with 8); in a bed the marks
+// and the appends, which were two atomics per kept pair and one per 32 pairs
+// on a single counter (250,000 packed spheres, 737,000 pairs kept: 32.9 us
+// then, 31.3 with plain marks and 1 round, 22.5 with 8 rounds).
 // Appends idx to list (length *count) for every lane whose pred holds (one
 // atomic per warp); every lane of the warp calls it.
 __device__ __forceinline__ void appendList(int* list, int* count, bool pred, int idx) {
@@ -474,17 +480,41 @@ __device__ __forceinline__ void appendList(int* list, int* count, bool pred, int
   if (pred) list[base + __popc(m & ((1u << lane) - 1u))] = idx;
 }
 
-// Appends idx below list[0] (list[-1], list[-2], ...: a list growing
-// downwards from its last slot), for every lane whose pred holds; every lane
-// of the warp calls it.
-__device__ __forceinline__ void appendListBack(int* list, int* count, bool pred, int idx) {
-  const unsigned m = __ballot_sync(0xffffffffu, pred);
-  if (!m) return;
+// Appends the kept pairs of a warp's rounds to a list that grows upwards
+// (dir 1) or downwards (dir -1) from list[0] and marks their partners: lane j
+// holds the ballot of round j in mine (0 beyond the rounds), round j's pairs
+// are first + step j + lane.  The flag words are clear (the last leapfrog
+// kernel left them so) and only this kernel writes them until the pair kernel
+// starts, always this value: a plain store marks a candidate whoever else
+// does.  Every lane of the warp calls it.
+__device__ __forceinline__ void appendRounds(DevState const& S, int* flags, int* list, int dir,
+                                             int* count, unsigned mine, int first, int step) {
+  const unsigned full = 0xffffffffu;
   const int lane = threadIdx.x & 31;
+  const int c = __popc(mine);
+  const int total = __reduce_add_sync(full, c);
+  if (!total) return;
+  int incl = c;
+#pragma unroll
+  for (int o = 1; o < kFilterRounds; o <<= 1) {
+    const int y = __shfl_up_sync(full, incl, o);
+    if (lane >= o) incl += y;
+  }
   int base = 0;
-  if (lane == 0) base = atomicAdd(count, __popc(m));
-  base = __shfl_sync(0xffffffffu, base, 0);
-  if (pred) list[-(base + __popc(m & ((1u << lane) - 1u)))] = idx;
+  if (lane == 0) base = atomicAdd(count, total);
+  base = __shfl_sync(full, base, 0);
+  for (unsigned some = __ballot_sync(full, c != 0); some; some &= some - 1u) {
+    const int j = __ffs(some) - 1;
+    const unsigned m = __shfl_sync(full, mine, j);
+    const int at = base + __shfl_sync(full, incl - c, j) + __popc(m & ((1u << lane) - 1u));
+    if (m >> lane & 1u) {
+      const int i = first + step * j + lane;
+      const int2 pr = S.upairs[i];
+      list[(long long)dir * at] = i;
+      flags[pr.x] = (int)kCandidate;
+      flags[(unsigned)pr.y & ((1u << 27) - 1u)] = (int)kCandidate;
+    }
+  }
 }
 
 // Whether particle t (posf: its FP32 continuous position) comes within the
@@ -515,47 +545,38 @@ __device__ __forceinline__ bool nearWall(DevState const& S, int t) {
   return false;
 }
 
-__global__ void __launch_bounds__(256) k_filter(DevState S, int pblocks) {
+// kSplit: FP32-split with non-spherical classes (the kept pairs in two lists).
+template <bool kSplit>
+__global__ void __launch_bounds__(256, 8) k_filter(DevState S, int pblocks) {
   pdlTrigger();   // the pair kernel may be scheduled; it waits for this one
   const int lane = threadIdx.x & 31;
-  unsigned* flags = reinterpret_cast<unsigned*>(contactFlags(S));
+  int* flags = contactFlags(S);
   if ((int)blockIdx.x < pblocks) {
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     const bool near = t < S.n && nearWall(S, t);
-    if (near) atomicOr(&flags[t], kCandidate);
+    if (near) flags[t] = (int)kCandidate;
     appendList(S.work, S.ctl + kCtlWork, near, t);
     return;
   }
   const int np = S.ctl[kCtlPairs];
-  constexpr int chunk = 32 * kFilterUnroll;
   const long long wq = ((long long)((int)blockIdx.x - pblocks) * blockDim.x + threadIdx.x) >> 5;
   const long long nwq = ((long long)(gridDim.x - pblocks) * blockDim.x) >> 5;
-  for (long long c0l = wq * chunk; c0l < np; c0l += nwq * chunk) {   // warp-uniform
-    const int c0 = (int)c0l;
-    int2 pr[kFilterUnroll];
-    float4 pa[kFilterUnroll], pb[kFilterUnroll];
-#pragma unroll
-    for (int j = 0; j < kFilterUnroll; ++j) {
-      const int i = c0 + 32 * j + lane;
-      pr[j] = i < np ? S.upairs[i] : make_int2(0, 0);
-    }
-#pragma unroll
-    for (int j = 0; j < kFilterUnroll; ++j) {
-      pa[j] = pb[j] = make_float4(0.f, 0.f, 0.f, 0.f);
-      if (c0 + 32 * j + lane < np) {
-        pa[j] = S.posf[pr[j].x];
-        pb[j] = S.posf[(unsigned)pr[j].y & ((1u << 27) - 1u)];
-      }
-    }
-#pragma unroll
-    for (int j = 0; j < kFilterUnroll; ++j) {
-      const int t = pr[j].x, u = (int)((unsigned)pr[j].y & ((1u << 27) - 1u));
-      bool keep = false;
-      if (c0 + 32 * j + lane < np) {
+  // (all warp-uniform) round j of a warp is the grid's j-th sweep over the list
+  const long long sweep = 32 * nwq;
+  const int rounds = (int)min((long long)S.ctl[kCtlRounds], (np + sweep - 1) / sweep);
+  for (long long c0 = 32 * wq; c0 < np; c0 += sweep * rounds) {
+    unsigned mine = 0, mine_cold = 0;
+    for (int j = 0; j < rounds; ++j) {
+      const long long c = c0 + sweep * j + lane;
+      bool keep = false, hot = false;
+      if (c < np) {
+        const int2 pr = S.upairs[c];
+        const int t = pr.x, u = (int)((unsigned)pr.y & ((1u << 27) - 1u));
+        const float4 pa = S.posf[t], pb = S.posf[u];
         // the largest margin of the instances (a superset of the contacts);
         // the period only for an entry with an image shift (code 13 is
         // none), which needs the instance's grid
-        const unsigned code = (unsigned)pr[j].y >> 27;
+        const unsigned code = (unsigned)pr.y >> 27;
         float sx = 0.f, sy = 0.f, sz = 0.f;
         if (code != 13u) {
           GridDesc const& bg = S.bgrids[S.inst[t]];
@@ -563,39 +584,40 @@ __global__ void __launch_bounds__(256) k_filter(DevState S, int pblocks) {
           sy = (float)((int)((code / 3u) % 3u) - 1) * bg.Lf[1];
           sz = (float)((int)(code / 9u) - 1) * bg.Lf[2];
         }
-        const float dx = (pb[j].x - pa[j].x) + sx;
-        const float dy = (pb[j].y - pa[j].y) + sy;
-        const float dz = (pb[j].z - pa[j].z) + sz;
-        const float R = pa[j].w + pb[j].w + S.filt_margin_max;
+        const float dx = (pb.x - pa.x) + sx;
+        const float dy = (pb.y - pa.y) + sy;
+        const float dz = (pb.z - pa.z) + sz;
+        const float R = pa.w + pb.w + S.filt_margin_max;
         keep = dx * dx + dy * dy + dz * dz <= R * R;
-      }
-      if (keep) {
-        atomicOr(&flags[t], kCandidate);
-        atomicOr(&flags[u], kCandidate);
-      }
-      if (S.any_convex && !S.pos64) {
-        // FP32-split with non-spherical classes: a pair in contact at the
-        // last evaluation (its share on t's side carries that evaluation's
-        // tag) goes to the front of the list, the others to the back, so the
-        // pair kernel runs the full closest-point searches and laws of the
-        // likely contacts in warps of their own and the searches that stop
-        // early in others (measured: 3 % off the convex pour's FP32-split
-        // step; the FP64 step, whose searches all run to their end, was 1 %
-        // slower with it).  A guess that a rebuild made stale only reorders.
-        bool hot = false;
-        if (keep) {
-          const int c = c0 + 32 * j + lane;
-          const long long e = (long long)S.pair_off[t] + (S.epos[c] & 0xFFFF);
-          hot = __float_as_int(static_cast<const float4*>(S.share)[2 * e].w) ==
-                S.ctl[kCtlEpoch] - 1;
+        if constexpr (kSplit) {
+          // a pair in contact at the last evaluation (its share on t's side
+          // carries that evaluation's tag) goes to the front of the list, the
+          // others to the back, so the pair kernel runs the full
+          // closest-point searches and laws of the likely contacts in warps
+          // of their own and the searches that stop early in others
+          // (measured: 3 % off the convex pour's FP32-split step; the FP64
+          // step, whose searches all run to their end, was 1 % slower with
+          // it).  A guess that a rebuild made stale only reorders.
+          if (keep) {
+            const long long e = (long long)S.pair_off[t] + (S.epos[c] & 0xFFFF);
+            hot = __float_as_int(static_cast<const float4*>(S.share)[2 * e].w) ==
+                  S.ctl[kCtlEpoch] - 1;
+          }
+        } else {
+          hot = keep;
         }
-        appendList(S.kept, S.ctl + kCtlKept, keep && hot, c0 + 32 * j + lane);
-        appendListBack(S.kept + (S.pair_cap / 2), S.ctl + kCtlKeptCold, keep && !hot,
-                       c0 + 32 * j + lane);
-      } else {
-        appendList(S.kept, S.ctl + kCtlKept, keep, c0 + 32 * j + lane);
+      }
+      const unsigned mh = __ballot_sync(0xffffffffu, hot);
+      if (lane == j) mine = mh;
+      if constexpr (kSplit) {
+        const unsigned mc = __ballot_sync(0xffffffffu, keep && !hot);
+        if (lane == j) mine_cold = mc;
       }
     }
+    appendRounds(S, flags, S.kept, 1, S.ctl + kCtlKept, mine, (int)c0, (int)sweep);
+    if constexpr (kSplit)
+      appendRounds(S, flags, S.kept + (S.pair_cap / 2), -1, S.ctl + kCtlKeptCold, mine_cold,
+                   (int)c0, (int)sweep);
   }
 }
 
@@ -923,14 +945,17 @@ void launch_row_scan(DevState const& S, const int* gate, cudaStream_t st) {
   k_scan_sums<<<1, kScanTile, 0, st>>>(S.pair_scan_tmp, ntiles, gate);
   k_scan_add<<<ntiles, kScanTile, 0, st>>>(S.pair_off, S.pair_scan_tmp, S.npairs, S.n, gate, S.ctl);
 }
+int filterBlocks(long long pairs, int nsm) {
+  const long long full = (pairs + 2047) / 2048, one = (pairs + 255) / 256;
+  return (int)std::max(1ll, std::max(full, std::min(one, 4ll * nsm)));
+}
 void launch_filter(DevState const& S, cudaStream_t st) {
   if (!S.n) return;
   const int pblocks = S.any_walls ? blocks(S.n, 256) : 0;
   // about 4 pairs per particle until the leapfrog start has counted them
-  const int qblocks = S.filter_qblocks > 0
-                          ? S.filter_qblocks
-                          : (4 * S.n + kFilterPairsPerBlock - 1) / kFilterPairsPerBlock;
-  k_filter<<<pblocks + qblocks, 256, 0, st>>>(S, pblocks);
+  const int qblocks = S.filter_qblocks > 0 ? S.filter_qblocks : filterBlocks(4ll * S.n, S.nsm);
+  if (S.any_convex && !S.pos64) k_filter<true><<<pblocks + qblocks, 256, 0, st>>>(S, pblocks);
+  else k_filter<false><<<pblocks + qblocks, 256, 0, st>>>(S, pblocks);
 }
 void launch_link(DevState const& S, const int* gate, cudaStream_t st) {
   if (S.n) k_link<<<4 * S.nsm, 256, 0, st>>>(S, gate);

@@ -55,6 +55,11 @@ void launch_scan(DevState const& S, const int* gate, cudaStream_t st);
 // exclusive scan of the row lengths into pair_off (total into kCtlEntries)
 void launch_row_scan(DevState const& S, const int* gate, cudaStream_t st);
 void launch_filter(DevState const& S, cudaStream_t st);
+// Blocks of the contact filter for a number of pairs: eight rounds of 32
+// pairs per warp (2,048 pairs per block), fewer while that leaves the chip
+// without four blocks per multiprocessor (a small system's pairs are then
+// tested in one round each).
+int filterBlocks(long long pairs, int nsm);
 void launch_link(DevState const& S, const int* gate, cudaStream_t st);
 void launch_diag_prefill(DevState const& S, cudaStream_t st);
 void launch_place(DevState const& S, const int* gate, cudaStream_t st);

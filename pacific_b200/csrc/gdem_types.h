@@ -38,6 +38,7 @@ enum CtlWords : int {
   kCtlEntriesMax = 8,  // most entries any rebuild needed since the last allocation check
   kCtlKeptCold = 9,  // kept pairs not in contact at the last evaluation (listed from the back)
   kCtlKept2 = 10,    // of those, the pairs the first search iteration left undecided (kept2)
+  kCtlRounds = 11,   // rounds of 32 pairs per append of this evaluation's contact filter
   kCtlWords = 16
 };
 
