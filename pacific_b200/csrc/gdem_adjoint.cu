@@ -15,11 +15,9 @@
 // Loss: L = sum_i |x_i(N) - x*_i|^2 + |v_i(N) - v*_i|^2.
 //
 // Reverse sweep: the transposed leapfrog per particle, and per contact the
-// transposed Jacobian of Phi applied to the adjoints of its outputs.  Each
-// Jacobian column is one evaluation of the contact law on Dual<1> numbers
-// seeded on that input (its own position, half-step velocities, the
-// tangential history and, once per contact, kn, en, muc).  States are
-// recomputed from checkpoints taken every K steps.  A forward run on
+// transposed Jacobian of Phi applied to the adjoints of its outputs, by the
+// chain rule through the law in reverse order (gdem_adjoint_vjp.cuh).  States
+// are recomputed from checkpoints taken every K steps.  A forward run on
 // Dual<3> numbers seeded on (kn, en, muc) gives the forward-mode gradient
 // that checks the parameter part of the adjoint.
 //
@@ -45,7 +43,7 @@
 #include <vector>
 
 #include "../../include/grains_b200.h"
-#include "gdem_adjoint_law.cuh"
+#include "gdem_adjoint_vjp.cuh"
 #include "gdem_setup.h"
 
 namespace gdem {
@@ -53,6 +51,12 @@ namespace {
 
 constexpr int kAdjCap = 32;      // contacts per particle
 constexpr int kAdjWalls = 8;     // walls
+// Lanes that share one particle's contacts.  A step of a calibration box is
+// the latency of one particle's serial work (4,096 particles are one warp per
+// multiprocessor): its cells, its contacts and its walls each go one to a
+// lane.  8 lanes cover the walls and most particles' contacts in one pass.
+constexpr int kAdjLanes = 8;
+constexpr int kAdjBlock = 128;
 
 struct AdjCheck : std::runtime_error {
   using std::runtime_error::runtime_error;
@@ -194,29 +198,39 @@ __device__ __forceinline__ int adjCellIndex(AdjGrid const& g, int d, double x) {
 }
 
 template <typename T>
-__global__ void k_adj_bin(int n, AdjGrid g, const T* x, int* cell, int* count) {
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= n) return;
-  const int i = adjCellIndex(g, 0, val(x[3 * t]));
-  const int j = adjCellIndex(g, 1, val(x[3 * t + 1]));
-  const int k = adjCellIndex(g, 2, val(x[3 * t + 2]));
+__device__ __forceinline__ void adjBin(AdjGrid const& g, int t, V3<T> x, int* cell, int* count) {
+  const int i = adjCellIndex(g, 0, val(x.x)), j = adjCellIndex(g, 1, val(x.y)),
+            k = adjCellIndex(g, 2, val(x.z));
   const int c = (k * g.nb[1] + j) * g.nb[0] + i;
   cell[t] = c;
   atomicAdd(&count[c], 1);
 }
 
-// Exclusive scan of the cell counts by one block of 1024 threads, chunk by
-// chunk; start[ncells] receives the total.
-__global__ void __launch_bounds__(1024) k_adj_scan(int ncells, const int* count, int* start) {
+template <typename T>
+__global__ void k_adj_bin(int n, AdjGrid g, const T* x, int* cell, int* count) {
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t < n) adjBin(g, t, ldv(x, t), cell, count);
+}
+
+// Exclusive scan of the cell counts by one block of 1024 threads, 4,096
+// cells at a time (a calibration box has about that many, so one pass);
+// start[ncells] receives the total, cursor a copy of the starts (k_adj_place
+// counts it up), and the counts are cleared for the next evaluation.
+__global__ void __launch_bounds__(1024) k_adj_scan(int ncells, int* count, int* start,
+                                                   int* cursor) {
+  constexpr int kPer = 4;
   __shared__ int warp_sum[32];
-  __shared__ int carry_s;
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  if (threadIdx.x == 0) carry_s = 0;
-  __syncthreads();
-  for (int base = 0; base < ncells; base += 1024) {
-    const int i = base + threadIdx.x;
-    const int v = i < ncells ? count[i] : 0;
-    int x = v;
+  int carry = 0;
+  for (int base = 0; base < ncells; base += 1024 * kPer) {
+    const int i0 = base + kPer * threadIdx.x;
+    int v[kPer], sum = 0;
+#pragma unroll
+    for (int j = 0; j < kPer; ++j) {
+      v[j] = i0 + j < ncells ? count[i0 + j] : 0;
+      sum += v[j];
+    }
+    int x = sum;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
       const int y = __shfl_up_sync(0xffffffffu, x, o);
@@ -234,150 +248,251 @@ __global__ void __launch_bounds__(1024) k_adj_scan(int ncells, const int* count,
       warp_sum[lane] = y;
     }
     __syncthreads();
-    const int carry = carry_s;
-    const int before = wid > 0 ? warp_sum[wid - 1] : 0;
-    if (i < ncells) start[i] = carry + before + x - v;
-    __syncthreads();
-    if (threadIdx.x == 0) carry_s = carry + warp_sum[31];
+    int at = carry + (wid > 0 ? warp_sum[wid - 1] : 0) + x - sum;
+#pragma unroll
+    for (int j = 0; j < kPer; ++j) {
+      if (i0 + j < ncells) {
+        start[i0 + j] = at;
+        cursor[i0 + j] = at;
+        count[i0 + j] = 0;
+      }
+      at += v[j];
+    }
+    carry += warp_sum[31];
     __syncthreads();
   }
-  if (threadIdx.x == 0) start[ncells] = carry_s;
+  if (threadIdx.x == 0) start[ncells] = carry;
 }
 
-__global__ void k_adj_place(int n, const int* cell, const int* start, int* fill, int* items) {
+__global__ void k_adj_place(int n, const int* cell, int* cursor, int* items) {
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= n) return;
-  const int c = cell[t];
-  items[start[c] + atomicAdd(&fill[c], 1)] = t;
+  if (t < n) items[atomicAdd(&cursor[cell[t]], 1)] = t;
+}
+
+// The value of v on lane src of the particle's lanes.
+__device__ __forceinline__ double laneOf(unsigned mask, double v, int src) {
+  return __shfl_sync(mask, v, src, kAdjLanes);
+}
+template <int N>
+__device__ __forceinline__ Dual<N> laneOf(unsigned mask, Dual<N> v, int src) {
+  v.v = laneOf(mask, v.v, src);
+#pragma unroll
+  for (int k = 0; k < N; ++k) v.d[k] = laneOf(mask, v.d[k], src);
+  return v;
+}
+template <typename T>
+__device__ __forceinline__ V3<T> laneOf(unsigned mask, V3<T> v, int src) {
+  return v3(laneOf(mask, v.x, src), laneOf(mask, v.y, src), laneOf(mask, v.z, src));
 }
 
 // ------------------------------------------------------------- forward --
 // Contact forces and the new contact lists at one step.  vel/omg are the
 // velocities the law sees (half-step ones, or the initial ones at the
 // leapfrog start).  zero_spring: the leapfrog start zeroes the cumulative
-// spring after the evaluation.
+// spring after the evaluation.  kAdjLanes lanes per particle: the 27 cells,
+// then the contacts, then the walls are shared out; the partners are taken in
+// ascending index and the forces added in that order, whatever the lanes'
+// order of finding them.
 template <typename T>
-__global__ void k_fwd_forces(int n, AdjTables A, AdjGrid G, const int* type, const T* x,
-                             const T* vel, const T* omg, ListsT<T> prev, int has_prev,
-                             ListsT<T> cur, T* F, T* Tq, T kn, T en, T muc, int zero_spring,
-                             int* overflow) {
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= n) return;
+__global__ void __launch_bounds__(kAdjBlock)
+    k_fwd_forces(int n, AdjTables A, AdjGrid G, const int* type, const T* x, const T* vel,
+                 const T* omg, ListsT<T> prev, int has_prev, ListsT<T> cur, T* F, T* Tq, T kn,
+                 T en, T muc, int zero_spring, int* overflow) {
+  constexpr int kGroups = kAdjBlock / kAdjLanes;
+  __shared__ int found_s[kGroups][kAdjCap], cand_s[kGroups][kAdjCap], count_s[kGroups];
+  const int grp = threadIdx.x / kAdjLanes, lane = threadIdx.x % kAdjLanes;
+  const unsigned mask = ((1u << kAdjLanes) - 1u) << (threadIdx.x & 31 & ~(kAdjLanes - 1));
+  const int t = blockIdx.x * kGroups + grp;
+  if (t >= n) return;   // (the particle's lanes together)
   TypeDesc const& tp = A.types[type[t]];
   const V3<T> xt = ldv(x, t);
   V3<T> Ft = vconst<T>(tp.weight[0], tp.weight[1], tp.weight[2]);
   V3<T> Tt = vconst<T>(0., 0., 0.);
   const V3<T> zero = vconst<T>(0., 0., 0.);
   // partners whose centres pass the contact-distance test, from the 27
-  // cells around t's, in ascending index
-  int cand[kAdjCap];
-  int nc = 0;
+  // cells around t's
+  if (lane == 0) count_s[grp] = 0;
+  __syncwarp(mask);
   {
     const int c = G.cell[t];
     const int ci = c % G.nb[0], cj = (c / G.nb[0]) % G.nb[1], ck = c / (G.nb[0] * G.nb[1]);
-    for (int k3 = max(ck - 1, 0); k3 <= min(ck + 1, G.nb[2] - 1); ++k3)
-      for (int j3 = max(cj - 1, 0); j3 <= min(cj + 1, G.nb[1] - 1); ++j3)
-        for (int i3 = max(ci - 1, 0); i3 <= min(ci + 1, G.nb[0] - 1); ++i3) {
-          const int cc = (k3 * G.nb[1] + j3) * G.nb[0] + i3;
-          for (int e = G.start[cc]; e < G.start[cc + 1]; ++e) {
-            const int u = G.items[e];
-            if (u == t) continue;
-            TypeDesc const& tu = A.types[type[u]];
-            const V3<T> xu = ldv(x, u);
-            const double dx = val(xu.x) - val(xt.x), dy = val(xu.y) - val(xt.y),
-                         dz = val(xu.z) - val(xt.z);
-            const double R = (tp.radius + tu.radius) * (1. + 1.e-9);
-            if (dx * dx + dy * dy + dz * dz >= R * R) continue;
-            if (nc < kAdjCap) cand[nc++] = u;
-            else atomicOr(overflow, 1);
-          }
-        }
-    for (int i = 1; i < nc; ++i) {
-      const int u = cand[i];
-      int j = i - 1;
-      while (j >= 0 && cand[j] > u) {
-        cand[j + 1] = cand[j];
-        --j;
+    for (int q = lane; q < 27; q += kAdjLanes) {
+      const int i3 = ci + q % 3 - 1, j3 = cj + (q / 3) % 3 - 1, k3 = ck + q / 9 - 1;
+      if (i3 < 0 || i3 >= G.nb[0] || j3 < 0 || j3 >= G.nb[1] || k3 < 0 || k3 >= G.nb[2]) continue;
+      const int cc = (k3 * G.nb[1] + j3) * G.nb[0] + i3;
+      for (int e = G.start[cc]; e < G.start[cc + 1]; ++e) {
+        const int u = G.items[e];
+        if (u == t) continue;
+        TypeDesc const& tu = A.types[type[u]];
+        const V3<T> xu = ldv(x, u);
+        const double dx = val(xu.x) - val(xt.x), dy = val(xu.y) - val(xt.y),
+                     dz = val(xu.z) - val(xt.z);
+        const double R = (tp.radius + tu.radius) * (1. + 1.e-9);
+        if (dx * dx + dy * dy + dz * dz >= R * R) continue;
+        const int at = atomicAdd(&count_s[grp], 1);
+        if (at < kAdjCap) found_s[grp][at] = u;
+        else atomicOr(overflow, 1);
       }
-      cand[j + 1] = u;
     }
   }
+  __syncwarp(mask);
+  const int nc = min(count_s[grp], kAdjCap);
+  for (int i = lane; i < nc; i += kAdjLanes) {
+    const int u = found_s[grp][i];
+    int rank = 0;
+    for (int j = 0; j < nc; ++j) rank += found_s[grp][j] < u;
+    cand_s[grp][rank] = u;
+  }
+  __syncwarp(mask);
   int k = 0;
-  for (int q = 0; q < nc; ++q) {
-    const int u = cand[q];
-    const int a = t < u ? t : u, b = t < u ? u : t;
-    TypeDesc const& ta = A.types[type[a]];
-    TypeDesc const& tb = A.types[type[b]];
-    const int j = has_prev ? findSlotT(prev, t, u) : -1;
-    const bool existed = j >= 0;
-    PairIn<T> in;
-    in.xa = ldv(x, a); in.xb = ldv(x, b);
-    in.va = ldv(vel, a); in.vb = ldv(vel, b);
-    in.wa = ldv(omg, a); in.wb = ldv(omg, b);
-    in.kd = existed ? ldv(prev.kd, (size_t)t * kAdjCap + j) : zero;
-    in.pn = existed ? ldv(prev.pn, (size_t)t * kAdjCap + j) : zero;
-    in.kn = kn; in.en = en; in.muc = muc;
-    PairY<T> y = pairContact(A, in, ta, tb, existed);
-    if (!y.contact) continue;
-    if (t == a) { Ft = Ft + y.fa; Tt = Tt + y.ta; }
-    else { Ft = Ft + y.fb; Tt = Tt + y.tb; }
-    if (k < kAdjCap) {
-      const size_t sl = (size_t)t * kAdjCap + k;
+  for (int q0 = 0; q0 < nc; q0 += kAdjLanes) {
+    V3<T> f = zero, tq = zero, kd, pn;
+    int u = 0;
+    bool hit = false;
+    if (q0 + lane < nc) {
+      u = cand_s[grp][q0 + lane];
+      const int a = t < u ? t : u, b = t < u ? u : t;
+      const int j = has_prev ? findSlotT(prev, t, u) : -1;
+      const bool existed = j >= 0;
+      PairIn<T> in;
+      in.xa = ldv(x, a); in.xb = ldv(x, b);
+      in.va = ldv(vel, a); in.vb = ldv(vel, b);
+      in.wa = ldv(omg, a); in.wb = ldv(omg, b);
+      in.kd = existed ? ldv(prev.kd, (size_t)t * kAdjCap + j) : zero;
+      in.pn = existed ? ldv(prev.pn, (size_t)t * kAdjCap + j) : zero;
+      in.kn = kn; in.en = en; in.muc = muc;
+      const PairY<T> y = pairContact(A, in, A.types[type[a]], A.types[type[b]], existed);
+      hit = y.contact;
+      if (hit) {
+        f = t == a ? y.fa : y.fb;
+        tq = t == a ? y.ta : y.tb;
+        kd = y.kd;
+        pn = y.pn;
+      }
+    }
+    unsigned hits = __ballot_sync(mask, hit) >> (threadIdx.x & 31 & ~(kAdjLanes - 1));
+    if (hit) {
+      const size_t sl = (size_t)t * kAdjCap + k + __popc(hits & ((1u << lane) - 1u));
       cur.partner[sl] = u;
-      stv(cur.kd, sl, zero_spring ? zero : y.kd);
-      stv(cur.pn, sl, y.pn);
-      ++k;
-    } else {
-      atomicOr(overflow, 1);
+      stv(cur.kd, sl, zero_spring ? zero : kd);
+      stv(cur.pn, sl, pn);
+    }
+    k += __popc(hits & ((1u << kAdjLanes) - 1u));
+    for (hits &= (1u << kAdjLanes) - 1u; hits; hits &= hits - 1u) {
+      const int src = __ffs(hits) - 1;
+      Ft = Ft + laneOf(mask, f, src);
+      Tt = Tt + laneOf(mask, tq, src);
     }
   }
-  cur.npart[t] = k;
-  for (int w = 0; w < A.nwalls; ++w) {
-    WallDesc const& wd = A.walls[w];
-    const size_t sl = (size_t)t * kAdjWalls + w;
-    const bool existed = has_prev && prev.wflag[sl];
-    WallIn<T> in;
-    in.x = xt; in.v = ldv(vel, t); in.w = ldv(omg, t);
-    in.kd = existed ? ldv(prev.wkd, sl) : zero;
-    in.pn = existed ? ldv(prev.wpn, sl) : zero;
-    in.kn = kn; in.en = en; in.muc = muc;
-    WallY<T> y = wallContact(A, in, tp, wd, existed);
-    cur.wflag[sl] = y.contact ? 1 : 0;
-    if (!y.contact) continue;
-    Ft = Ft + y.f;
-    Tt = Tt + y.t;
-    stv(cur.wkd, sl, zero_spring ? zero : y.kd);
-    stv(cur.wpn, sl, y.pn);
+  if (lane == 0) cur.npart[t] = k;
+  static_assert(kAdjWalls <= kAdjLanes, "one wall per lane");
+  {
+    V3<T> f = zero, tq = zero;
+    bool hit = false;
+    if (lane < A.nwalls) {
+      WallDesc const& wd = A.walls[lane];
+      const size_t sl = (size_t)t * kAdjWalls + lane;
+      const bool existed = has_prev && prev.wflag[sl];
+      WallIn<T> in;
+      in.x = xt; in.v = ldv(vel, t); in.w = ldv(omg, t);
+      in.kd = existed ? ldv(prev.wkd, sl) : zero;
+      in.pn = existed ? ldv(prev.wpn, sl) : zero;
+      in.kn = kn; in.en = en; in.muc = muc;
+      const WallY<T> y = wallContact(A, in, tp, wd, existed);
+      hit = y.contact;
+      cur.wflag[sl] = hit ? 1 : 0;
+      if (hit) {
+        f = y.f;
+        tq = y.t;
+        stv(cur.wkd, sl, zero_spring ? zero : y.kd);
+        stv(cur.wpn, sl, y.pn);
+      }
+    }
+    unsigned hits = __ballot_sync(mask, hit) >> (threadIdx.x & 31 & ~(kAdjLanes - 1));
+    for (hits &= (1u << kAdjLanes) - 1u; hits; hits &= hits - 1u) {
+      const int src = __ffs(hits) - 1;
+      Ft = Ft + laneOf(mask, f, src);
+      Tt = Tt + laneOf(mask, tq, src);
+    }
   }
-  stv(F, t, Ft);
-  stv(Tq, t, Tt);
+  if (lane == 0) {
+    stv(F, t, Ft);
+    stv(Tq, t, Tt);
+  }
 }
 
-// Opening kick + drift: vh = v + F h / m, wh = w + T h / I, x' = x + vh dt.
+// Closing kick (unless v, w are the step's full velocities already): v = vh +
+// F h / m, w = wh + T h / I.
 template <typename T>
-__global__ void k_fwd_move(int n, AdjTables A, const int* type, const T* x, const T* v,
-                           const T* w, const T* F, const T* Tq, T* xo, T* vh, T* wh) {
+__device__ __forceinline__ void closeKick(AdjTables const& A, TypeDesc const& tp, int closed, V3<T> F,
+                                          V3<T> Tq, V3<T>& v, V3<T>& w) {
+  if (closed) return;
+  const double h = 0.5 * A.dt;
+  v = v + vscale(F, Scal<T>::make(h / tp.mass));
+  w = w + vscale(Tq, Scal<T>::make(h / tp.inertia[0]));
+}
+
+// The closing kick of the step before (closeKick on vi, wi), then this step's
+// opening kick + drift: vh = v + F h / m, wh = w + T h / I, x' = x + vh dt;
+// the particle is counted into its cell on the way.
+template <typename T>
+__global__ void k_fwd_move(int n, AdjTables A, AdjGrid G, const int* type, int closed, const T* x,
+                           const T* vi, const T* wi, const T* F, const T* Tq, T* xo, T* vh, T* wh,
+                           int* cell, int* count) {
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= n) return;
   TypeDesc const& tp = A.types[type[t]];
   const double h = 0.5 * A.dt;
-  const V3<T> vv = ldv(v, t) + vscale(ldv(F, t), Scal<T>::make(h / tp.mass));
-  const V3<T> ww = ldv(w, t) + vscale(ldv(Tq, t), Scal<T>::make(h / tp.inertia[0]));
+  const V3<T> f = ldv(F, t), tq = ldv(Tq, t);
+  V3<T> v = ldv(vi, t), w = ldv(wi, t);
+  closeKick(A, tp, closed, f, tq, v, w);
+  const V3<T> vv = v + vscale(f, Scal<T>::make(h / tp.mass));
+  const V3<T> ww = w + vscale(tq, Scal<T>::make(h / tp.inertia[0]));
   stv(vh, t, vv);
   stv(wh, t, ww);
-  stv(xo, t, ldv(x, t) + vscale(vv, Scal<T>::make(A.dt)));
+  const V3<T> xn = ldv(x, t) + vscale(vv, Scal<T>::make(A.dt));
+  stv(xo, t, xn);
+  adjBin(G, t, xn, cell, count);
 }
 
-// Closing kick: v = vh + F h / m, w = wh + T h / I.
+// The full state after a step (closeKick on vi, wi), into its own arrays.
 template <typename T>
-__global__ void k_fwd_close(int n, AdjTables A, const int* type, const T* vh, const T* wh,
-                            const T* F, const T* Tq, T* v, T* w) {
+__global__ void k_fwd_state(int n, AdjTables A, const int* type, int closed, const T* x,
+                            const T* vi, const T* wi, const T* F, const T* Tq, T* xo, T* vo, T* wo,
+                            T* Fo, T* To) {
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= n) return;
-  TypeDesc const& tp = A.types[type[t]];
-  const double h = 0.5 * A.dt;
-  stv(v, t, ldv(vh, t) + vscale(ldv(F, t), Scal<T>::make(h / tp.mass)));
-  stv(w, t, ldv(wh, t) + vscale(ldv(Tq, t), Scal<T>::make(h / tp.inertia[0])));
+  const V3<T> f = ldv(F, t), tq = ldv(Tq, t);
+  V3<T> v = ldv(vi, t), w = ldv(wi, t);
+  closeKick(A, A.types[type[t]], closed, f, tq, v, w);
+  stv(xo, t, ldv(x, t));
+  stv(vo, t, v);
+  stv(wo, t, w);
+  stv(Fo, t, f);
+  stv(To, t, tq);
+}
+
+// The used part of one step's contact lists, kAdjLanes lanes per particle.
+template <typename T>
+__global__ void __launch_bounds__(kAdjBlock) k_copy_lists(int n, ListsT<T> dst, ListsT<T> src) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  const int t = i / kAdjLanes, lane = i % kAdjLanes;
+  if (t >= n) return;
+  const int np = src.npart[t];
+  if (lane == 0) dst.npart[t] = np;
+  for (int k = lane; k < np; k += kAdjLanes) {
+    const size_t sl = (size_t)t * kAdjCap + k;
+    dst.partner[sl] = src.partner[sl];
+    stv(dst.kd, sl, ldv(src.kd, sl));
+    stv(dst.pn, sl, ldv(src.pn, sl));
+  }
+  const size_t ws = (size_t)t * kAdjWalls + lane;
+  const int wf = src.wflag[ws];
+  dst.wflag[ws] = wf;
+  if (wf) {
+    stv(dst.wkd, ws, ldv(src.wkd, ws));
+    stv(dst.wpn, ws, ldv(src.wpn, ws));
+  }
 }
 
 // Per-particle squared error of positions and velocities.
@@ -392,178 +507,150 @@ __global__ void k_fwd_loss(int n, const T* x, const T* v, const double* tx, cons
 }
 
 // ------------------------------------------------------------- reverse --
-// Closing kick of step s, transposed: lvh = lv, lF += lv h / m, and the same
-// for the rotation.
-__global__ void k_bwd_close(int n, AdjTables A, const int* type, const double* lv,
-                            const double* lw, double* lF, double* lT, double* lvh, double* lwh) {
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= n) return;
+// Adjoints of the particles' x, v, w, F, T after a step (or, at the leapfrog
+// start, of its inputs), 3 per particle each.
+struct AdjState {
+  double *x, *v, *w, *F, *T;
+};
+// Adjoints of one step's contact history, in the layout of its lists; only
+// the entries of the lists in use are meaningful.
+struct AdjHist {
+  double *kd, *pn, *wkd, *wpn;
+};
+
+// One step, transposed: the closing kick, the contact forces and the opening
+// kick + drift, from the adjoints at step s (in) to those at s - 1 (out);
+// start: the leapfrog start's evaluation alone (no kicks; the spring it left
+// was zeroed).  Per contact the adjoints of t's own inputs come from one
+// sweep of contactBar, once from either side; the history's go to the slots
+// of step s - 1 that supplied it, and kn, en, muc's to the lower index.
+// kAdjLanes lanes per particle, one contact or wall each, summed over the
+// lanes in a fixed tree.
+__global__ void __launch_bounds__(kAdjBlock)
+    k_bwd_step(int n, AdjTables A, const int* type, const double* x, const double* vel,
+               const double* omg, ListsT<double> prev, int has_prev, ListsT<double> cur,
+               AdjState in, AdjState out, AdjHist h_in, AdjHist h_out, double* lp, double kn,
+               double en, double muc, int start) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  const int t = i / kAdjLanes, lane = i % kAdjLanes;
+  const unsigned mask = ((1u << kAdjLanes) - 1u) << (threadIdx.x & 31 & ~(kAdjLanes - 1));
+  if (t >= n) return;   // (the particle's lanes together)
   TypeDesc const& tp = A.types[type[t]];
   const double h = 0.5 * A.dt;
-  for (int d = 0; d < 3; ++d) {
-    lvh[3 * t + d] = lv[3 * t + d];
-    lF[3 * t + d] += lv[3 * t + d] * (h / tp.mass);
-    lwh[3 * t + d] = lw[3 * t + d];
-    lT[3 * t + d] += lw[3 * t + d] * (h / tp.inertia[0]);
+  const W3 zero = w3zero();
+  // adjoint of the force and torque of particle p: the closing kick's share added
+  auto forceBar = [&](int p, TypeDesc const& q, W3& f, W3& tq) {
+    f = ldd(in.F, p);
+    tq = ldd(in.T, p);
+    if (!start) {
+      f = f + (h / q.mass) * ldd(in.v, p);
+      tq = tq + (h / q.inertia[0]) * ldd(in.w, p);
+    }
+  };
+  W3 lFt, lTt;
+  forceBar(t, tp, lFt, lTt);
+  const W3 xt = ldd(x, t), vt = ldd(vel, t), wt = ldd(omg, t);
+  W3 gx = zero, gv = zero, gw = zero, gp = zero;
+  // the history adjoints of step s - 1 start from zero
+  if (has_prev) {
+    const int pp = prev.npart[t];
+    for (int k = lane; k < pp; k += kAdjLanes) {
+      stv(h_out.kd, (size_t)t * kAdjCap + k, zero);
+      stv(h_out.pn, (size_t)t * kAdjCap + k, zero);
+    }
+    stv(h_out.wkd, (size_t)t * kAdjWalls + lane, zero);
+    stv(h_out.wpn, (size_t)t * kAdjWalls + lane, zero);
   }
-}
-
-// Opening kick + drift of step s (from s - 1), transposed: the adjoints of
-// x, v, w, F, T at s - 1 from those of x_s, vh, wh.
-__global__ void k_bwd_move(int n, AdjTables A, const int* type, const double* lx,
-                           const double* lvh, const double* lwh, double* lv, double* lw,
-                           double* lF, double* lT) {
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= n) return;
-  TypeDesc const& tp = A.types[type[t]];
-  const double h = 0.5 * A.dt;
-  for (int d = 0; d < 3; ++d) {
-    const double g = lvh[3 * t + d] + lx[3 * t + d] * A.dt;
-    lv[3 * t + d] = g;
-    lF[3 * t + d] = g * (h / tp.mass);
-    lw[3 * t + d] = lwh[3 * t + d];
-    lT[3 * t + d] = lwh[3 * t + d] * (h / tp.inertia[0]);
-  }
-}
-
-__device__ __forceinline__ double dotY(V3<double> l, V3<Dual<1>> y) {
-  return l.x * y.x.d[0] + l.y * y.y.d[0] + l.z * y.z.d[0];
-}
-__device__ __forceinline__ void seedVec(V3<Dual<1>>& v, int c) {
-  if (c == 0) v.x.d[0] = 1.;
-  else if (c == 1) v.y.d[0] = 1.;
-  else v.z.d[0] = 1.;
-}
-__device__ __forceinline__ V3<Dual<1>> lift(V3<double> a) { return promote<Dual<1>>(a); }
-
-// Contact forces of step s, transposed.  For every contact of particle t the
-// law is re-evaluated on Dual<1> numbers once per input of t's (position,
-// velocity, angular velocity; the history it carried in; kn, en, muc once
-// per contact, by its lower index), and the derivative of every output is
-// contracted with that output's adjoint.  The history adjoints go to the
-// slots of step s - 1 that supplied the history.
-__global__ void k_bwd_forces(int n, AdjTables A, const int* type, const double* x,
-                             const double* vel, const double* omg, ListsT<double> prev,
-                             int has_prev, ListsT<double> cur, const double* lF, const double* lT,
-                             const double* lkd, const double* lpn, const double* lwkd,
-                             const double* lwpn, int spring_zeroed, double* lx, double* lvh,
-                             double* lwh, double* lkd_prev, double* lpn_prev, double* lwkd_prev,
-                             double* lwpn_prev, double* lp, double kn, double en, double muc) {
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= n) return;
-  TypeDesc const& tp = A.types[type[t]];
-  double gx[3] = {0., 0., 0.}, gv[3] = {0., 0., 0.}, gw[3] = {0., 0., 0.};
-  double gp[3] = {0., 0., 0.};
-  const V3<double> zero = v3(0., 0., 0.);
+  __syncwarp(mask);
   const int np = cur.npart[t];
-  for (int k = 0; k < np; ++k) {
+  for (int k = lane; k < np; k += kAdjLanes) {
     const size_t sl = (size_t)t * kAdjCap + k;
     const int u = cur.partner[sl];
-    const int a = t < u ? t : u, b = t < u ? u : t;
-    TypeDesc const& ta = A.types[type[a]];
-    TypeDesc const& tb = A.types[type[b]];
+    TypeDesc const& tu = A.types[type[u]];
     const int j = has_prev ? findSlotT(prev, t, u) : -1;
     const bool existed = j >= 0;
     const size_t pj = (size_t)t * kAdjCap + (j >= 0 ? j : 0);
-    PairIn<double> in;
-    in.xa = ldd(x, a); in.xb = ldd(x, b);
-    in.va = ldd(vel, a); in.vb = ldd(vel, b);
-    in.wa = ldd(omg, a); in.wb = ldd(omg, b);
-    in.kd = existed ? ldd(prev.kd, pj) : zero;
-    in.pn = existed ? ldd(prev.pn, pj) : zero;
-    const V3<double> lFa = ldd(lF, a), lTa = ldd(lT, a), lFb = ldd(lF, b), lTb = ldd(lT, b);
-    const V3<double> lk = spring_zeroed ? zero : ldd(lkd, sl), ln = ldd(lpn, sl);
-    const bool mine_a = t == a;
-    const bool memory = modelOf(A, ta.mat, tb.mat).memory != 0;
-    // inputs seeded by t: 0-8 own x, v, w; 9-14 history (when carried in);
-    // 15-17 kn, en, muc (lower index only)
-    const int nseed = 9 + ((existed && memory) ? 6 : 0) + (mine_a ? 3 : 0);
-    double ghist[6] = {0., 0., 0., 0., 0., 0.};
-    for (int s = 0; s < nseed; ++s) {
-      int slot = s;
-      if (s >= 9 && !(existed && memory)) slot = s + 6;
-      PairIn<Dual<1>> din;
-      din.xa = lift(in.xa); din.xb = lift(in.xb);
-      din.va = lift(in.va); din.vb = lift(in.vb);
-      din.wa = lift(in.wa); din.wb = lift(in.wb);
-      din.kd = lift(in.kd); din.pn = lift(in.pn);
-      din.kn = dconst<1>(kn); din.en = dconst<1>(en); din.muc = dconst<1>(muc);
-      if (slot < 3) seedVec(mine_a ? din.xa : din.xb, slot);
-      else if (slot < 6) seedVec(mine_a ? din.va : din.vb, slot - 3);
-      else if (slot < 9) seedVec(mine_a ? din.wa : din.wb, slot - 6);
-      else if (slot < 12) seedVec(din.kd, slot - 9);
-      else if (slot < 15) seedVec(din.pn, slot - 12);
-      else if (slot == 15) din.kn.d[0] = 1.;
-      else if (slot == 16) din.en.d[0] = 1.;
-      else din.muc.d[0] = 1.;
-      PairY<Dual<1>> y = pairContact(A, din, ta, tb, existed);
-      if (!y.contact) continue;
-      const double g = dotY(lFa, y.fa) + dotY(lTa, y.ta) + dotY(lFb, y.fb) + dotY(lTb, y.tb) +
-                       dotY(lk, y.kd) + dotY(ln, y.pn);
-      if (slot < 3) gx[slot] += g;
-      else if (slot < 6) gv[slot - 3] += g;
-      else if (slot < 9) gw[slot - 6] += g;
-      else if (slot < 15) ghist[slot - 9] += g;
-      else gp[slot - 15] += g;
-    }
-    if (existed && memory) {
-      for (int d = 0; d < 3; ++d) {
-        lkd_prev[3 * pj + d] = ghist[d];
-        lpn_prev[3 * pj + d] = ghist[3 + d];
-      }
+    const bool mine = t < u;   // t is the law's first body
+    const W3 xu = ldd(x, u);
+    W3 lFu, lTu;
+    forceBar(u, tu, lFu, lTu);
+    LawArgs a, g;
+    W3 pen;
+    const W3 xa = mine ? xt : xu, xb = mine ? xu : xt;
+    const double ra = mine ? tp.radius : tu.radius, rb = mine ? tu.radius : tp.radius;
+    if (!sphereSphereG(xa, ra, xb, rb, a.pc, pen)) continue;
+    a.pen = pen;
+    const W3 vu = ldd(vel, u), wu = ldd(omg, u);
+    a.x0 = xa; a.v0 = mine ? vt : vu; a.w0 = mine ? wt : wu;
+    a.x1 = xb; a.v1 = mine ? vu : vt; a.w1 = mine ? wu : wt;
+    a.kd = existed ? ldd(prev.kd, pj) : zero;
+    a.pn = existed ? ldd(prev.pn, pj) : zero;
+    a.kn = kn; a.en = en; a.muc = muc;
+    ModelDesc const& m = mine ? modelOf(A, tp.mat, tu.mat) : modelOf(A, tu.mat, tp.mat);
+    contactBar(m, A.dt, a, mine ? tp.mass : tu.mass, mine ? tu.mass : tp.mass, existed,
+               mine ? lFt : lFu, mine ? lTt : lTu, mine ? lFu : lFt, mine ? lTu : lTt,
+               start ? zero : ldd(h_in.kd, sl), ldd(h_in.pn, sl), g);
+    sphereSphereBar(xa, ra, xb, rb, g.pc, g.pen, g.x0, g.x1);
+    acc(gx, mine ? g.x0 : g.x1);
+    acc(gv, mine ? g.v0 : g.v1);
+    acc(gw, mine ? g.w0 : g.w1);
+    if (mine) acc(gp, v3(g.kn, g.en, g.muc));
+    if (existed && m.memory) {
+      stv(h_out.kd, pj, g.kd);
+      stv(h_out.pn, pj, g.pn);
     }
   }
-  for (int w = 0; w < A.nwalls; ++w) {
-    const size_t sl = (size_t)t * kAdjWalls + w;
-    if (!cur.wflag[sl]) continue;
-    WallDesc const& wd = A.walls[w];
+  if (lane < A.nwalls && cur.wflag[(size_t)t * kAdjWalls + lane]) {
+    const size_t sl = (size_t)t * kAdjWalls + lane;
+    WallDesc const& wd = A.walls[lane];
     const bool existed = has_prev && prev.wflag[sl];
-    const bool memory = modelOf(A, tp.mat, wd.mat).memory != 0;
-    WallIn<double> in;
-    in.x = ldd(x, t); in.v = ldd(vel, t); in.w = ldd(omg, t);
-    in.kd = existed ? ldd(prev.wkd, sl) : zero;
-    in.pn = existed ? ldd(prev.wpn, sl) : zero;
-    const V3<double> lFt = ldd(lF, t), lTt = ldd(lT, t);
-    const V3<double> lk = spring_zeroed ? zero : ldd(lwkd, sl), ln = ldd(lwpn, sl);
-    const int nseed = 9 + ((existed && memory) ? 6 : 0) + 3;
-    double ghist[6] = {0., 0., 0., 0., 0., 0.};
-    for (int s = 0; s < nseed; ++s) {
-      int slot = s;
-      if (s >= 9 && !(existed && memory)) slot = s + 6;
-      WallIn<Dual<1>> din;
-      din.x = lift(in.x); din.v = lift(in.v); din.w = lift(in.w);
-      din.kd = lift(in.kd); din.pn = lift(in.pn);
-      din.kn = dconst<1>(kn); din.en = dconst<1>(en); din.muc = dconst<1>(muc);
-      if (slot < 3) seedVec(din.x, slot);
-      else if (slot < 6) seedVec(din.v, slot - 3);
-      else if (slot < 9) seedVec(din.w, slot - 6);
-      else if (slot < 12) seedVec(din.kd, slot - 9);
-      else if (slot < 15) seedVec(din.pn, slot - 12);
-      else if (slot == 15) din.kn.d[0] = 1.;
-      else if (slot == 16) din.en.d[0] = 1.;
-      else din.muc.d[0] = 1.;
-      WallY<Dual<1>> y = wallContact(A, din, tp, wd, existed);
-      if (!y.contact) continue;
-      const double g = dotY(lFt, y.f) + dotY(lTt, y.t) + dotY(lk, y.kd) + dotY(ln, y.pn);
-      if (slot < 3) gx[slot] += g;
-      else if (slot < 6) gv[slot - 3] += g;
-      else if (slot < 9) gw[slot - 6] += g;
-      else if (slot < 15) ghist[slot - 9] += g;
-      else gp[slot - 15] += g;
-    }
-    if (existed && memory) {
-      for (int d = 0; d < 3; ++d) {
-        lwkd_prev[3 * sl + d] = ghist[d];
-        lwpn_prev[3 * sl + d] = ghist[3 + d];
+    ModelDesc const& m = modelOf(A, tp.mat, wd.mat);
+    LawArgs a, g;
+    W3 pen;
+    if (sphereWallG(xt, tp.radius, wd, a.pc, pen)) {
+      a.pen = pen;
+      a.x0 = xt; a.v0 = vt; a.w0 = wt;
+      a.x1 = v3(wd.centre[0], wd.centre[1], wd.centre[2]);
+      a.v1 = zero; a.w1 = zero;
+      a.kd = existed ? ldd(prev.wkd, sl) : zero;
+      a.pn = existed ? ldd(prev.wpn, sl) : zero;
+      a.kn = kn; a.en = en; a.muc = muc;
+      contactBar(m, A.dt, a, tp.mass, 1.e20, existed, lFt, lTt, zero, zero,
+                 start ? zero : ldd(h_in.wkd, sl), ldd(h_in.wpn, sl), g);
+      sphereWallBar(xt, tp.radius, wd, g.pc, g.pen, g.x0);
+      acc(gx, g.x0);
+      acc(gv, g.v0);
+      acc(gw, g.w0);
+      acc(gp, v3(g.kn, g.en, g.muc));
+      if (existed && m.memory) {
+        stv(h_out.wkd, sl, g.kd);
+        stv(h_out.wpn, sl, g.pn);
       }
     }
   }
-  for (int d = 0; d < 3; ++d) {
-    lx[3 * t + d] += gx[d];
-    lvh[3 * t + d] += gv[d];
-    lwh[3 * t + d] += gw[d];
-    lp[3 * t + d] += gp[d];
+  __syncwarp(mask);
+#pragma unroll
+  for (int o = kAdjLanes / 2; o > 0; o >>= 1) {
+    auto add = [&](W3& q) {
+      q = q + v3(__shfl_xor_sync(mask, q.x, o, kAdjLanes), __shfl_xor_sync(mask, q.y, o, kAdjLanes),
+                 __shfl_xor_sync(mask, q.z, o, kAdjLanes));
+    };
+    add(gx); add(gv); add(gw); add(gp);
   }
+  if (lane != 0) return;
+  stv(lp, t, ldd(lp, t) + gp);
+  if (start) {
+    stv(out.v, t, ldd(in.v, t) + gv);
+    return;
+  }
+  // opening kick + drift, transposed
+  const W3 lx = ldd(in.x, t) + gx;
+  const W3 lv = ldd(in.v, t) + gv + A.dt * lx, lw = ldd(in.w, t) + gw;
+  stv(out.x, t, lx);
+  stv(out.v, t, lv);
+  stv(out.w, t, lw);
+  stv(out.F, t, (h / tp.mass) * lv);
+  stv(out.T, t, (h / tp.inertia[0]) * lw);
 }
 
 __global__ void k_bwd_seed(int n, const double* x, const double* v, const double* tx,
@@ -607,14 +694,44 @@ struct AdjointSystem {
   double *d_x0 = nullptr, *d_v0 = nullptr, *d_w0 = nullptr;
   int* d_overflow = nullptr;
   AdjGrid G{};
-  int *d_cell = nullptr, *d_count = nullptr, *d_fill = nullptr, *d_start = nullptr,
+  int *d_cell = nullptr, *d_count = nullptr, *d_cursor = nullptr, *d_start = nullptr,
       *d_items = nullptr;
   std::vector<void*> allocs;
+  // A run's working memory: blocks handed out in order, kept for the next run
+  // up to kKeepBytes in all and given back with the system.  (A run of the
+  // calibration case needs some 500 arrays; allocating and freeing them took
+  // longer than its kernels.)
+  struct Block {
+    char* p;
+    size_t size, used;
+  };
+  std::vector<Block> work;
+  static constexpr size_t kKeepBytes = size_t(1) << 30, kBlockBytes = size_t(32) << 20;
   cudaStream_t st = nullptr;
 
   ~AdjointSystem() {
     for (void* p : allocs) cudaFree(p);
+    for (auto const& b : work) cudaFree(b.p);
     if (st) cudaStreamDestroy(st);
+  }
+  template <typename T>
+  T* scratch(size_t count) {
+    const size_t bytes = (std::max<size_t>(count, 1) * sizeof(T) + 255) & ~size_t(255);
+    for (auto& b : work)
+      if (b.size - b.used >= bytes) {
+        T* p = reinterpret_cast<T*>(b.p + b.used);
+        b.used += bytes;
+        return p;
+      }
+    Block b{nullptr, std::max(bytes, kBlockBytes), bytes};
+    if (cudaMalloc(&b.p, b.size) != cudaSuccess) {
+      // (a block larger than the array asked for may not fit any more)
+      cudaGetLastError();
+      b.size = bytes;
+      ACK(cudaMalloc(&b.p, b.size));
+    }
+    work.push_back(b);
+    return reinterpret_cast<T*>(b.p);
   }
   template <typename T>
   T* alloc(size_t count) {
@@ -626,30 +743,23 @@ struct AdjointSystem {
   template <typename T>
   ListsT<T> allocLists() {
     ListsT<T> L;
-    L.partner = alloc<int>((size_t)n * kAdjCap);
-    L.npart = alloc<int>(n);
-    L.kd = alloc<T>((size_t)n * kAdjCap * 3);
-    L.pn = alloc<T>((size_t)n * kAdjCap * 3);
-    L.wflag = alloc<int>((size_t)n * kAdjWalls);
-    L.wkd = alloc<T>((size_t)n * kAdjWalls * 3);
-    L.wpn = alloc<T>((size_t)n * kAdjWalls * 3);
-    ACK(cudaMemsetAsync(L.npart, 0, n * sizeof(int), st));
+    L.partner = scratch<int>((size_t)n * kAdjCap);
+    L.npart = scratch<int>(n);
+    L.kd = scratch<T>((size_t)n * kAdjCap * 3);
+    L.pn = scratch<T>((size_t)n * kAdjCap * 3);
+    L.wflag = scratch<int>((size_t)n * kAdjWalls);
+    L.wkd = scratch<T>((size_t)n * kAdjWalls * 3);
+    L.wpn = scratch<T>((size_t)n * kAdjWalls * 3);
+    // (k_fwd_forces writes the flags of the walls there are)
     ACK(cudaMemsetAsync(L.wflag, 0, (size_t)n * kAdjWalls * sizeof(int), st));
     return L;
   }
   template <typename T>
   void copyLists(ListsT<T> const& dst, ListsT<T> const& src) {
-    auto cp = [&](void* d, const void* s, size_t bytes) {
-      ACK(cudaMemcpyAsync(d, s, bytes, cudaMemcpyDeviceToDevice, st));
-    };
-    cp(dst.partner, src.partner, (size_t)n * kAdjCap * sizeof(int));
-    cp(dst.npart, src.npart, (size_t)n * sizeof(int));
-    cp(dst.kd, src.kd, (size_t)n * kAdjCap * 3 * sizeof(T));
-    cp(dst.pn, src.pn, (size_t)n * kAdjCap * 3 * sizeof(T));
-    cp(dst.wflag, src.wflag, (size_t)n * kAdjWalls * sizeof(int));
-    cp(dst.wkd, src.wkd, (size_t)n * kAdjWalls * 3 * sizeof(T));
-    cp(dst.wpn, src.wpn, (size_t)n * kAdjWalls * 3 * sizeof(T));
+    k_copy_lists<T><<<laneBlocks(), kAdjBlock, 0, st>>>(n, dst, src);
   }
+  // blocks of a kernel with kAdjLanes lanes per particle
+  int laneBlocks() const { return (int)(((long long)n * kAdjLanes + kAdjBlock - 1) / kAdjBlock); }
 
   void create(std::string const& xml) {
     readAdjointSetup(xml, setup);
@@ -694,7 +804,8 @@ struct AdjointSystem {
     }
     G.ncells = G.nb[0] * G.nb[1] * G.nb[2];
     d_count = alloc<int>(G.ncells);
-    d_fill = alloc<int>(G.ncells);
+    d_cursor = alloc<int>(G.ncells);
+    ACK(cudaMemset(d_count, 0, (size_t)G.ncells * sizeof(int)));
     d_start = alloc<int>((size_t)G.ncells + 1);
     G.start = d_start;
   }
@@ -722,15 +833,25 @@ struct AdjointSystem {
     else ACK(cudaMemset(d_w0, 0, 3 * (size_t)n * sizeof(double)));
   }
 
-  // Frees the buffers allocated after a mark (one run's working memory).
+  // Takes the working memory back at the end of a run; what is beyond
+  // kKeepBytes is freed.
   struct Scope {
     AdjointSystem* sys;
-    size_t mark;
-    explicit Scope(AdjointSystem* s) : sys(s), mark(s->allocs.size()) {}
+    explicit Scope(AdjointSystem* s) : sys(s) {}
     ~Scope() {
       if (sys->st) cudaStreamSynchronize(sys->st);
-      for (size_t k = mark; k < sys->allocs.size(); ++k) cudaFree(sys->allocs[k]);
-      sys->allocs.resize(mark);
+      size_t kept = 0;
+      std::vector<Block> keep;
+      for (auto& b : sys->work) {
+        if (kept + b.size <= kKeepBytes) {
+          kept += b.size;
+          b.used = 0;
+          keep.push_back(b);
+        } else {
+          cudaFree(b.p);
+        }
+      }
+      sys->work.swap(keep);
     }
   };
 
@@ -749,64 +870,88 @@ struct AdjointSystem {
   template <typename T>
   State<T> allocState() {
     State<T> S;
-    S.x = alloc<T>(3 * (size_t)n); S.v = alloc<T>(3 * (size_t)n); S.w = alloc<T>(3 * (size_t)n);
-    S.F = alloc<T>(3 * (size_t)n); S.Tq = alloc<T>(3 * (size_t)n);
+    for (T** p : {&S.x, &S.v, &S.w, &S.F, &S.Tq}) *p = scratch<T>(3 * (size_t)n);
     return S;
   }
+  // Where the forward run is: positions, the velocities (closed: after the
+  // step's closing kick, else the half-step ones), forces and torques.
   template <typename T>
-  void copyState(State<T> const& d, State<T> const& s) {
-    const size_t b = 3 * (size_t)n * sizeof(T);
-    for (auto pr : {std::make_pair(d.x, s.x), std::make_pair(d.v, s.v), std::make_pair(d.w, s.w),
-                    std::make_pair(d.F, s.F), std::make_pair(d.Tq, s.Tq)})
-      ACK(cudaMemcpyAsync(pr.first, pr.second, b, cudaMemcpyDeviceToDevice, st));
-  }
+  struct Point {
+    const T *x, *v, *w;
+    int closed;
+    T *F, *Tq;
+  };
 
-  // Contact forces at positions x (the grid is rebuilt from them first).
+  // Contact forces at positions x, whose cells are counted.
   template <typename T>
   void forces(const T* x, const T* vel, const T* omg, ListsT<T> const& prev, int has_prev,
               ListsT<T> const& cur, T* F, T* Tq, T kn, T en, T muc, int zero_spring) {
-    ACK(cudaMemsetAsync(d_count, 0, (size_t)G.ncells * sizeof(int), st));
-    ACK(cudaMemsetAsync(d_fill, 0, (size_t)G.ncells * sizeof(int), st));
-    k_adj_bin<T><<<nblk(n), 128, 0, st>>>(n, G, x, d_cell, d_count);
-    k_adj_scan<<<1, 1024, 0, st>>>(G.ncells, d_count, d_start);
-    k_adj_place<<<nblk(n), 128, 0, st>>>(n, d_cell, d_start, d_fill, d_items);
-    k_fwd_forces<T><<<nblk(n), 128, 0, st>>>(n, A, G, d_type, x, vel, omg, prev, has_prev, cur,
-                                             F, Tq, kn, en, muc, zero_spring, d_overflow);
+    k_adj_scan<<<1, 1024, 0, st>>>(G.ncells, d_count, d_start, d_cursor);
+    k_adj_place<<<nblk(n), 128, 0, st>>>(n, d_cell, d_cursor, d_items);
+    k_fwd_forces<T><<<laneBlocks(), kAdjBlock, 0, st>>>(n, A, G, d_type, x, vel, omg, prev,
+                                                        has_prev, cur, F, Tq, kn, en, muc,
+                                                        zero_spring, d_overflow);
   }
 
   // Leapfrog start: forces at (x0, v0, w0) with no history, spring zeroed.
   template <typename T>
-  void start(State<T>& S, ListsT<T>& L, T kn, T en, T muc, int seed_v0 = -1) {
+  Point<T> start(State<T> const& S, ListsT<T> const& L, T kn, T en, T muc, int seed_v0 = -1) {
     const int n3 = 3 * n;
+    // (a run that failed part way may have left counts behind)
+    ACK(cudaMemsetAsync(d_count, 0, (size_t)G.ncells * sizeof(int), st));
     k_promote<T><<<nblk(n3), 128, 0, st>>>(n3, d_x0, S.x);
     k_promote<T><<<nblk(n3), 128, 0, st>>>(n3, d_v0, S.v);
     if (seed_v0 >= 0) k_seed<T><<<1, 1, 0, st>>>(S.v, seed_v0);
     k_promote<T><<<nblk(n3), 128, 0, st>>>(n3, d_w0, S.w);
+    k_adj_bin<T><<<nblk(n), 128, 0, st>>>(n, G, S.x, d_cell, d_count);
     forces<T>(S.x, S.v, S.w, L, 0, L, S.F, S.Tq, kn, en, muc, 1);
     ACK(cudaGetLastError());
+    return {S.x, S.v, S.w, 1, S.F, S.Tq};
   }
-  // One step: move into (xs, vh, wh), forces with history prev -> cur,
-  // closing kick; S.x becomes xs.
+  // One step from P: move into (xs, vh, wh), then the forces there with
+  // history prev -> cur; P becomes the new point, before its closing kick.
   template <typename T>
-  void advance(State<T>& S, T* xs, T* vh, T* wh, ListsT<T> const& prev, ListsT<T> const& cur,
+  void advance(Point<T>& P, T* xs, T* vh, T* wh, ListsT<T> const& prev, ListsT<T> const& cur,
                T kn, T en, T muc) {
-    k_fwd_move<T><<<nblk(n), 128, 0, st>>>(n, A, d_type, S.x, S.v, S.w, S.F, S.Tq, xs, vh, wh);
-    forces<T>(xs, vh, wh, prev, 1, cur, S.F, S.Tq, kn, en, muc, 0);
-    k_fwd_close<T><<<nblk(n), 128, 0, st>>>(n, A, d_type, vh, wh, S.F, S.Tq, S.v, S.w);
-    ACK(cudaMemcpyAsync(S.x, xs, 3 * (size_t)n * sizeof(T), cudaMemcpyDeviceToDevice, st));
+    k_fwd_move<T><<<nblk(n), 128, 0, st>>>(n, A, G, d_type, P.closed, P.x, P.v, P.w, P.F, P.Tq, xs,
+                                           vh, wh, d_cell, d_count);
+    forces<T>(xs, vh, wh, prev, 1, cur, P.F, P.Tq, kn, en, muc, 0);
     ACK(cudaGetLastError());
+    P.x = xs; P.v = vh; P.w = wh; P.closed = 0;
+  }
+  // The full state at P into S.
+  template <typename T>
+  void stateOf(Point<T> const& P, State<T> const& S) {
+    k_fwd_state<T><<<nblk(n), 128, 0, st>>>(n, A, d_type, P.closed, P.x, P.v, P.w, P.F, P.Tq, S.x,
+                                            S.v, S.w, S.F, S.Tq);
+  }
+  // Targets to the device (x, then v).
+  double* targets(const double* tx, const double* tv) {
+    const size_t n3 = 3 * (size_t)n;
+    double* d = scratch<double>(2 * n3);
+    ACK(cudaMemcpyAsync(d, tx, n3 * sizeof(double), cudaMemcpyHostToDevice, st));
+    ACK(cudaMemcpyAsync(d + n3, tv, n3 * sizeof(double), cudaMemcpyHostToDevice, st));
+    return d;
   }
   template <typename T>
-  void lossOf(State<T> const& S, const double* tx, const double* tv, std::vector<T>& per) {
-    double* dtx = alloc<double>(3 * (size_t)n);
-    double* dtv = alloc<double>(3 * (size_t)n);
-    T* out = alloc<T>(n);
-    ACK(cudaMemcpyAsync(dtx, tx, 3 * (size_t)n * sizeof(double), cudaMemcpyHostToDevice, st));
-    ACK(cudaMemcpyAsync(dtv, tv, 3 * (size_t)n * sizeof(double), cudaMemcpyHostToDevice, st));
-    k_fwd_loss<T><<<nblk(n), 128, 0, st>>>(n, S.x, S.v, dtx, dtv, out);
+  void lossOf(State<T> const& S, const double* dt, std::vector<T>& per) {
+    T* out = scratch<T>(n);
+    k_fwd_loss<T><<<nblk(n), 128, 0, st>>>(n, S.x, S.v, dt, dt + 3 * (size_t)n, out);
     per.resize(n);
     ACK(cudaMemcpyAsync(per.data(), out, n * sizeof(T), cudaMemcpyDeviceToHost, st));
     ACK(cudaStreamSynchronize(st));
+  }
+  // Two sets of the arrays a step moves into, used alternately.
+  template <typename T>
+  struct Pair {
+    T *x[2], *v[2], *w[2];
+  };
+  template <typename T>
+  Pair<T> allocPair() {
+    Pair<T> b;
+    for (int k = 0; k < 2; ++k)
+      for (T** p : {&b.x[k], &b.v[k], &b.w[k]}) *p = scratch<T>(3 * (size_t)n);
+    return b;
   }
 
   // Forward run (and, with gradients requested, the reverse sweep) in FP64.
@@ -821,106 +966,86 @@ struct AdjointSystem {
     const size_t n3 = 3 * (size_t)n;
     ACK(cudaMemsetAsync(d_overflow, 0, sizeof(int), st));
     State<double> S = allocState<double>();
-    double* xs = alloc<double>(n3);
-    double* vh = alloc<double>(n3);
-    double* wh = alloc<double>(n3);
+    Pair<double> B = allocPair<double>();
     ListsT<double> L[2] = {allocLists<double>(), allocLists<double>()};
     const int nseg = (nsteps + K - 1) / K;
     std::vector<State<double>> ck;
     std::vector<ListsT<double>> ckL;
-    start(S, L[0], kn, en, muc);
-    if (grads) {
+    Point<double> P = start(S, L[0], kn, en, muc);
+    auto checkpoint = [&](ListsT<double> const& lists) {
       ck.push_back(allocState<double>()); ckL.push_back(allocLists<double>());
-      copyState(ck[0], S); copyLists(ckL[0], L[0]);
-    }
+      stateOf(P, ck.back()); copyLists(ckL.back(), lists);
+    };
+    if (grads) checkpoint(L[0]);
     for (int s = 1; s <= nsteps; ++s) {
-      advance(S, xs, vh, wh, L[(s - 1) & 1], L[s & 1], kn, en, muc);
-      if (grads && s % K == 0 && s < nsteps) {
-        ck.push_back(allocState<double>()); ckL.push_back(allocLists<double>());
-        copyState(ck.back(), S); copyLists(ckL.back(), L[s & 1]);
-      }
+      advance(P, B.x[s & 1], B.v[s & 1], B.w[s & 1], L[(s - 1) & 1], L[s & 1], kn, en, muc);
+      if (grads && s % K == 0 && s < nsteps) checkpoint(L[s & 1]);
     }
+    State<double> E = allocState<double>();
+    stateOf(P, E);
     checkOverflow();
-    if (x_out) ACK(cudaMemcpy(x_out, S.x, n3 * sizeof(double), cudaMemcpyDeviceToHost));
-    if (v_out) ACK(cudaMemcpy(v_out, S.v, n3 * sizeof(double), cudaMemcpyDeviceToHost));
+    if (x_out) ACK(cudaMemcpy(x_out, E.x, n3 * sizeof(double), cudaMemcpyDeviceToHost));
+    if (v_out) ACK(cudaMemcpy(v_out, E.v, n3 * sizeof(double), cudaMemcpyDeviceToHost));
+    double* target = nullptr;
     if (tx && tv) {
+      target = targets(tx, tv);
       std::vector<double> per;
-      lossOf(S, tx, tv, per);
+      lossOf(E, target, per);
       double Ls = 0.;
       for (double a : per) Ls += a;
       if (loss) *loss = Ls;
     }
     if (!grads) return;
     // ------------------------------------------------------ reverse sweep
-    double *lx = alloc<double>(n3), *lv = alloc<double>(n3), *lw = alloc<double>(n3);
-    double *lF = alloc<double>(n3), *lT = alloc<double>(n3);
-    double *lvh = alloc<double>(n3), *lwh = alloc<double>(n3), *lp = alloc<double>(n3);
+    AdjState adj[2];
+    AdjHist hist[2];
     const size_t nh = (size_t)n * kAdjCap * 3, nwh = (size_t)n * kAdjWalls * 3;
-    double *lkd[2], *lpn[2], *lwkd[2], *lwpn[2];
     for (int k = 0; k < 2; ++k) {
-      lkd[k] = alloc<double>(nh); lpn[k] = alloc<double>(nh);
-      lwkd[k] = alloc<double>(nwh); lwpn[k] = alloc<double>(nwh);
-      ACK(cudaMemsetAsync(lkd[k], 0, nh * sizeof(double), st));
-      ACK(cudaMemsetAsync(lpn[k], 0, nh * sizeof(double), st));
-      ACK(cudaMemsetAsync(lwkd[k], 0, nwh * sizeof(double), st));
-      ACK(cudaMemsetAsync(lwpn[k], 0, nwh * sizeof(double), st));
+      for (double** a : {&adj[k].x, &adj[k].v, &adj[k].w, &adj[k].F, &adj[k].T})
+        *a = scratch<double>(n3);
+      hist[k].kd = scratch<double>(nh); hist[k].pn = scratch<double>(nh);
+      hist[k].wkd = scratch<double>(nwh); hist[k].wpn = scratch<double>(nwh);
     }
-    double* dtx = alloc<double>(n3);
-    double* dtv = alloc<double>(n3);
-    ACK(cudaMemcpyAsync(dtx, tx, n3 * sizeof(double), cudaMemcpyHostToDevice, st));
-    ACK(cudaMemcpyAsync(dtv, tv, n3 * sizeof(double), cudaMemcpyHostToDevice, st));
-    k_bwd_seed<<<nblk(n), 128, 0, st>>>(n, S.x, S.v, dtx, dtv, lx, lv);
-    for (double* z : {lw, lF, lT, lp}) ACK(cudaMemsetAsync(z, 0, n3 * sizeof(double), st));
+    double* lp = scratch<double>(n3);
+    // after the last step nothing depends on its history, w, F or T
+    for (double* z : {hist[0].kd, hist[0].pn}) ACK(cudaMemsetAsync(z, 0, nh * sizeof(double), st));
+    for (double* z : {hist[0].wkd, hist[0].wpn}) ACK(cudaMemsetAsync(z, 0, nwh * sizeof(double), st));
+    for (double* z : {adj[0].w, adj[0].F, adj[0].T, lp}) ACK(cudaMemsetAsync(z, 0, n3 * sizeof(double), st));
+    k_bwd_seed<<<nblk(n), 128, 0, st>>>(n, E.x, E.v, target, target + n3, adj[0].x, adj[0].v);
     // per-step storage of one segment
-    std::vector<double*> Xs(K + 1), Vh(K + 1), Wh(K + 1);
-    std::vector<ListsT<double>> Ls(K + 1);
-    for (int k = 0; k <= K; ++k) {
-      Xs[k] = alloc<double>(n3); Vh[k] = alloc<double>(n3); Wh[k] = alloc<double>(n3);
+    const int len = std::min(K, nsteps);
+    std::vector<double*> Xs(len + 1), Vh(len + 1), Wh(len + 1);
+    std::vector<ListsT<double>> Ls(len + 1);
+    for (int k = 1; k <= len; ++k) {
+      Xs[k] = scratch<double>(n3); Vh[k] = scratch<double>(n3); Wh[k] = scratch<double>(n3);
       Ls[k] = allocLists<double>();
     }
-    State<double> R = allocState<double>();
     int cur = 0;
     for (int seg = nseg - 1; seg >= 0; --seg) {
       const int c = seg * K, e = std::min(c + K, nsteps);
-      copyState(R, ck[seg]);
-      copyLists(Ls[0], ckL[seg]);
+      Ls[0] = ckL[seg];
+      // (the step's forces overwrite F, T: those of a checkpoint are not needed again)
+      Point<double> R{ck[seg].x, ck[seg].v, ck[seg].w, 1, ck[seg].F, ck[seg].Tq};
       for (int s = c + 1; s <= e; ++s)
         advance(R, Xs[s - c], Vh[s - c], Wh[s - c], Ls[s - c - 1], Ls[s - c], kn, en, muc);
       for (int s = e; s >= c + 1; --s) {
-        const int prv = cur ^ 1;
-        k_bwd_close<<<nblk(n), 128, 0, st>>>(n, A, d_type, lv, lw, lF, lT, lvh, lwh);
-        ACK(cudaMemsetAsync(lkd[prv], 0, nh * sizeof(double), st));
-        ACK(cudaMemsetAsync(lpn[prv], 0, nh * sizeof(double), st));
-        ACK(cudaMemsetAsync(lwkd[prv], 0, nwh * sizeof(double), st));
-        ACK(cudaMemsetAsync(lwpn[prv], 0, nwh * sizeof(double), st));
-        k_bwd_forces<<<nblk(n), 128, 0, st>>>(
-            n, A, d_type, Xs[s - c], Vh[s - c], Wh[s - c], Ls[s - c - 1], 1, Ls[s - c], lF, lT,
-            lkd[cur], lpn[cur], lwkd[cur], lwpn[cur], 0, lx, lvh, lwh, lkd[prv], lpn[prv],
-            lwkd[prv], lwpn[prv], lp, kn, en, muc);
-        k_bwd_move<<<nblk(n), 128, 0, st>>>(n, A, d_type, lx, lvh, lwh, lv, lw, lF, lT);
+        k_bwd_step<<<laneBlocks(), kAdjBlock, 0, st>>>(
+            n, A, d_type, Xs[s - c], Vh[s - c], Wh[s - c], Ls[s - c - 1], 1, Ls[s - c], adj[cur],
+            adj[cur ^ 1], hist[cur], hist[cur ^ 1], lp, kn, en, muc, 0);
         ACK(cudaGetLastError());
-        cur = prv;
+        cur ^= 1;
       }
     }
     // leapfrog start: forces at (x0, v0, w0), the spring it leaves is zeroed
-    ACK(cudaMemsetAsync(lvh, 0, n3 * sizeof(double), st));
-    ACK(cudaMemsetAsync(lwh, 0, n3 * sizeof(double), st));
-    {
-      const int prv = cur ^ 1;
-      k_bwd_forces<<<nblk(n), 128, 0, st>>>(
-          n, A, d_type, d_x0, d_v0, d_w0, ckL[0], 0, ckL[0], lF, lT, lkd[cur], lpn[cur],
-          lwkd[cur], lwpn[cur], 1, lx, lvh, lwh, lkd[prv], lpn[prv], lwkd[prv], lwpn[prv], lp,
-          kn, en, muc);
-      ACK(cudaGetLastError());
-    }
-    std::vector<double> hv(n3), hvh(n3), hp(n3);
-    ACK(cudaMemcpyAsync(hv.data(), lv, n3 * sizeof(double), cudaMemcpyDeviceToHost, st));
-    ACK(cudaMemcpyAsync(hvh.data(), lvh, n3 * sizeof(double), cudaMemcpyDeviceToHost, st));
+    k_bwd_step<<<laneBlocks(), kAdjBlock, 0, st>>>(n, A, d_type, d_x0, d_v0, d_w0, ckL[0], 0, ckL[0],
+                                                   adj[cur], adj[cur ^ 1], hist[cur], hist[cur ^ 1],
+                                                   lp, kn, en, muc, 1);
+    ACK(cudaGetLastError());
+    std::vector<double> hp(n3);
+    if (dLdv0) ACK(cudaMemcpyAsync(dLdv0, adj[cur ^ 1].v, n3 * sizeof(double), cudaMemcpyDeviceToHost, st));
     ACK(cudaMemcpyAsync(hp.data(), lp, n3 * sizeof(double), cudaMemcpyDeviceToHost, st));
     ACK(cudaStreamSynchronize(st));
     checkOverflow();
-    if (dLdv0)
-      for (size_t i = 0; i < n3; ++i) dLdv0[i] = hv[i] + hvh[i];
     if (dLdp) {
       dLdp[0] = dLdp[1] = dLdp[2] = 0.;
       for (int t = 0; t < n; ++t)
@@ -944,17 +1069,17 @@ struct AdjointSystem {
     if (seed_v && (seed_particle >= n || seed_component < 0 || seed_component > 2))
       throw std::runtime_error("seed out of range");
     if (!seed_v) { kn.d[0] = 1.; en.d[1] = 1.; muc.d[2] = 1.; }
-    const size_t n3 = 3 * (size_t)n;
     State<D> S = allocState<D>();
-    D* xs = alloc<D>(n3);
-    D* vh = alloc<D>(n3);
-    D* wh = alloc<D>(n3);
+    Pair<D> B = allocPair<D>();
     ListsT<D> L[2] = {allocLists<D>(), allocLists<D>()};
-    start(S, L[0], kn, en, muc, seed_v ? 3 * seed_particle + seed_component : -1);
-    for (int s = 1; s <= nsteps; ++s) advance(S, xs, vh, wh, L[(s - 1) & 1], L[s & 1], kn, en, muc);
+    Point<D> P = start(S, L[0], kn, en, muc, seed_v ? 3 * seed_particle + seed_component : -1);
+    for (int s = 1; s <= nsteps; ++s)
+      advance(P, B.x[s & 1], B.v[s & 1], B.w[s & 1], L[(s - 1) & 1], L[s & 1], kn, en, muc);
+    State<D> E = allocState<D>();
+    stateOf(P, E);
     checkOverflow();
     std::vector<D> per;
-    lossOf(S, tx, tv, per);
+    lossOf(E, targets(tx, tv), per);
     double Lv = 0., g[3] = {0., 0., 0.};
     for (auto const& a : per) {
       Lv += a.v;
