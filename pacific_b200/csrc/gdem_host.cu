@@ -32,6 +32,7 @@
 
 #include "../../include/grains_b200.h"
 #include "gdem_kernels.cuh"
+#include "gdem_divide.cuh"
 #include "gdem_setup.h"
 #include "xml_reader.hpp"
 
@@ -263,6 +264,15 @@ void polyMassProperties(PolyFile const& P, double& vol, double* Iv) {
   }
 }
 
+// Reciprocals of the FP64 leapfrog's divisors (divideBy).
+void setReciprocals(TypeDesc& t) {
+  t.rcp_mass_c = reciprocalFor(t.mass * t.coupling);
+  for (int d = 0; d < 3; ++d) {
+    t.rcp_inertia[d] = reciprocalFor(t.inertia[d]);
+    t.rcp_inertia_c[d] = reciprocalFor(t.coupling * t.inertia[d]);
+  }
+}
+
 InstanceDesc readInstance(std::string const& path) {
   auto doc = parseXmlFile(path);
   XmlNode const* root = doc.get();
@@ -374,6 +384,7 @@ InstanceDesc readInstance(std::string const& path) {
       t.inv_inertia[d] = 1. / t.inertia[d];
       t.inv_inertia_c[d] = t.inv_inertia[d];
     }
+    setReciprocals(t);
     t.eqrad = std::pow((0.75 / PI) * vol, 1. / 3.);                   // getEquivalentSphereRadius
     // crust shrink factors (RigidBodyWithCrust ctor, RigidBodyWithCrust.cpp:58-78)
     for (int d = 0; d < 3; ++d)
@@ -1718,6 +1729,7 @@ int gdem_set_fluid(gdem_handle h, double fluid_density, int corrected_accelerati
         if (corrected_acceleration) t.coupling -= fluid_density / t.density;
         t.inv_mass = 1. / (t.mass * t.coupling);
         for (int d = 0; d < 3; ++d) t.inv_inertia_c[d] = 1. / (t.coupling * t.inertia[d]);
+        setReciprocals(t);
       }
     // the kernels read the class table when they run: no graph to recapture
     CK(cudaMemcpy(s->d_types, s->h_types.data(), s->h_types.size() * sizeof(TypeDesc),

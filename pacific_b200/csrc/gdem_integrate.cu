@@ -381,10 +381,12 @@ template <bool kFast, bool kBasis>
 constexpr int kMoveBlock() { return kBasis ? 256 : 128; }
 
 // Leapfrog of each particle (128-thread blocks: FP32-split spheres eight per
-// multiprocessor at 64 registers, FP64 six at 80; both measured faster at 1M
-// than 256-thread blocks -- three, four or five per multiprocessor for
-// FP32-split, three or four for FP64; the kernel is bound by the latency of
-// its loads).  FP32-split with an orientation matrix: two 256-thread blocks.  With kStepSum the force and torque of this
+// multiprocessor at 64 registers; measured faster at 1M than 256-thread blocks
+// at three, four or five: it is bound by the latency of its loads.  FP64
+// spheres six at 80: 256,000 spheres 22.8 us, 22.1 with five, 22.4 with
+// seven, but a packed bed of 60,000 17.9 us against 16.9 and 18.7).  With an
+// orientation matrix: two 256-thread blocks, an instantiation of its own in
+// both modes (a convex FP64 pour's move 21.5 -> 13.8 us).  With kStepSum the force and torque of this
 // evaluation: the weight for a particle the contact filter did not mark as a
 // candidate, else the weight plus its shares (sumShares); without it, the
 // stored F, T (the opening kick of a call continues from the last evaluation
@@ -401,7 +403,7 @@ constexpr int kMoveBlock() { return kBasis ? 256 : 128; }
 // takes no share and is not read by the pair kernel, so its leapfrog runs at
 // once; a candidate waits for the pair kernel before it reads its shares.
 template <bool kFast, bool kBasis>
-__global__ void __launch_bounds__(kMoveBlock<kFast, kBasis>(), (kFast && kBasis) ? 2 : (kFast ? 8 : 6))
+__global__ void __launch_bounds__(kMoveBlock<kFast, kBasis>(), kBasis ? 2 : (kFast ? 8 : 6))
     k_move(DevState S, int flags) {
   int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= S.n) return;
@@ -981,7 +983,8 @@ void launch_move(DevState const& S, int flags, int fast, cudaStream_t st) {
   M.x2 = S.x; M.v2 = S.v; M.w2 = S.w; M.wbf2 = S.wbf; M.q2 = S.q; M.basis2 = S.basis;
   M.wrap2 = S.wrap;
   const int nb = blocks(S.n, 256);
-  if (!fast) launchAfterPrevious(k_move<false, false>, blocks(S.n, kMoveBlock<false, false>()), kMoveBlock<false, false>(), st, M, flags);   // basis tested at run time
+  if (!fast && S.basis) launchAfterPrevious(k_move<false, true>, nb, 256, st, M, flags);
+  else if (!fast) launchAfterPrevious(k_move<false, false>, blocks(S.n, kMoveBlock<false, false>()), kMoveBlock<false, false>(), st, M, flags);
   else if (S.basis) launchAfterPrevious(k_move<true, true>, nb, 256, st, M, flags);
   else launchAfterPrevious(k_move<true, false>, blocks(S.n, kMoveBlock<true, false>()), kMoveBlock<true, false>(), st, M, flags);
 }

@@ -14,48 +14,45 @@
 //     (Base/src/Cell.cpp:172-184, Base/src/LinkedCell.cpp:1502-1547).
 #pragma once
 #include "gdem_device.cuh"
+#include "gdem_divide.cuh"
 
 namespace gdem {
+
+__device__ __forceinline__ d3 divideBy(d3 a, double b, double rb) {
+  return mk(divideBy(a.x, b, rb), divideBy(a.y, b, rb), divideBy(a.z, b, rb));
+}
 
 // Angular acceleration in the body frame; the gyroscopic term for
 // non-spherical classes (predictor mode).
 __device__ __forceinline__ d3 dOmega(TypeDesc const& t, d3 tbf, d3 om) {
   const double c = t.coupling;
-  if (t.shape == 0)
-    return mk(tbf.x / (c * t.inertia[0]), tbf.y / (c * t.inertia[1]), tbf.z / (c * t.inertia[2]));
   const double* I = t.inertia;
-  return mk(tbf.x / (c * I[0]) + om.y * om.z * (I[1] - I[2]) / I[0],
-            tbf.y / (c * I[1]) + om.z * om.x * (I[2] - I[0]) / I[1],
-            tbf.z / (c * I[2]) + om.x * om.y * (I[0] - I[1]) / I[2]);
+  const double* rI = t.rcp_inertia;
+  const double* rIc = t.rcp_inertia_c;
+  return mk(divideBy(tbf.x, c * I[0], rIc[0]) + divideBy(om.y * om.z * (I[1] - I[2]), I[0], rI[0]),
+            divideBy(tbf.y, c * I[1], rIc[1]) + divideBy(om.z * om.x * (I[2] - I[0]), I[1], rI[1]),
+            divideBy(tbf.z, c * I[2], rIc[2]) + divideBy(om.x * om.y * (I[0] - I[1]), I[2], rI[2]));
 }
 
-// SSP-RK3 update of the body-fixed angular velocity over h.  For a sphere
-// the acceleration does not depend on omega, so K1 = K2 = K3 and one
-// evaluation gives the same bits as three.
+// Increment of the body-fixed angular velocity over h: SSP-RK3.
 __device__ __forceinline__ d3 rk3(TypeDesc const& t, d3 tbf, d3 wbf, double h) {
-  if (t.shape == 0) {
-    d3 K = dOmega(t, tbf, wbf);
-    K = K * h;
-    return wbf + ((K + K) + 4. * K) / 6.;
-  }
   d3 K1 = dOmega(t, tbf, wbf);
   K1 = K1 * h;
   d3 K2 = dOmega(t, tbf, wbf + K1);
   K2 = K2 * h;
   d3 K3 = dOmega(t, tbf, wbf + 0.25 * (K1 + K2));
   K3 = K3 * h;
-  return wbf + ((K1 + K2) + 4. * K3) / 6.;
+  return divideBy((K1 + K2) + 4. * K3, 6., 1. / 6.);
 }
-
-// advanceVelocity: v, w_bf (and the space-frame w) over h.
-__device__ __forceinline__ void kick(TypeDesc const& tp, d3 F, d3 T, d3& v, d3& wbf, d3& w,
-                                     dq q, double h) {
-  dq pc = conj(q);
-  d3 tbf = multToVector3(pc, vecq(T, q));
-  const double c = tp.coupling;
-  v = v + (F / (tp.mass * c)) * h;
-  wbf = rk3(tp, tbf, wbf, h);
-  w = multToVector3(q, vecq(wbf, pc));
+// The same for a sphere: the acceleration does not depend on omega, so
+// K1 = K2 = K3 and one evaluation gives the same bits as three.
+__device__ __forceinline__ d3 rk3Sphere(TypeDesc const& t, d3 tbf, double h) {
+  const double c = t.coupling;
+  d3 K = mk(divideBy(tbf.x, c * t.inertia[0], t.rcp_inertia_c[0]),
+            divideBy(tbf.y, c * t.inertia[1], t.rcp_inertia_c[1]),
+            divideBy(tbf.z, c * t.inertia[2], t.rcp_inertia_c[2]));
+  K = K * h;
+  return divideBy((K + K) + 4. * K, 6., 1. / 6.);
 }
 
 // Signed periodic wrap counts, one byte per axis.
@@ -191,31 +188,43 @@ __device__ __forceinline__ void leapfrogSphere(TypeDesc const& tp, d3 F, d3 T, b
 }
 
 // One particle's leapfrog: optionally the closing kick of the previous step
-// (with this step's F, T over hc), then optionally the opening kick over h
+// (with this step's F, T over h), then optionally the opening kick over h
 // and the drift over dt with the quaternion and orientation update.
 // basis: 9 entries (row-major) or null.  dx receives the translation.
-template <bool kFast>
-__device__ __forceinline__ void leapfrog(TypeDesc const& tp, d3 F, d3 T, bool close, double hc,
-                                         bool move, double h, double dt, d3& x, d3& v,
-                                         d3& wbf, d3& w, dq& q, double* basis, d3& dx,
-                                         int* status) {
-  if (close) {
-    if (kFast) kickFast(tp, F, T, v, wbf, w, q, hc);
-    else kick(tp, F, T, v, wbf, w, q, hc);
-  }
-  dx = mk(0., 0., 0.);
-  if (!move) return;
+// kSphere: every class of the system is a sphere.
+template <bool kFast, bool kSphere>
+__device__ __forceinline__ void leapfrog(TypeDesc const& tp, d3 F, d3 T, bool close, bool move,
+                                         double h, double dt, d3& x, d3& v, d3& wbf, d3& w, dq& q,
+                                         double* basis, d3& dx, int* status) {
   dq pc = conj(q);
-  d3 tbf = multToVector3(pc, vecq(T, q));
-  const double c = tp.coupling;
-  if (kFast) {
+  if constexpr (kFast) {
+    if (close) kickFast(tp, F, T, v, wbf, w, q, h);
+    dx = mk(0., 0., 0.);
+    if (!move) return;
+    const d3 tbf = multToVector3(pc, vecq(T, q));
     v = v + F * (h * tp.inv_mass);
     wbf = rk3Fast(tp, tbf, wbf, h);
   } else {
-    v = v + (F / (tp.mass * c)) * h;
+    // SecondOrderLeapFrog::advanceVelocity, once per kick: both kicks see the
+    // same F, T and q, so what depends on these alone is computed once (and,
+    // for a sphere, the whole increment of the angular velocity)
+    const d3 tbf = multToVector3(pc, vecq(T, q));
+    const d3 dv = divideBy(F, tp.mass * tp.coupling, tp.rcp_mass_c) * h;
+    if (kSphere || tp.shape == 0) {
+      const d3 dw = rk3Sphere(tp, tbf, h);
+      if (close) { v = v + dv; wbf = wbf + dw; }
+      if (move) { v = v + dv; wbf = wbf + dw; }
+    } else {
+      if (close) { v = v + dv; wbf = wbf + rk3(tp, tbf, wbf, h); }
+      if (move) { v = v + dv; wbf = wbf + rk3(tp, tbf, wbf, h); }
+    }
+    dx = mk(0., 0., 0.);
+    if (!move) {
+      if (close) w = multToVector3(q, vecq(wbf, pc));
+      return;
+    }
   }
   dx = v * dt;
-  if (!kFast) wbf = rk3(tp, tbf, wbf, h);
   w = multToVector3(q, vecq(wbf, pc));
   const d3 meanw = w;     // same expression as w (ParticleKinematics.cpp:79-82)
   x = x + dx;
@@ -271,11 +280,9 @@ __device__ __forceinline__ void loadMoveIn(DevState const& S, int t, MoveIn& m) 
   m.x = ld3(S.x, cap, t); m.v = ld3(S.v, cap, t); m.w = ld3(S.w, cap, t);
   m.wbf = kSphereW ? mk(0., 0., 0.) : ld3(S.wbf, cap, t);
   m.q = qmk(mk(S.q[t], S.q[cap + t], S.q[2 * cap + t]), S.q[3 * cap + t]);
-  // FP32-split: the basis array exists only in the instantiation for
-  // systems that carry one (convex bodies), a compile-time choice that keeps
-  // it in registers.  FP64: one instantiation tests for it at run time, in
-  // advanceParticle (the faster of the two on B200 for that path, measured).
-  if constexpr (kFast && kBasis) {
+  // the orientation matrix exists only in the instantiation for systems that
+  // carry one (convex bodies), a compile-time choice that keeps it in registers
+  if constexpr (kBasis) {
 #pragma unroll
     for (int k = 0; k < 9; ++k) m.bas[k] = S.basis[k * cap + t];
   }
@@ -297,19 +304,12 @@ __device__ __forceinline__ void advanceParticle(DevState const& S, int t, TypeDe
   d3 x = m.x, v = m.v, w = m.w, wbf = m.wbf;
   dq q = m.q;
   double* bas = m.bas;
-  double* bp = nullptr;
-  if constexpr (kFast) {
-    if constexpr (kBasis) bp = bas;
-  } else if (S.basis) {
-#pragma unroll
-    for (int k = 0; k < 9; ++k) bas[k] = S.basis[k * cap + t];
-    bp = bas;
-  }
+  double* bp = kBasis ? bas : nullptr;
   d3 dx;
   if constexpr (kSphereW)
     leapfrogSphere(tp, F, T, close, 0.5 * dt, move, 0.5 * dt, dt, x, v, w, q, dx, S.status);
   else
-    leapfrog<kFast>(tp, F, T, close, 0.5 * dt, move, 0.5 * dt, dt, x, v, wbf, w, q, bp, dx, S.status);
+    leapfrog<kFast, !kBasis>(tp, F, T, close, move, 0.5 * dt, dt, x, v, wbf, w, q, bp, dx, S.status);
   int wr = m.wrap;
   if (move) {
     int wd[3];
@@ -321,7 +321,7 @@ __device__ __forceinline__ void advanceParticle(DevState const& S, int t, TypeDe
   st3(S.x2, cap, t, x); st3(S.v2, cap, t, v); st3(S.w2, cap, t, w);
   if (!kSphereW) st3(S.wbf2, cap, t, wbf);
   S.q2[t] = q.v.x; S.q2[cap + t] = q.v.y; S.q2[2 * cap + t] = q.v.z; S.q2[3 * cap + t] = q.w;
-  if (bp) {
+  if constexpr (kBasis) {
 #pragma unroll
     for (int k = 0; k < 9; ++k) S.basis2[k * cap + t] = bas[k];
   }

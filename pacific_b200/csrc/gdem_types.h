@@ -92,6 +92,9 @@ struct TypeDesc {
   // fluid-corrected acceleration, else 1; the kicks divide by m c and c I
   double coupling;
   double inv_inertia_c[3];   // 1 / (c inertia) (FP32-split leapfrog)
+  // correctly rounded reciprocals of the FP64 leapfrog's divisors mass c,
+  // inertia and c inertia (divideBy; 0: divide by them instead)
+  double rcp_mass_c, rcp_inertia[3], rcp_inertia_c[3];
 };
 
 // HookeMemory / Hooke parameters (HookeMemoryContactForceModel.cpp:12-27).
