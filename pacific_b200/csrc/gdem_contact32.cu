@@ -154,16 +154,6 @@ __device__ __forceinline__ void hodc32(ModelDesc const& m, float kn, float beta,
 
 __device__ __forceinline__ float3 tof(d3 a) { return f3((float)a.x, (float)a.y, (float)a.z); }
 
-__device__ __forceinline__ void loadHistF(HistTable const& t, int slot, float3& kd, float3& pn, float3& sp) {
-  const float* v = static_cast<const float*>(t.vals) + 9 * (size_t)slot;
-  kd = f3(v[0], v[1], v[2]); pn = f3(v[3], v[4], v[5]); sp = f3(v[6], v[7], v[8]);
-}
-__device__ __forceinline__ void storeHistF(HistTable const& t, int slot, float3 kd, float3 pn, float3 sp) {
-  float* v = static_cast<float*>(t.vals) + 9 * (size_t)slot;
-  v[0] = kd.x; v[1] = kd.y; v[2] = kd.z; v[3] = pn.x; v[4] = pn.y; v[5] = pn.z;
-  v[6] = sp.x; v[7] = sp.y; v[8] = sp.z;
-}
-
 // Hooke law (no tangential memory) in FP32, seen from p0 (same structure as
 // hooke64).  lev0 / lev1 are the contact point relative to p0 / p1; w0, w1
 // the space-fixed angular velocities.
@@ -315,37 +305,28 @@ __global__ void __launch_bounds__(256) k_pairs_fill32(DevState S, const int* gat
 // One pair in the canonical orientation -- p0 (slot s0, the lower ID) at its
 // own position, p1 at its periodic image seen from p0 -- with the exact
 // narrow phase on the FP64 master positions, the FP32 law (FP64 when
-// ill-conditioned) and the contact history (the new entry written when
-// insert).  Returns true for a contact, with the force f on p0, the torques
+// ill-conditioned) and the contact memory (entry c of the pair list's,
+// written back).  Returns true for a contact, with the force f on p0, the torques
 // c0 = lev0 x f and c1 = lev1 x f of the lever arms from p0 and p1, and the
 // rolling torque mr (rolling: the model has rolling resistance); delta gets
 // the overlap (+inf without contact).  kConvex: some class is not a sphere,
 // so the GJK narrow phase is compiled in (it is kept out of the sphere-only
 // kernel, whose registers it would triple).
 template <bool kConvex>
-__device__ __forceinline__ bool evalPair32(DevState const& S, GridDesc const& g, int s0, int s1,
+__device__ __forceinline__ bool evalPair32(DevState const& S, GridDesc const& g, int c, int s0, int s1,
                                            int prio0, int prio1, int id0, int id1,
                                            TypeDesc const& tp0,
                                            TypeDesc const& tp1, d3 x0, d3 x1, d3 v0, d3 v1,
-                                           d3 w0, d3 w1, bool insert, int& nlaw, int& nre,
+                                           d3 w0, d3 w1, int& nlaw, int& nre,
                                            GjkTally& gjk, double& delta, float3& f, float3& c0,
                                            float3& c1, float3& mr, bool& rolling) {
   const int cap = S.cap;
-  const unsigned tag = (unsigned)S.ctl[kCtlEpoch], tag_old = tag - 1u;
-  // spheres: the history lookup's first probe (key and values) is read
-  // before the narrow phase -- the key depends on the two IDs only -- so its
-  // loads overlap the narrow phase
-  const unsigned long long hkey = pairKey(min(id0, id1), max(id0, id1));
-  uint32_t hslot = 0;
-  unsigned long long hfirst = 0;
+  const int now = S.ctl[kCtlEpoch];
+  // spheres: the pair's memory is read before the narrow phase, so that its
+  // loads overlap it
   float hv[9];
-  if constexpr (!kConvex) {
-    hslot = hashSlot(hkey, S.hist_old.log2cap);
-    hfirst = S.hist_old.keys[hslot];
-    const float* p = static_cast<const float*>(S.hist_old.vals) + 9 * (size_t)hslot;
-#pragma unroll
-    for (int k = 0; k < 9; ++k) hv[k] = p[k];
-  }
+  int written = -1;
+  if constexpr (!kConvex) written = memLoad(S.pmem, c, hv, false);
   Contact64 ct;
   if (!kConvex || (tp0.shape == 0 && tp1.shape == 0)) {
     ct = sphereSphere64(x0, tp0.radius, tp0.crust, x1, tp1.radius, tp1.crust);
@@ -359,7 +340,7 @@ __device__ __forceinline__ bool evalPair32(DevState const& S, GridDesc const& g,
       recordVertex(S, tp0, s0, prio0, c0v);
       recordVertex(S, tp1, s1, prio1, c1v);
     }
-    if (insert) gjk.add(ct.gjk_iters);   // each pair counted once
+    gjk.add(ct.gjk_iters);
   }
   delta = ct.contact && ct.dist < 0. ? ct.dist : __longlong_as_double(0x7ff0000000000000ll);
   if (!ct.contact || !(ct.dist < 0.)) return false;
@@ -372,39 +353,28 @@ __device__ __forceinline__ bool evalPair32(DevState const& S, GridDesc const& g,
   const Body64 b1{x1, v1, w1, tp1.mass, tp1.eqrad};
   float3 kd = f3(0.f, 0.f, 0.f), pn = kd, sp = kd;
   int re;
-  if (insert) ++nlaw;   // each pair counted once, by its lower ID
+  ++nlaw;
   if (m.memory) {
-    // the table holds the lower ID's view; p0 may be the higher ID (the
+    // the memory is the lower ID's view; p0 may be the higher ID (the
     // reference's pair orientation), whose view is the negation
     const bool flip = id0 > id1;
-    const unsigned long long key = hkey;
-    int old;
-    if constexpr (!kConvex) {
-      if (hfirst == tagged(key, tag_old)) old = (int)hslot;
-      else if (tagOf(hfirst) != (tag_old & kTagMask)) old = -1;
-      else old = histFindAfter(S.hist_old, key, tag_old, hslot);
-    } else {
-      old = histFind(S.hist_old, key, tag_old);
+    const bool spring = m.rolling != 0;
+    if (kConvex || spring) written = memLoad(S.pmem, c, hv, spring);
+    const bool existed = remembered(S, written, now);
+    if (existed) {
+      const float sg = flip ? -1.f : 1.f;
+      kd = f3(sg * hv[0], sg * hv[1], sg * hv[2]);
+      pn = f3(sg * hv[3], sg * hv[4], sg * hv[5]);
+      sp = f3(sg * hv[6], spring ? sg * hv[7] : 0.f, spring ? sg * hv[8] : 0.f);
     }
-    if (old >= 0) {
-      if (!kConvex && old == (int)hslot) {
-        kd = f3(hv[0], hv[1], hv[2]); pn = f3(hv[3], hv[4], hv[5]); sp = f3(hv[6], hv[7], hv[8]);
-      } else {
-        loadHistF(S.hist_old, old, kd, pn, sp);
-      }
-      if (flip) { kd = -kd; pn = -pn; sp = -sp; }
-    }
-    contactLaw32(m, S.dt, ct, b0, b1, old >= 0, kd, pn, sp, f, mr, re);
-    if (insert) {
-      int slot = histInsert(S.hist_new, key, tag);
-      if (slot < 0) raise(S.status, kErrHashFull);
-      else if (flip) storeHistF(S.hist_new, slot, -kd, -pn, -sp);
-      else storeHistF(S.hist_new, slot, kd, pn, sp);
-    }
+    contactLaw32(m, S.dt, ct, b0, b1, existed, kd, pn, sp, f, mr, re);
+    if (flip) { kd = -kd; pn = -pn; sp = -sp; }
+    const float out[9] = {kd.x, kd.y, kd.z, pn.x, pn.y, pn.z, sp.x, sp.y, sp.z};
+    memStore(S.pmem, c, out, now, spring || !existed);
   } else {
     contactLaw32(m, S.dt, ct, b0, b1, false, kd, pn, sp, f, mr, re);
   }
-  if (insert) nre += re;
+  nre += re;
   c0 = crossf(lev0, f);
   c1 = crossf(lev1, f);
   rolling = m.rolling != 0;
@@ -422,91 +392,126 @@ __device__ __forceinline__ void storeShare32(DevState const& S, int64_t entry, i
   sh[1] = make_float4(c.x, c.y, c.z, 0.f);
 }
 
-// The wall contacts of particle t (near a wall per the contact filter): the
-// geometry from the FP64 position, the force law in FP32 (FP64 when
-// ill-conditioned); their sum is the particle's wall share.
+// Contact of particle t (class ta, row of the wall list) with wall k of its
+// instance: the geometry from the FP64 position, the force law in FP32 (FP64
+// when ill-conditioned).  Returns true for a contact, with its force f, the
+// lever arm's torque c and, with a rolling model (rolling), the rolling
+// torque mr.
 template <bool kConvex>
-__device__ __forceinline__ void wallsOf32(DevState const& S, int t, int tag, int& nlaw, int& nre,
-                                          GjkTally& gjk, StatsTally& st) {
+__device__ __forceinline__ bool wallContact32(DevState const& S, GridDesc const& g, int row, int t,
+                                              int k, TypeDesc const& ta, d3 xt, d3 vt, d3 wt,
+                                              int& curw, bool& walls_gjk, int& nlaw, int& nre,
+                                              GjkTally& gjk, StatsTally& st, float3& f, float3& c,
+                                              float3& mr, bool& rolling) {
   const int cap = S.cap;
-  const int inst = S.inst[t];
-  GridDesc const& g = S.grids[inst];
-  const unsigned utag = (unsigned)tag, tag_old = utag - 1u;
-  const int ida = S.id[t];
-  TypeDesc const& ta = S.types[S.type[t]];
-  const d3 xt = ld3(S.x, cap, t), vt = ld3(S.v, cap, t), wt = ld3(S.w, cap, t);
-  float3 Fw = f3(0.f, 0.f, 0.f), Tw = f3(0.f, 0.f, 0.f);
-  bool any = false;
-  // the particle's polyhedron vertex runs through its wall calls in order
-  int curw = kConvex ? startVertex(S, ta, t) : 0;
-  bool walls_gjk = false;
-  for (int k = 0; k < g.wall_count; ++k) {
-    WallDesc const& wd = S.walls[g.wall_begin + k];
-    if (kConvex && ta.shape != 0) {
-      // the shrunk body lies inside its circumscribed sphere and the shrunk
-      // wall inside the wall's box: when the sphere is farther from the box
-      // than the two crusts (with a margin far above the rounding), the
-      // closest-point search would decide "no contact"; skip it
-      double d2 = 0.;
+  WallDesc const& wd = S.walls[g.wall_begin + k];
+  if (kConvex && ta.shape != 0) {
+    // the shrunk body lies inside its circumscribed sphere and the shrunk
+    // wall inside the wall's box: when the sphere is farther from the box
+    // than the two crusts (with a margin far above the rounding), the
+    // closest-point search would decide "no contact"; skip it
+    double d2 = 0.;
 #pragma unroll
-      for (int d = 0; d < 3; ++d) {
-        const double c = d == 0 ? xt.x : (d == 1 ? xt.y : xt.z);
-        const double e = fabs(c - wd.centre[d]) - wd.extent[d];
-        if (e > 0.) d2 += e * e;
-      }
-      const double lim = (ta.radius + ta.crust + wd.crust) * (1. + 1.e-9);
-      if (d2 > lim * lim) {
-        if (S.diag) S.wall_delta[(size_t)t * S.max_walls + k] = __longlong_as_double(0x7ff0000000000000ll);
-        continue;
-      }
+    for (int d = 0; d < 3; ++d) {
+      const double x = d == 0 ? xt.x : (d == 1 ? xt.y : xt.z);
+      const double e = fabs(x - wd.centre[d]) - wd.extent[d];
+      if (e > 0.) d2 += e * e;
     }
-    int cw = 0;
-    Contact64 ct = (!kConvex || ta.shape == 0)
-        ? sphereWall64(xt, ta.radius, ta.crust, wd)
-        : convexContact64(convexOf(ta, S), crustXForm(S.basis, cap, t, ta.scaling, xt),
-                          ta.radius, ta.crust, convexOf(wd),
-                          identityXForm(wd.scaling, mk(wd.centre[0], wd.centre[1], wd.centre[2])),
-                          wd.radius, wd.crust, curw, cw, true);
-    if (kConvex) gjk.add(ct.gjk_iters);
-    if (kConvex && ct.gjk_iters > 0) walls_gjk = true;
-    if (S.diag) S.wall_delta[(size_t)t * S.max_walls + k] = ct.contact ? ct.dist : __longlong_as_double(0x7ff0000000000000ll);
-    if (ct.error) raise(S.status, kErrContactOverlap);
-    if (!ct.contact || !(ct.dist < 0.)) continue;
-    st.add(ct.dist);
-    ModelDesc const& m = S.models[g.model_base + ta.mat * kMaxMat + wd.mat];
-    const float3 lev0 = tof(ct.point - xt);
-    const d3 zero = mk(0., 0., 0.);
-    const Body64 b0{xt, vt, wt, ta.mass, ta.eqrad};
-    const Body64 b1{mk(wd.centre[0], wd.centre[1], wd.centre[2]), zero, zero, 1.e20, wd.eqrad};
-    float3 f, mr, kd = f3(0.f, 0.f, 0.f), pn = kd, sp = kd;
-    int re;
-    ++nlaw;
-    if (m.memory) {
-      const unsigned long long key = wallKey(ida, k);
-      int old = histFind(S.hist_old, key, tag_old);
-      if (old >= 0) loadHistF(S.hist_old, old, kd, pn, sp);
-      contactLaw32(m, S.dt, ct, b0, b1, old >= 0, kd, pn, sp, f, mr, re);
-      int slot = histInsert(S.hist_new, key, utag);
-      if (slot < 0) raise(S.status, kErrHashFull);
-      else storeHistF(S.hist_new, slot, kd, pn, sp);
-    } else {
-      contactLaw32(m, S.dt, ct, b0, b1, false, kd, pn, sp, f, mr, re);
+    const double lim = (ta.radius + ta.crust + wd.crust) * (1. + 1.e-9);
+    if (d2 > lim * lim) {
+      if (S.diag) S.wall_delta[(size_t)t * S.max_walls + k] = __longlong_as_double(0x7ff0000000000000ll);
+      return false;
     }
-    nre += re;
-    if (S.diag) {
-      double* fd = S.wall_force + 3 * ((size_t)t * S.max_walls + k);
-      fd[0] = f.x; fd[1] = f.y; fd[2] = f.z;
-    }
-    Fw = Fw + f;
-    Tw = Tw + crossf(lev0, f);
-    if (m.rolling) Tw = Tw + mr;
-    any = true;
   }
-  if (walls_gjk) recordVertex(S, ta, t, kWallPriority, curw);
+  int cw = 0;
+  Contact64 ct = (!kConvex || ta.shape == 0)
+      ? sphereWall64(xt, ta.radius, ta.crust, wd)
+      : convexContact64(convexOf(ta, S), crustXForm(S.basis, cap, t, ta.scaling, xt),
+                        ta.radius, ta.crust, convexOf(wd),
+                        identityXForm(wd.scaling, mk(wd.centre[0], wd.centre[1], wd.centre[2])),
+                        wd.radius, wd.crust, curw, cw, true);
+  if (kConvex) gjk.add(ct.gjk_iters);
+  if (kConvex && ct.gjk_iters > 0) walls_gjk = true;
+  if (S.diag) S.wall_delta[(size_t)t * S.max_walls + k] = ct.contact ? ct.dist : __longlong_as_double(0x7ff0000000000000ll);
+  if (ct.error) raise(S.status, kErrContactOverlap);
+  if (!ct.contact || !(ct.dist < 0.)) return false;
+  st.add(ct.dist);
+  ModelDesc const& m = S.models[g.model_base + ta.mat * kMaxMat + wd.mat];
+  const float3 lev0 = tof(ct.point - xt);
+  const d3 zero = mk(0., 0., 0.);
+  const Body64 b0{xt, vt, wt, ta.mass, ta.eqrad};
+  const Body64 b1{mk(wd.centre[0], wd.centre[1], wd.centre[2]), zero, zero, 1.e20, wd.eqrad};
+  float3 kd = f3(0.f, 0.f, 0.f), pn = kd, sp = kd;
+  int re;
+  ++nlaw;
+  if (m.memory) {
+    const int now = S.ctl[kCtlEpoch];
+    const long long at = (long long)row * S.max_walls + k;
+    const bool spring = m.rolling != 0;
+    float hv[9];
+    const bool existed = remembered(S, memLoad(S.wmem, at, hv, spring), now);
+    if (existed) {
+      kd = f3(hv[0], hv[1], hv[2]); pn = f3(hv[3], hv[4], hv[5]);
+      sp = f3(hv[6], spring ? hv[7] : 0.f, spring ? hv[8] : 0.f);
+    }
+    contactLaw32(m, S.dt, ct, b0, b1, existed, kd, pn, sp, f, mr, re);
+    const float out[9] = {kd.x, kd.y, kd.z, pn.x, pn.y, pn.z, sp.x, sp.y, sp.z};
+    memStore(S.wmem, at, out, now, spring || !existed);
+  } else {
+    contactLaw32(m, S.dt, ct, b0, b1, false, kd, pn, sp, f, mr, re);
+  }
+  nre += re;
+  if (S.diag) {
+    double* fd = S.wall_force + 3 * ((size_t)t * S.max_walls + k);
+    fd[0] = f.x; fd[1] = f.y; fd[2] = f.z;
+  }
+  c = crossf(lev0, f);
+  rolling = m.rolling != 0;
+  return true;
+}
+
+// One wall item of the evaluation: a (particle, wall) slot of the wall list
+// (spheres), whose contact is its share, or a particle of it, whose walls are
+// taken in order and summed into its first slot's share.  (A sphere in an edge
+// or corner used to take its walls in turn: their laws' latencies added up.)
+template <bool kConvex>
+__device__ __forceinline__ void wallItem32(DevState const& S, int item, int tag, int& nlaw, int& nre,
+                                           GjkTally& gjk, StatsTally& st) {
+  const int row = kConvex ? item : item / S.max_walls;
+  const int t = S.wlist[row];
+  GridDesc const& g = S.grids[S.inst[t]];
+  TypeDesc const& ta = S.types[S.type[t]];
+  const d3 xt = ld3(S.x, S.cap, t), vt = ld3(S.v, S.cap, t), wt = ld3(S.w, S.cap, t);
+  float3 f, c, mr;
+  bool rolling = false, any = false, walls_gjk = false;
+  int curw = 0;
+  if constexpr (kConvex) {
+    // the particle's polyhedron vertex runs through its wall calls in order
+    curw = startVertex(S, ta, t);
+    float3 Fw = f3(0.f, 0.f, 0.f), Tw = f3(0.f, 0.f, 0.f);
+    for (int k = 0; k < g.wall_count; ++k) {
+      if (!wallContact32<kConvex>(S, g, row, t, k, ta, xt, vt, wt, curw, walls_gjk, nlaw, nre, gjk,
+                                  st, f, c, mr, rolling))
+        continue;
+      Fw = Fw + f;
+      Tw = Tw + c;
+      if (rolling) Tw = Tw + mr;
+      any = true;
+    }
+    if (walls_gjk) recordVertex(S, ta, t, kWallPriority, curw);
+    f = Fw;
+    c = Tw;
+    rolling = false;
+    item = row * S.max_walls;
+  } else {
+    any = wallContact32<kConvex>(S, g, row, t, item - row * S.max_walls, ta, xt, vt, wt, curw,
+                                 walls_gjk, nlaw, nre, gjk, st, f, c, mr, rolling);
+  }
   if (!any) return;
-  float4* ws = static_cast<float4*>(S.wshare) + 2 * (size_t)t;
-  ws[0] = make_float4(Fw.x, Fw.y, Fw.z, 0.f);
-  ws[1] = make_float4(Tw.x, Tw.y, Tw.z, 0.f);
+  float4* ws = static_cast<float4*>(S.wshare) + (size_t)kWallShare32 * item;
+  ws[0] = make_float4(f.x, f.y, f.z, __int_as_float(tag));
+  ws[1] = make_float4(c.x, c.y, c.z, rolling ? 1.f : 0.f);
+  if (rolling) ws[2] = make_float4(mr.x, mr.y, mr.z, 0.f);
   atomicOr(reinterpret_cast<unsigned*>(&contactFlags(S)[t]), kNearWall);
 }
 
@@ -558,8 +563,8 @@ __device__ __forceinline__ void pairItem32(DevState const& S, int c, int tag, in
   double dl;
   bool rolling;
   const bool hit = evalPair32<kConvex>(
-      S, g, a, b, pa, pb, flip ? idu : idt, flip ? idt : idu, S.types[flip ? tyu : tyt], S.types[flip ? tyt : tyu],
-      flip ? xu : xt, flip ? xt + (-shift) : xu + shift, vt, vu, wt, wu, true, nlaw, nre, gjk, dl, f, c0, c1, mr, rolling);
+      S, g, c, a, b, pa, pb, flip ? idu : idt, flip ? idt : idu, S.types[flip ? tyu : tyt], S.types[flip ? tyt : tyu],
+      flip ? xu : xt, flip ? xt + (-shift) : xu + shift, vt, vu, wt, wu, nlaw, nre, gjk, dl, f, c0, c1, mr, rolling);
   const int64_t rt = (int64_t)offt + et, ru = (int64_t)offu + eu;
   // force on t (the lower ID) and the two torques
   const float3 mt = rolling ? mr : f3(0.f, 0.f, 0.f);
@@ -672,8 +677,15 @@ __global__ void __launch_bounds__(128) k_pairsep32(DevState S) {
 // grid: first the pairs the contact filter kept, then the particles near a
 // wall.  Its trigger comes after its wait, so the leapfrog kernel, which
 // starts at the trigger, sees the filter's candidate marks complete.
+// What bounds the sphere kernel is latency: about 1,350 instructions per
+// contact in chains of divisions and square roots at 10 to 12 warps per
+// multiprocessor (issue slots 23 % busy, DRAM 5 % on a packed bed).  With the
+// memory in the pair list instead of a hash table and the wall slots as items
+// of their own, a bed of 250,000 spheres took 277 -> 155 us at two resident
+// blocks (174 registers), 111 us at three (168, the cap here; four, 128
+// registers with spills, 111 us there and 16.7 against 15.4 us at 7,777).
 template <bool kConvex>
-__global__ void __launch_bounds__(128) k_pairlaw32(DevState S) {
+__global__ void __launch_bounds__(128, kConvex ? 1 : 3) k_pairlaw32(DevState S) {
   pdlWait();      // the contact filter's lists
   pdlTrigger();   // the leapfrog kernel may start; its candidates wait for this kernel
   // the pairs in contact at the last evaluation (all kept pairs, without
@@ -689,7 +701,7 @@ __global__ void __launch_bounds__(128) k_pairlaw32(DevState S) {
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < nk + nw; i += stride) {
     if (i < nh) pairItem32<kConvex>(S, S.kept[i], tag, nlaw, nre, gjk, st);
     else if (i < nk) pairItem32<kConvex>(S, S.kept2[i - nh], tag, nlaw, nre, gjk, st);
-    else wallsOf32<kConvex>(S, S.work[i - nk], tag, nlaw, nre, gjk, st);
+    else wallItem32<kConvex>(S, S.work[i - nk], tag, nlaw, nre, gjk, st);
   }
   // warp-aggregated counters (every lane of the warp reaches this point)
   const int wl = __reduce_add_sync(0xffffffffu, nlaw), wr = __reduce_add_sync(0xffffffffu, nre);
@@ -717,7 +729,7 @@ void launch_pairsep32(DevState const& S, cudaStream_t st) {
 }
 void launch_pairlaw32(DevState const& S, cudaStream_t st) {
   if (!S.n) return;
-  const int grid = (S.forces_bps > 0 ? S.forces_bps : 4) * S.nsm;
+  const int grid = (S.forces_bps > 0 ? S.forces_bps : (S.any_convex ? 4 : 3)) * S.nsm;
   if (S.any_convex) launchAfterPrevious(k_pairlaw32<true>, grid, 128, st, S);
   else launchAfterPrevious(k_pairlaw32<false>, grid, 128, st, S);
 }

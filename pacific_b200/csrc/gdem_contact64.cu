@@ -77,49 +77,30 @@ __global__ void __launch_bounds__(256) k_pairs_fill64(DevState S, const int* gat
   appendUpperPairs(S, t, valid ? S.pairs + S.pair_off[t] : S.pairs, nu, S.status);
 }
 
-__device__ __forceinline__ void loadHist(HistTable const& t, int slot, d3& kd, d3& pn, d3& sp) {
-  const double* v = static_cast<const double*>(t.vals) + 9 * (size_t)slot;
-  kd = mk(v[0], v[1], v[2]); pn = mk(v[3], v[4], v[5]); sp = mk(v[6], v[7], v[8]);
-}
-__device__ __forceinline__ void storeHist(HistTable const& t, int slot, d3 kd, d3 pn, d3 sp) {
-  double* v = static_cast<double*>(t.vals) + 9 * (size_t)slot;
-  v[0] = kd.x; v[1] = kd.y; v[2] = kd.z; v[3] = pn.x; v[4] = pn.y; v[5] = pn.z;
-  v[6] = sp.x; v[7] = sp.y; v[8] = sp.z;
-}
-
 // One pair in the canonical orientation -- p0 (slot s0, the lower ID) at its
 // own position, p1 at its periodic image seen from p0 -- with the
 // reference's expressions (closest points, Hooke / HookeMemory) and the
-// contact history (the new entry written when insert).  Returns true for a
+// contact memory (entry c of the pair list's, written back).  Returns true for a
 // contact, with the force f on p0, the torques c0 = (point - x0) x f and
 // c1m = (point - x1) x (-f) of p0 and p1, and the rolling torque mr
 // (rolling: the model has rolling resistance); delta gets the distance
 // (+inf without contact).  kConvex: some class is not a sphere, so the GJK
 // narrow phase is compiled in.
 template <bool kConvex>
-__device__ __forceinline__ bool evalPair64(DevState const& S, GridDesc const& g, int s0, int s1,
+__device__ __forceinline__ bool evalPair64(DevState const& S, GridDesc const& g, int c, int s0, int s1,
                                            int prio0, int prio1, int id0, int id1,
                                            TypeDesc const& tp0,
                                            TypeDesc const& tp1, d3 x0, d3 x1, d3 v0, d3 v1,
-                                           d3 w0, d3 w1, bool insert, GjkTally& gjk,
+                                           d3 w0, d3 w1, GjkTally& gjk,
                                            double& delta, d3& f, d3& c0, d3& c1m, d3& mr,
                                            bool& rolling) {
   const int cap = S.cap;
-  const unsigned tag = (unsigned)S.ctl[kCtlEpoch], tag_old = tag - 1u;
-  // spheres: the history lookup's first probe (key and values) is read
-  // before the narrow phase -- the key depends on the two IDs only -- so its
-  // loads overlap the narrow phase
-  const unsigned long long hkey = pairKey(min(id0, id1), max(id0, id1));
-  uint32_t hslot = 0;
-  unsigned long long hfirst = 0;
+  const int now = S.ctl[kCtlEpoch];
+  // spheres: the pair's memory is read before the narrow phase, so that its
+  // loads overlap it
   double hv[9];
-  if constexpr (!kConvex) {
-    hslot = hashSlot(hkey, S.hist_old.log2cap);
-    hfirst = S.hist_old.keys[hslot];
-    const double* p = static_cast<const double*>(S.hist_old.vals) + 9 * (size_t)hslot;
-#pragma unroll
-    for (int k = 0; k < 9; ++k) hv[k] = p[k];
-  }
+  int written = -1;
+  if constexpr (!kConvex) written = memLoad(S.pmem, c, hv, false);
   Contact64 ct;
   if (!kConvex || (tp0.shape == 0 && tp1.shape == 0)) {
     ct = sphereSphere64(x0, tp0.radius, tp0.crust, x1, tp1.radius, tp1.crust);
@@ -133,42 +114,31 @@ __device__ __forceinline__ bool evalPair64(DevState const& S, GridDesc const& g,
       recordVertex(S, tp0, s0, prio0, c0v);
       recordVertex(S, tp1, s1, prio1, c1v);
     }
-    if (insert) gjk.add(ct.gjk_iters);   // each pair counted once
+    gjk.add(ct.gjk_iters);
   }
   delta = ct.contact ? ct.dist : __longlong_as_double(0x7ff0000000000000ll);
   if (!ct.contact || !(ct.dist < 0.)) return false;
   if (ct.error) raise(S.status, kErrContactOverlap);
   ModelDesc const& m = S.models[g.model_base + tp0.mat * kMaxMat + tp1.mat];
   if (m.memory) {
-    // the table holds the lower ID's view; p0 may be the higher ID (the
+    // the memory is the lower ID's view; p0 may be the higher ID (the
     // reference's pair orientation), whose view is the negation
     const bool flip = id0 > id1;
-    const unsigned long long key = hkey;
-    int old;
-    if constexpr (!kConvex) {
-      if (hfirst == tagged(key, tag_old)) old = (int)hslot;
-      else if (tagOf(hfirst) != (tag_old & kTagMask)) old = -1;
-      else old = histFindAfter(S.hist_old, key, tag_old, hslot);
-    } else {
-      old = histFind(S.hist_old, key, tag_old);
-    }
-    d3 kd, pn, sp;
-    if (old >= 0) {
-      if (!kConvex && old == (int)hslot) {
-        kd = mk(hv[0], hv[1], hv[2]); pn = mk(hv[3], hv[4], hv[5]); sp = mk(hv[6], hv[7], hv[8]);
-      } else {
-        loadHist(S.hist_old, old, kd, pn, sp);
-      }
-      if (flip) { kd = -kd; pn = -pn; sp = -sp; }
+    const bool spring = m.rolling != 0;
+    if (kConvex || spring) written = memLoad(S.pmem, c, hv, spring);
+    const bool existed = remembered(S, written, now);
+    d3 kd = mk(0., 0., 0.), pn = kd, sp = kd;
+    if (existed) {
+      const double sg = flip ? -1. : 1.;
+      kd = mk(sg * hv[0], sg * hv[1], sg * hv[2]);
+      pn = mk(sg * hv[3], sg * hv[4], sg * hv[5]);
+      sp = mk(sg * hv[6], spring ? sg * hv[7] : 0., spring ? sg * hv[8] : 0.);
     }
     hodc64(m, S.dt, ct.point, ct.overlap, x0, v0, w0, tp0.mass, tp0.eqrad, x1, v1, w1, tp1.mass,
-           tp1.eqrad, old >= 0, kd, pn, sp, f, mr);
-    if (insert) {
-      int slot = histInsert(S.hist_new, key, tag);
-      if (slot < 0) raise(S.status, kErrHashFull);
-      else if (flip) storeHist(S.hist_new, slot, -kd, -pn, -sp);
-      else storeHist(S.hist_new, slot, kd, pn, sp);
-    }
+           tp1.eqrad, existed, kd, pn, sp, f, mr);
+    if (flip) { kd = -kd; pn = -pn; sp = -sp; }
+    const double out[9] = {kd.x, kd.y, kd.z, pn.x, pn.y, pn.z, sp.x, sp.y, sp.z};
+    memStore(S.pmem, c, out, now, spring || !existed);
   } else {
     hooke64(m, ct.point, ct.overlap, x0, v0, w0, tp0.mass, tp0.eqrad, x1, v1, w1, tp1.mass,
             tp1.eqrad, f, mr);
@@ -192,72 +162,107 @@ __device__ __forceinline__ void storeShare64(DevState const& S, int64_t entry, i
   sh[3] = make_double2(c.z, 0.);
 }
 
-// The wall contacts of particle t (near a wall per the contact filter): the
-// particle is p0, the obstacle p1 (mass Component::m_massObstacle); their
-// sum is the particle's wall share.
+// Contact of particle t (class ta, row of the wall list) with wall k of its
+// instance: the particle is p0, the obstacle p1 (mass Component::
+// m_massObstacle).  Returns true for a contact, with its force f, the lever
+// arm's torque c and, with a rolling model (rolling), the rolling torque mr.
 template <bool kConvex>
-__device__ __forceinline__ void wallsOf64(DevState const& S, int t, int tag, GjkTally& gjk,
-                                          StatsTally& st) {
+__device__ __forceinline__ bool wallContact64(DevState const& S, GridDesc const& g, int row, int t,
+                                              int k, TypeDesc const& ta, d3 xt, d3 vt, d3 wt,
+                                              int& curw, bool& walls_gjk, GjkTally& gjk,
+                                              StatsTally& st, d3& f, d3& c, d3& mr, bool& rolling) {
   const int cap = S.cap;
-  GridDesc const& g = S.grids[S.inst[t]];
-  const int ida = S.id[t];
-  TypeDesc const& ta = S.types[S.type[t]];
-  const d3 xt = ld3(S.x, cap, t), vt = ld3(S.v, cap, t), wt = ld3(S.w, cap, t);
-  const double dt = S.dt;
-  const unsigned utag = (unsigned)tag, tag_old = utag - 1u;
-  d3 Fw = mk(0., 0., 0.), Tw = mk(0., 0., 0.);
-  bool any = false;
-  // the particle's polyhedron vertex runs through its wall calls in order
-  int curw = kConvex ? startVertex(S, ta, t) : 0;
-  bool walls_gjk = false;
-  for (int k = 0; k < g.wall_count; ++k) {
-    WallDesc const& wd = S.walls[g.wall_begin + k];
-    int cw = 0;
-    Contact64 ct = (!kConvex || ta.shape == 0)
-        ? sphereWall64(xt, ta.radius, ta.crust, wd)
-        : convexContact64(convexOf(ta, S), crustXForm(S.basis, cap, t, ta.scaling, xt),
-                          ta.radius, ta.crust, convexOf(wd),
-                          identityXForm(wd.scaling, mk(wd.centre[0], wd.centre[1], wd.centre[2])),
-                          wd.radius, wd.crust, curw, cw);
-    if (kConvex) gjk.add(ct.gjk_iters);
-    if (kConvex && ct.gjk_iters > 0) walls_gjk = true;
-    if (S.diag) S.wall_delta[(size_t)t * S.max_walls + k] = ct.contact ? ct.dist : __longlong_as_double(0x7ff0000000000000ll);
-    if (ct.error) raise(S.status, kErrContactOverlap);
-    if (!ct.contact || !(ct.dist < 0.)) continue;
-    st.add(ct.dist);
-    ModelDesc const& m = S.models[g.model_base + ta.mat * kMaxMat + wd.mat];
-    d3 f, mr;
-    const d3 zero = mk(0., 0., 0.);
-    const d3 wc = mk(wd.centre[0], wd.centre[1], wd.centre[2]);
-    if (m.memory) {
-      const unsigned long long key = wallKey(ida, k);
-      int old = histFind(S.hist_old, key, tag_old);
-      d3 kd, pn, sp;
-      if (old >= 0) loadHist(S.hist_old, old, kd, pn, sp);
-      hodc64(m, dt, ct.point, ct.overlap, xt, vt, wt, ta.mass, ta.eqrad, wc, zero, zero, 1.e20,
-             wd.eqrad, old >= 0, kd, pn, sp, f, mr);
-      int slot = histInsert(S.hist_new, key, utag);
-      if (slot < 0) raise(S.status, kErrHashFull);
-      else storeHist(S.hist_new, slot, kd, pn, sp);
-    } else {
-      hooke64(m, ct.point, ct.overlap, xt, vt, wt, ta.mass, ta.eqrad, wc, zero, zero, 1.e20,
-              wd.eqrad, f, mr);
+  WallDesc const& wd = S.walls[g.wall_begin + k];
+  int cw = 0;
+  Contact64 ct = (!kConvex || ta.shape == 0)
+      ? sphereWall64(xt, ta.radius, ta.crust, wd)
+      : convexContact64(convexOf(ta, S), crustXForm(S.basis, cap, t, ta.scaling, xt),
+                        ta.radius, ta.crust, convexOf(wd),
+                        identityXForm(wd.scaling, mk(wd.centre[0], wd.centre[1], wd.centre[2])),
+                        wd.radius, wd.crust, curw, cw);
+  if (kConvex) gjk.add(ct.gjk_iters);
+  if (kConvex && ct.gjk_iters > 0) walls_gjk = true;
+  if (S.diag) S.wall_delta[(size_t)t * S.max_walls + k] = ct.contact ? ct.dist : __longlong_as_double(0x7ff0000000000000ll);
+  if (ct.error) raise(S.status, kErrContactOverlap);
+  if (!ct.contact || !(ct.dist < 0.)) return false;
+  st.add(ct.dist);
+  ModelDesc const& m = S.models[g.model_base + ta.mat * kMaxMat + wd.mat];
+  const d3 zero = mk(0., 0., 0.);
+  const d3 wc = mk(wd.centre[0], wd.centre[1], wd.centre[2]);
+  if (m.memory) {
+    const int now = S.ctl[kCtlEpoch];
+    const long long at = (long long)row * S.max_walls + k;
+    const bool spring = m.rolling != 0;
+    double hv[9];
+    const bool existed = remembered(S, memLoad(S.wmem, at, hv, spring), now);
+    d3 kd = zero, pn = zero, sp = zero;
+    if (existed) {
+      kd = mk(hv[0], hv[1], hv[2]); pn = mk(hv[3], hv[4], hv[5]);
+      sp = mk(hv[6], spring ? hv[7] : 0., spring ? hv[8] : 0.);
     }
-    if (S.diag) {
-      double* fd = S.wall_force + 3 * ((size_t)t * S.max_walls + k);
-      fd[0] = f.x; fd[1] = f.y; fd[2] = f.z;
-    }
-    Fw = Fw + f;
-    Tw = Tw + cross(ct.point - xt, f);
-    if (m.rolling) Tw = Tw + mr;
-    any = true;
+    hodc64(m, S.dt, ct.point, ct.overlap, xt, vt, wt, ta.mass, ta.eqrad, wc, zero, zero, 1.e20,
+           wd.eqrad, existed, kd, pn, sp, f, mr);
+    const double out[9] = {kd.x, kd.y, kd.z, pn.x, pn.y, pn.z, sp.x, sp.y, sp.z};
+    memStore(S.wmem, at, out, now, spring || !existed);
+  } else {
+    hooke64(m, ct.point, ct.overlap, xt, vt, wt, ta.mass, ta.eqrad, wc, zero, zero, 1.e20,
+            wd.eqrad, f, mr);
   }
-  if (walls_gjk) recordVertex(S, ta, t, kWallPriority, curw);
+  if (S.diag) {
+    double* fd = S.wall_force + 3 * ((size_t)t * S.max_walls + k);
+    fd[0] = f.x; fd[1] = f.y; fd[2] = f.z;
+  }
+  c = cross(ct.point - xt, f);
+  rolling = m.rolling != 0;
+  return true;
+}
+
+// One wall item of the evaluation: a (particle, wall) slot of the wall list
+// (spheres), whose contact is its share, or a particle of it, whose walls are
+// taken in order and summed into its first slot's share.
+template <bool kConvex>
+__device__ __forceinline__ void wallItem64(DevState const& S, int item, int tag, GjkTally& gjk,
+                                           StatsTally& st) {
+  const int row = kConvex ? item : item / S.max_walls;
+  const int t = S.wlist[row];
+  GridDesc const& g = S.grids[S.inst[t]];
+  TypeDesc const& ta = S.types[S.type[t]];
+  const d3 xt = ld3(S.x, S.cap, t), vt = ld3(S.v, S.cap, t), wt = ld3(S.w, S.cap, t);
+  d3 f, c, mr = mk(0., 0., 0.);
+  bool rolling = false, any = false, walls_gjk = false;
+  int curw = 0;
+  if constexpr (kConvex) {
+    // the particle's polyhedron vertex runs through its wall calls in order
+    curw = startVertex(S, ta, t);
+    d3 Fw = mk(0., 0., 0.), Tw = mk(0., 0., 0.);
+    for (int k = 0; k < g.wall_count; ++k) {
+      if (!wallContact64<kConvex>(S, g, row, t, k, ta, xt, vt, wt, curw, walls_gjk, gjk, st, f, c, mr,
+                                  rolling))
+        continue;
+      Fw = Fw + f;
+      Tw = Tw + c;
+      if (rolling) Tw = Tw + mr;
+      any = true;
+    }
+    if (walls_gjk) recordVertex(S, ta, t, kWallPriority, curw);
+    f = Fw;
+    c = Tw;
+    rolling = false;
+    item = row * S.max_walls;
+  } else {
+    any = wallContact64<kConvex>(S, g, row, t, item - row * S.max_walls, ta, xt, vt, wt, curw,
+                                 walls_gjk, gjk, st, f, c, mr, rolling);
+  }
   if (!any) return;
-  double2* ws = static_cast<double2*>(S.wshare) + 3 * (size_t)t;
-  ws[0] = make_double2(Fw.x, Fw.y);
-  ws[1] = make_double2(Fw.z, Tw.x);
-  ws[2] = make_double2(Tw.y, Tw.z);
+  double2* ws = static_cast<double2*>(S.wshare) + (size_t)kWallShare64 * item;
+  ws[0] = make_double2(__longlong_as_double((long long)tag), f.x);
+  ws[1] = make_double2(f.y, f.z);
+  ws[2] = make_double2(c.x, c.y);
+  ws[3] = make_double2(c.z, rolling ? 1. : 0.);
+  if (rolling) {
+    ws[4] = make_double2(mr.x, mr.y);
+    ws[5] = make_double2(mr.z, 0.);
+  }
   atomicOr(reinterpret_cast<unsigned*>(&contactFlags(S)[t]), kNearWall);
 }
 
@@ -309,8 +314,8 @@ __device__ __forceinline__ void pairItem64(DevState const& S, int c, int tag, Gj
   double dl;
   bool rolling;
   const bool hit = evalPair64<kConvex>(
-      S, g, a, b, pa, pb, flip ? idu : idt, flip ? idt : idu, S.types[flip ? tyu : tyt], S.types[flip ? tyt : tyu],
-      flip ? xu : xt, flip ? xt + (-shift) : xu + shift, vt, vu, wt, wu, true, gjk, dl, f, c0, c1m, mr, rolling);
+      S, g, c, a, b, pa, pb, flip ? idu : idt, flip ? idt : idu, S.types[flip ? tyu : tyt], S.types[flip ? tyt : tyu],
+      flip ? xu : xt, flip ? xt + (-shift) : xu + shift, vt, vu, wt, wu, gjk, dl, f, c0, c1m, mr, rolling);
   const int64_t rt = (int64_t)offt + et, ru = (int64_t)offu + eu;
   // p0's share (f, its torque) and p1's (-f, its torque), given to t and u
   const d3 t0 = rolling ? c0 + mr : c0, t1 = rolling ? c1m + (-mr) : c1m;
@@ -342,8 +347,13 @@ __device__ __forceinline__ void pairItem64(DevState const& S, int c, int tag, Gj
 // grid: first the pairs the contact filter kept, then the particles near a
 // wall.  Its trigger comes after its wait, so the leapfrog kernel, which
 // starts at the trigger, sees the filter's candidate marks complete.
+// The sphere kernel is bound by latency like the FP32-split one; four blocks
+// per multiprocessor (128 registers, some spilled) beat two and three where
+// there is work for them: packed beds of 60,000 and 250,000 spheres 39.6 and
+// 120.8 us, with three 40.5 and 126.6, with two 37.2 and 159.9 (before: 79.8
+// and 307.7, with the memory in a hash table and a particle's walls in turn).
 template <bool kConvex>
-__global__ void __launch_bounds__(128) k_pairlaw64(DevState S) {
+__global__ void __launch_bounds__(128, kConvex ? 1 : 4) k_pairlaw64(DevState S) {
   pdlWait();      // the contact filter's lists
   pdlTrigger();   // the leapfrog kernel may start; its candidates wait for this kernel
   const int nk = S.ctl[kCtlKept], nw = S.ctl[kCtlWork];
@@ -353,7 +363,7 @@ __global__ void __launch_bounds__(128) k_pairlaw64(DevState S) {
   StatsTally st;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < nk + nw; i += stride) {
     if (i < nk) pairItem64<kConvex>(S, S.kept[i], tag, gjk, st);
-    else wallsOf64<kConvex>(S, S.work[i - nk], tag, gjk, st);
+    else wallItem64<kConvex>(S, S.work[i - nk], tag, gjk, st);
   }
   // (every lane of the warp reaches this point: no thread leaves the loop early)
   if constexpr (kConvex) gjk.flush(S.gjk_counts);

@@ -286,10 +286,16 @@ __device__ __forceinline__ ConvexRef convexOf(WallDesc const& w) {
 // list, which is the lower ID after a reload.  Returns true when u is p0.
 // The contact law is evaluated with the reference's p0 so that its FP64
 // result has the reference's rounding.
+// The cell by a product with 1 / edge; within 1e-6 of a cell face, where its
+// rounding (below 1e-9 cells for any grid) could decide, by the division.
+__device__ __forceinline__ int referenceCell(GridDesc const& g, int d, double x) {
+  const double q = (x - g.lc_origin[d]) * g.inv_edge[d];
+  const double f = floor(q);
+  if (q - f > 1.e-6 && q - f < 1. - 1.e-6) return (int)f;
+  return (int)floor((x - g.lc_origin[d]) / g.edge[d]);
+}
 __device__ __forceinline__ int referenceCellNumber(GridDesc const& g, d3 x) {
-  const int i = (int)floor((x.x - g.lc_origin[0]) / g.edge[0]);
-  const int j = (int)floor((x.y - g.lc_origin[1]) / g.edge[1]);
-  const int k = (int)floor((x.z - g.lc_origin[2]) / g.edge[2]);
+  const int i = referenceCell(g, 0, x.x), j = referenceCell(g, 1, x.y), k = referenceCell(g, 2, x.z);
   return j * g.nb[2] * g.nb[0] + k * g.nb[0] + i;
 }
 __device__ __forceinline__ bool referenceFlip(GridDesc const& g, d3 xt, d3 xu, const int* sh) {

@@ -7,20 +7,29 @@
 
 namespace gdem {
 
-// Contact-history table: open addressing with linear probing, keyed on the
-// unordered particle pair or on (particle, wall).  Values are stored as seen
+// Contact memory.  It lives beside what uses it: per pair of the compact pair
+// list and per wall of each particle in the wall list (MemView), where the
+// pair kernel's lanes read and write it in list order.  Values are as seen
 // from the lower-ID body (or the particle, for a wall); the other body's view
 // is the negation, as in the reference where p1 holds (-kdelta, -normal,
-// -spring) (HookeMemoryContactForceModel.cpp:191-192).  Two tables
-// alternate: the one written by force evaluation e is read by evaluation
-// e + 1, so entries not touched in a step disappear, which is what
-// Component::updateContactMap (Component.cpp:583-595) does.
+// -spring) (HookeMemoryContactForceModel.cpp:191-192).  An entry carries the
+// evaluation that last wrote it: the plain step uses it when that is the
+// evaluation before, so entries not touched in a step disappear, which is what
+// Component::updateContactMap (Component.cpp:583-595) does; the coupled step
+// uses it whenever it was ever written.
 //
-// Key layout: bits 54-63 the evaluation tag (e mod 1024), bits 27-53 the
-// lower particle ID, bits 0-26 the higher particle ID or, for a wall,
-// 2^27 - 1 - wall index.  A slot whose tag is not the current evaluation's is
-// free, so a table needs no clearing between uses; the host clears each
-// table once every 512 of its uses, before a tag value can come round again.
+// HistTable carries the memory across what changes the lists (a rebuild, a
+// new state, a larger allocation) and in and out of the library: open
+// addressing with linear probing, keyed on the unordered particle pair or on
+// (particle, wall).  The plain step's table is emptied before the lists are
+// saved into it; the coupled step's keeps the entries of every pair that ever
+// touched.  (The table used to be read and written by every evaluation, at
+// random places of two tables: 1M spheres 5 of the pair kernel's 24 us, a
+// packed bed two thirds of its memory traffic.)
+//
+// Key layout: bits 54-63 a tag (0 for an entry, 1023 for a free slot), bits
+// 27-53 the lower particle ID, bits 0-26 the higher particle ID or, for a
+// wall, 2^27 - 1 - wall index.
 constexpr int kTagShift = 54;
 constexpr unsigned kTagMask = 1023u;
 constexpr int kMaxIdBits = 27;
@@ -66,22 +75,7 @@ __device__ inline int histFind(HistTable const& t, unsigned long long base, unsi
   }
   return -1;
 }
-// histFind after its first probe (slot first, key k0 read there) matched
-// neither the key nor an empty slot: the lookup from the next slot on.
-__device__ inline int histFindAfter(HistTable const& t, unsigned long long base, unsigned tag,
-                                    uint32_t first) {
-  const uint32_t mask = (1u << t.log2cap) - 1;
-  const unsigned long long key = tagged(base, tag);
-  uint32_t s = (first + 1) & mask;
-  for (uint32_t probe = 1; probe <= mask; ++probe) {
-    const unsigned long long k = t.keys[s];
-    if (k == key) return (int)s;
-    if (tagOf(k) != (tag & kTagMask)) return -1;
-    s = (s + 1) & mask;
-  }
-  return -1;
-}
-// Claims a slot for base with tag (one writer per key and evaluation); -1
+// Claims a slot for base with tag (one writer per key at a time); -1
 // when every slot carries the tag already (table full).
 __device__ inline int histInsert(HistTable const& t, unsigned long long base, unsigned tag) {
   const uint32_t mask = (1u << t.log2cap) - 1;
@@ -101,6 +95,67 @@ __device__ inline int histInsert(HistTable const& t, unsigned long long base, un
     s = (s + 1) & mask;
   }
   return -1;
+}
+
+// Contact memory in list order: n entries in planes of vectors, so that
+// neighbouring entries' loads coalesce.  FP32: (kdelta, evaluation),
+// (normal, spring x), (spring y, z); FP64: five pairs of doubles in the same
+// order.  The last plane (spring y, z) only matters with rolling resistance.
+struct MemView {
+  void* p;
+  long long n;
+};
+constexpr size_t kMemBytes32 = 40, kMemBytes64 = 80;
+__device__ __forceinline__ int memLoad(MemView m, long long i, float* v, bool spring) {
+  const float4* A = static_cast<const float4*>(m.p);
+  const float4 a = A[i], b = A[m.n + i];
+  v[0] = a.x; v[1] = a.y; v[2] = a.z;
+  v[3] = b.x; v[4] = b.y; v[5] = b.z; v[6] = b.w;
+  if (spring) {
+    const float2 c = reinterpret_cast<const float2*>(A + 2 * m.n)[i];
+    v[7] = c.x; v[8] = c.y;
+  }
+  return __float_as_int(a.w);
+}
+__device__ __forceinline__ void memStore(MemView m, long long i, const float* v, int evaluation,
+                                         bool spring) {
+  float4* A = static_cast<float4*>(m.p);
+  A[i] = make_float4(v[0], v[1], v[2], __int_as_float(evaluation));
+  A[m.n + i] = make_float4(v[3], v[4], v[5], v[6]);
+  if (spring) reinterpret_cast<float2*>(A + 2 * m.n)[i] = make_float2(v[7], v[8]);
+}
+__device__ __forceinline__ int memLoad(MemView m, long long i, double* v, bool spring) {
+  const double2* A = static_cast<const double2*>(m.p);
+  const double2 a = A[i], b = A[m.n + i], c = A[2 * m.n + i], d = A[3 * m.n + i];
+  v[0] = a.x; v[1] = a.y; v[2] = b.x;
+  v[3] = c.x; v[4] = c.y; v[5] = d.x; v[6] = d.y;
+  if (spring) {
+    const double2 e = A[4 * m.n + i];
+    v[7] = e.x; v[8] = e.y;
+  }
+  return (int)__double_as_longlong(b.y);
+}
+__device__ __forceinline__ void memStore(MemView m, long long i, const double* v, int evaluation,
+                                         bool spring) {
+  double2* A = static_cast<double2*>(m.p);
+  A[i] = make_double2(v[0], v[1]);
+  A[m.n + i] = make_double2(v[2], __longlong_as_double((long long)evaluation));
+  A[2 * m.n + i] = make_double2(v[3], v[4]);
+  A[3 * m.n + i] = make_double2(v[5], v[6]);
+  if (spring) A[4 * m.n + i] = make_double2(v[7], v[8]);
+}
+// The evaluation that last wrote entry i (-1: none), and marking it so.
+__device__ __forceinline__ int memEvaluation(MemView m, long long i, float) {
+  return __float_as_int(static_cast<const float4*>(m.p)[i].w);
+}
+__device__ __forceinline__ int memEvaluation(MemView m, long long i, double) {
+  return (int)__double_as_longlong(static_cast<const double2*>(m.p)[m.n + i].y);
+}
+__device__ __forceinline__ void memForget(MemView m, long long i, float) {
+  static_cast<float4*>(m.p)[i].w = __int_as_float(-1);
+}
+__device__ __forceinline__ void memForget(MemView m, long long i, double) {
+  static_cast<double2*>(m.p)[m.n + i].y = __longlong_as_double(-1ll);
 }
 
 // Overlap statistics of the contacts over the evaluations since the last
@@ -173,12 +228,20 @@ struct DevState {
   // from that pair (written by the pair kernel for a contact, tagged with the
   // evaluation counter), summed in row order by the leapfrog kernel
   void* share;
-  void* wshare;           // per particle: the sum of its wall contacts (this evaluation)
+  // wall list (rebuilt with the pair list): the particles that can come near a
+  // wall before the next rebuild, and each particle's index in it (or -1);
+  // per listed particle and wall of its instance (max_walls slots) the
+  // contact memory and this evaluation's share
+  int* wlist; int* wrow;
+  int wall_cap;           // listed particles allocated
+  void* wshare;           // kWallShare vectors per slot
   int* nact;              // flag words, two buffers of cap (contactFlags)
   float4* posf;           // FP32 continuous position since the last rebuild + circumscribed radius
-  int* work;              // particles near a wall (this evaluation), ctl[kCtlWork]
+  // this evaluation's wall items, ctl[kCtlWork]: slots of the wall list
+  // (spheres) or, with non-spherical classes, its particles
+  int* work;
   int nsm;                // multiprocessors of the device (persistent grids)
-  int forces_bps;         // blocks per multiprocessor of the pair kernel's persistent grid (0: 4)
+  int forces_bps;         // blocks per multiprocessor of the pair kernel's persistent grid (0: the default)
   double* pair_delta;     // diagnostics: overlap of each entry (+inf: no contact)
   double* wall_delta;     // diagnostics: overlap with each wall slot
   double* pair_force;     // diagnostics: contact force on the lower ID (3 per entry)
@@ -187,7 +250,9 @@ struct DevState {
   ContactStats* cstats;   // overlap statistics over all evaluations
   double* wall_force;     // diagnostics: wall contact force on the particle (3 per slot)
   int diag;
-  HistTable hist_old, hist_new;
+  MemView pmem, wmem;     // contact memory of the pair list and of the wall list
+  HistTable hist;         // the memory across rebuilds
+  int prune;              // memory of ended contacts is dropped (the plain step)
   int* status;
   GridDesc const* grids;  // reference linked-cell grids (cell reports, periodic wrap)
   GridDesc const* bgrids; // pair-list grids: cells at least 2 rmax + skin wide
@@ -206,6 +271,7 @@ struct DevState {
   int any_walls;          // some instance has walls
   float filt_margin_max;  // largest contact-filter margin of the instances
   int filter_qblocks;     // contact filter: blocks for the pairs (0: from the particle count)
+  int filter_wblocks;     // and for the wall list
 };
 
 // ----------------------------------------------------------- FP64 helpers --
@@ -271,6 +337,23 @@ __device__ __forceinline__ d3 rotateVector(dq q, d3 v) {
 }
 
 __device__ __forceinline__ void raise(int* status, int bits) { atomicOr(status, bits); }
+
+// 16-byte words of a wall share: force with the evaluation tag, torque of the
+// lever arm with a rolling flag, rolling torque.
+constexpr int kWallShare32 = 3, kWallShare64 = 6;
+
+// Pairs of the compact list whose entries are allocated.
+__device__ __forceinline__ int listedPairs(DevState const& S) {
+  return (int)min((long long)S.ctl[kCtlPairs], S.pmem.n);
+}
+__device__ __forceinline__ int listedWalls(DevState const& S) {
+  return min(S.ctl[kCtlWallRows], S.wall_cap);
+}
+// Whether memory last written by evaluation e is still the contact's at
+// evaluation now.
+__device__ __forceinline__ bool remembered(DevState const& S, int e, int now) {
+  return S.prune ? e == now - 1 : e >= 0;
+}
 
 // Cell of a neighbour offset (di, dj, dk) around (i, j, k) of grid g, with
 // the periodic minimum-image wrap.  Returns the global cell key or -1, and the

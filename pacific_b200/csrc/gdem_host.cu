@@ -123,6 +123,7 @@ void makePairGrid(InstanceDesc& I, double skin) {
     if (I.box_per[d] && n < 3) n = 3;
     b.nb[d] = n;
     b.edge[d] = size / n;
+    b.inv_edge[d] = 1. / b.edge[d];
     b.lc_origin[d] = I.box_org[d];
     if (I.box_per[d]) {
       b.lc_origin[d] += -b.edge[d];
@@ -518,6 +519,7 @@ InstanceDesc readInstance(std::string const& path) {
     if (!n) n = 1;
     g.nb[d] = n;
     g.edge[d] = size / n;
+    g.inv_edge[d] = 1. / g.edge[d];
     g.lc_origin[d] = org[d];
     g.L[d] = size;
     g.periodic[d] = per[d];
@@ -580,7 +582,7 @@ struct System {
   std::vector<int> h_type, h_inst; // uploaded classes (instance-local) and instances, by ID
   std::vector<int> ref_ids;        // reload particle IDs by particle index (empty: index + 1)
   double tune_skin = -1.;          // skin as a multiple of rmax (< 0: the XML's or 0.25)
-  int tune_bps = 0;                // force-kernel blocks per multiprocessor (0: 4)
+  int tune_bps = 0;                // force-kernel blocks per multiprocessor (0: the default)
   std::vector<int> type_base;     // first global type of each instance
   std::vector<int> id_base;       // first particle ID of each instance
   std::vector<int> inst_n;
@@ -597,9 +599,8 @@ struct System {
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
   bool have_state = false, started = false, diag = false, use_graphs = true;
   // contact memory of ended contacts dropped each evaluation (the plain
-  // step) or carried (the coupled step); the tables are four times larger
-  // when it is carried, since the entries of every pair that ever touched
-  // stay
+  // step) or kept (the coupled step); its table is four times larger when it
+  // is kept, since the entries of every pair that ever touched stay
   bool prune_memory = true;
   // the last force evaluation: 0 none since the state was set, 1 recorded by
   // the diagnostics, 2 run without them
@@ -607,9 +608,10 @@ struct System {
   bool id_order = false;           // state arrays are in particle-ID order (not yet binned)
   double last_ms = 0.;
   int status_host = 0;
-  cudaGraphExec_t graph[2][2] = {{nullptr, nullptr}, {nullptr, nullptr}};
-  long parity = 0;                 // force evaluations so far (state and history swap together)
-  long epoch = 0;                  // host copy of the evaluation counter (history tags)
+  cudaGraphExec_t graph[2] = {nullptr, nullptr};   // an evaluation inside a call, and its last
+  long epoch = 0;                  // host copy of the evaluation counter
+  bool lists_hold = false;         // the lists (not the table) hold the contact memory
+  bool lists_sized = false;        // the lists' allocations are checked against this state
   long epoch_t0 = 0;               // evaluation counter at the leapfrog's t0 (contact features)
   bool graph_conditional = false;  // the graphs rebuild through a conditional node
   std::vector<void*> allocs;
@@ -628,8 +630,7 @@ struct System {
 
   ~System() { release(); }
   void release() {
-    for (auto& row : graph)
-      for (auto& gx : row) if (gx) { cudaGraphExecDestroy(gx); gx = nullptr; }
+    for (auto& gx : graph) if (gx) { cudaGraphExecDestroy(gx); gx = nullptr; }
     for (void* p : allocs) cudaFree(p);
     allocs.clear();
     if (d_grids) cudaFree(d_grids);
@@ -658,8 +659,7 @@ struct System {
     return p;
   }
   void invalidateGraphs() {
-    for (auto& row : graph)
-      for (auto& gx : row) if (gx) { cudaGraphExecDestroy(gx); gx = nullptr; }
+    for (auto& gx : graph) if (gx) { cudaGraphExecDestroy(gx); gx = nullptr; }
   }
   void freeAlloc(void* p) {
     for (auto& a : allocs)
@@ -859,15 +859,14 @@ struct System {
     CK(cudaMemset(S.npairs, 0, c * sizeof(int)));
     CK(cudaMemset(S.pair_off, 0, (c + 1) * sizeof(int)));
     S.pairs = nullptr; S.upairs = nullptr; S.epos = nullptr; S.kept = nullptr; S.kept2 = nullptr;
+    S.pmem = MemView{nullptr, 0};
     S.share = nullptr;
     S.pair_cap = 0;
     S.pair_delta = nullptr; S.wall_delta = nullptr; S.diag = 0;
     S.pair_force = nullptr; S.wall_force = nullptr;
     allocatePairs((long long)16 * (long long)c + 4096);
-    S.wshare = alloc<char>(c * (precision == GDEM_FP64 ? 48 : 32));
     S.nact = alloc<int>(2 * c);
     CK(cudaMemset(S.nact, 0, 2 * c * sizeof(int)));
-    S.work = alloc<int>(c);
     S.cstats = alloc<ContactStats>(1);
     CK(cudaMemset(S.cstats, 0, sizeof(ContactStats)));
     {
@@ -876,16 +875,20 @@ struct System {
       CK(cudaDeviceGetAttribute(&S.nsm, cudaDevAttrMultiProcessorCount, dev));
     }
     S.posf = alloc<float4>(c);
-    int l2 = nextPow2Log((size_t)8 * c + 64) + (prune_memory ? 0 : 2);
-    size_t hc = size_t(1) << l2;
-    size_t vsz = precision == GDEM_FP64 ? sizeof(double) : sizeof(float);
-    for (HistTable* t : {&S.hist_old, &S.hist_new}) {
-      t->log2cap = l2;
-      t->keys = alloc<unsigned long long>(hc);
-      t->vals = alloc<char>(hc * 9 * vsz);
-      // all-ones keys: tag 1023, which the first 512 uses of a table never carry
-      CK(cudaMemset(t->keys, 0xFF, hc * sizeof(unsigned long long)));
-    }
+    S.prune = prune_memory ? 1 : 0;
+    S.hist.log2cap = nextPow2Log((size_t)8 * c + 64) + (prune_memory ? 0 : 2);
+    const size_t hc = size_t(1) << S.hist.log2cap;
+    S.hist.keys = alloc<unsigned long long>(hc);
+    S.hist.vals = alloc<char>(hc * 9 * (precision == GDEM_FP64 ? sizeof(double) : sizeof(float)));
+    CK(cudaMemset(S.hist.keys, 0xFF, hc * sizeof(unsigned long long)));   // kEmptyKey
+    S.wlist = nullptr; S.work = nullptr; S.wshare = nullptr;
+    S.wmem = MemView{nullptr, 0};
+    S.wall_cap = 0;
+    S.wrow = alloc<int>(S.any_walls ? c : 1);
+    // the wall list: every particle of a small system, a quarter of a large
+    // one's (a wall layer is far thinner; sizeLists grows it before the steps
+    // that follow a new state, checkCapacity during a run)
+    if (S.any_walls) allocateWalls(c <= 16384 ? (long long)c : (long long)c / 4);
     S.status = alloc<int>(1);
     CK(cudaMemset(S.status, 0, sizeof(int)));
     S.law_counts = alloc<unsigned long long>(2);
@@ -911,7 +914,8 @@ struct System {
   void allocatePairs(long long entries) {
     if (entries > (long long)INT_MAX - 64)
       throw std::runtime_error("pair list too large for 32-bit row offsets");
-    for (void* p : {(void*)S.pairs, (void*)S.upairs, (void*)S.epos, (void*)S.kept, (void*)S.kept2, S.share,
+    saveMemory(true);
+    for (void* p : {(void*)S.pairs, (void*)S.upairs, (void*)S.epos, (void*)S.kept, (void*)S.kept2, S.share, S.pmem.p,
                     (void*)S.pair_delta, (void*)S.pair_force})
       if (p) freeAlloc(p);
     const size_t e = (size_t)entries, pc = e / 2 + 1;
@@ -922,6 +926,8 @@ struct System {
     S.kept = alloc<int>(pc);
     // the cold pairs' first pass (FP32-split, non-spherical classes)
     S.kept2 = (precision == GDEM_FP32_SPLIT && S.any_convex) ? alloc<int>(pc) : nullptr;
+    const size_t mb = precision == GDEM_FP64 ? kMemBytes64 : kMemBytes32;
+    S.pmem = MemView{alloc<char>(pc * mb), (long long)pc};
     const size_t sb = precision == GDEM_FP64 ? 64 : 32;
     S.share = alloc<char>(e * sb);
     // (on the library's stream, which does not synchronise with the legacy
@@ -939,26 +945,72 @@ struct System {
     CK(cudaStreamSynchronize(stream));
     invalidateGraphs();
   }
-  // Grows the pair list when the most entries a rebuild needed since the
-  // last check exceed 80 % of the allocation (to 1.5 times that need);
-  // the next evaluation rebuilds.  Synchronises the stream.  Returns whether
-  // it grew.
-  bool checkPairCapacity() {
-    int hwm = 0;
-    CK(cudaStreamSynchronize(stream));
-    CK(cudaMemcpy(&hwm, S.ctl + kCtlEntriesMax, sizeof(int), cudaMemcpyDeviceToHost));
-    CK(cudaMemsetAsync(S.ctl + kCtlEntriesMax, 0, sizeof(int), stream));
-    CK(cudaStreamSynchronize(stream));
-    if ((double)hwm <= 0.8 * (double)S.pair_cap) return false;
-    allocatePairs(std::max((long long)(1.5 * (double)hwm) + 4096, (long long)S.pair_cap));
-    return true;
-  }
-  // Sizes the pair list for the current state before the leapfrog start: the
-  // rebuild up to the scan of the row lengths (it only reorders the state),
-  // then the allocation check.
-  void sizePairList() {
+  // The arrays sized by the wall list's particles (rebuilt before the next
+  // evaluation): the list, the evaluation's wall items, the slots' memory and
+  // shares (tag words all ones: no evaluation's tag).
+  void allocateWalls(long long rows) {
+    if (rows * S.max_walls > (long long)INT_MAX - 64)
+      throw std::runtime_error("wall list too large for 32-bit slots");
+    saveMemory(true);
+    if (S.wshare) freeAlloc(S.wshare);
+    const bool fp64 = precision == GDEM_FP64;
+    const size_t slots = (size_t)rows * S.max_walls;
+    // (one allocation; every part a multiple of 16 bytes)
+    auto round16 = [](size_t b) { return (b + 15) & ~size_t(15); };
+    const size_t sb = slots * 16 * (fp64 ? kWallShare64 : kWallShare32);
+    const size_t mb = round16(slots * (fp64 ? kMemBytes64 : kMemBytes32));
+    const size_t wb = round16(slots * sizeof(int));
+    char* p = alloc<char>(sb + mb + wb + rows * sizeof(int));
+    S.wall_cap = (int)rows;
+    S.wshare = p;
+    S.wmem = MemView{p + sb, (long long)slots};
+    S.work = reinterpret_cast<int*>(p + sb + mb);
+    S.wlist = reinterpret_cast<int*>(p + sb + mb + wb);
+    CK(cudaMemsetAsync(S.wshare, 0xFF, sb, stream));
     static const int one = 1;
+    if (S.ctl) CK(cudaMemcpyAsync(S.ctl + kCtlNeed, &one, sizeof(int), cudaMemcpyHostToDevice, stream));
+    CK(cudaStreamSynchronize(stream));
+    invalidateGraphs();
+  }
+  // Grows the pair list (the wall list) when the most entries (particles) a
+  // rebuild needed since the last check exceed 80 % of the allocation, to 1.5
+  // times that need; the next evaluation rebuilds.  Synchronises the stream.
+  void checkCapacity() {
+    int ctl[kCtlWords];
+    CK(cudaStreamSynchronize(stream));
+    CK(cudaMemcpy(ctl, S.ctl, sizeof(ctl), cudaMemcpyDeviceToHost));
+    CK(cudaMemsetAsync(S.ctl + kCtlEntriesMax, 0, sizeof(int), stream));
+    CK(cudaMemsetAsync(S.ctl + kCtlWallRowsMax, 0, sizeof(int), stream));
+    CK(cudaStreamSynchronize(stream));
+    const int hwm = ctl[kCtlEntriesMax], rows = std::max(ctl[kCtlWallRowsMax], ctl[kCtlWallRows]);
+    if ((double)hwm > 0.8 * (double)S.pair_cap)
+      allocatePairs(std::max((long long)(1.5 * (double)hwm) + 4096, (long long)S.pair_cap));
+    if (S.any_walls && S.wall_cap < S.cap && (double)rows > 0.8 * (double)S.wall_cap)
+      allocateWalls(std::min((long long)S.cap, (long long)(1.5 * (double)rows) + 4096));
+  }
+  // The contact memory of the last evaluation from the lists into its table
+  // (where the host reads it); with leave the table then holds it and the
+  // next rebuild's lists take it from there.  Nothing to do while the table
+  // holds it anyway.
+  void saveMemory(bool leave) {
+    if (!lists_hold) return;
+    if (prune_memory) launch_mem_clear(S, nullptr, stream);
+    launch_mem_save(S, nullptr, 0, precision == GDEM_FP64, stream);
+    if (leave) {
+      CK(cudaMemsetAsync(S.ctl + kCtlMemory, 0, sizeof(int), stream));
+      lists_hold = false;
+    }
+    CK(cudaGetLastError());
+    CK(cudaStreamSynchronize(stream));
+  }
+  // Sizes the lists for the current state before its first evaluation: the
+  // rebuild up to the scan of the row lengths and the wall list (it only
+  // reorders the state), then the allocation check; the evaluation rebuilds.
+  void sizeLists() {
+    static const int one = 1;
+    saveMemory(true);
     CK(cudaMemcpyAsync(S.ctl + kCtlActive, &one, sizeof(int), cudaMemcpyHostToDevice, stream));
+    CK(cudaMemcpyAsync(S.ctl + kCtlNeed, &one, sizeof(int), cudaMemcpyHostToDevice, stream));
     const int* gate = S.ctl + kCtlActive;
     launch_bin(S, gate, stream);
     launch_scan(S, gate, stream);
@@ -969,14 +1021,23 @@ struct System {
     if (precision == GDEM_FP64) launch_pairs64(S, gate, 0, stream);
     else launch_pairs32(S, gate, 0, stream);
     launch_row_scan(S, gate, stream);
+    launch_wall_rows(S, gate, stream);
     CK(cudaGetLastError());
     id_order = false;
-    checkPairCapacity();
+    int status = 0;   // (too short a wall list is what this finds)
+    CK(cudaStreamSynchronize(stream));
+    CK(cudaMemcpy(&status, S.status, sizeof(int), cudaMemcpyDeviceToHost));
+    status &= ~(int)kErrPairsFull;
+    CK(cudaMemcpy(S.status, &status, sizeof(int), cudaMemcpyHostToDevice));
+    checkCapacity();
+    lists_sized = true;
   }
 
   // Host AoS arrays (by ID) -> staging -> SoA state in ID order.
   void loadState(const double* x, const double* v, const double* w, const double* wbf,
                  const double* q, const double* F, const double* T) {
+    saveMemory(true);   // (the lists name the particles by slot)
+    lists_sized = !S.any_walls || S.wall_cap == S.cap;
     size_t n = (size_t)S.n;
     double* st = d_stage;
     double *dx = st, *dv = st + 3 * n, *dw = st + 6 * n, *dwb = st + 9 * n, *dq = st + 12 * n,
@@ -996,24 +1057,15 @@ struct System {
     id_order = true;
   }
 
-  // The contact-history tables alternate with every force evaluation.
-  void swapHist() { std::swap(S.hist_old, S.hist_new); }
-
-  // The table that evaluation e (1-based) writes is refilled every 512 of its
-  // uses with the tag e - 1, which none of its next 512 uses carries.
-  void maybeClearHistory(long e) {
-    if ((e % 512) >= 2) return;
-    size_t hc = size_t(1) << S.hist_new.log2cap;
-    unsigned long long v = tagged((1ull << kTagShift) - 1, (unsigned)(e - 1));
-    timed("hist_fill", [&] { launch_fill64(S.hist_new.keys, hc, v, stream); });
-  }
-
   // Pair-list rebuild: cells, counting sort, permutation into cell order,
   // pair search.  gate: the control word that tells gated kernels whether
   // this step rebuilds (plain launches), or null inside the graph's
   // conditional node.
   void rebuild(const int* gate) {
     id_order = false;
+    const bool fp64 = precision == GDEM_FP64;
+    if (prune_memory) timed("mem_clear", [&] { launch_mem_clear(S, gate, stream); });
+    timed("mem_save", [&] { launch_mem_save(S, gate, 1, fp64, stream); });
     timed("bin", [&] { launch_bin(S, gate, stream); });
     timed("scan", [&] { launch_scan(S, gate, stream); });
     timed("place", [&] { launch_place(S, gate, stream); });
@@ -1030,6 +1082,8 @@ struct System {
       timed("pairs_fill32", [&] { launch_pairs32(S, gate, 1, stream); });
     }
     timed("link", [&] { launch_link(S, gate, stream); });
+    if (S.any_walls) timed("wall_rows", [&] { launch_wall_rows(S, gate, stream); });
+    timed("mem_load", [&] { launch_mem_load(S, gate, fp64, stream); });
   }
   // Contact filter, pair kernel (contacts and walls), then the leapfrog
   // kernel: the sums of the shares and the leapfrog parts in flags (at the
@@ -1043,18 +1097,15 @@ struct System {
       timed("pairlaw32", [&] { launch_pairlaw32(S, stream); });
     }
     timed("move", [&] { launch_move(S, flags | kStepSum, precision == GDEM_FP32_SPLIT, stream); });
-    if (!prune_memory)
-      timed("hist_carry", [&] { launch_hist_carry(S, precision == GDEM_FP64, stream); });
   }
   // One force evaluation with plain launches: decide, gated rebuild, filter,
   // forces, move.
   void evaluate(int flags) {
-    maybeClearHistory(epoch + 1);
     timed("decide", [&] { launch_decide(S, cudaGraphConditionalHandle(), 0, stream); });
     rebuild(S.ctl + kCtlActive);
     forcesAndMove(flags);
+    lists_hold = true;
     ++epoch;
-    swapHist();
   }
 
   // The same evaluation as one graph: decide -> conditional node holding the
@@ -1107,30 +1158,27 @@ struct System {
     graph_conditional = conditional;
     return ex;
   }
-  // Graph of evaluation kind k (0: inside a call, 1: last of a call) for the
-  // current history-table parity; built on first use.
+  // Graph of evaluation kind k (0: inside a call, 1: last of a call); built
+  // on first use.
   void launchEvaluation(int k, int flags) {
-    maybeClearHistory(epoch + 1);
-    const int par = (int)(parity & 1);
-    if (!graph[k][par]) graph[k][par] = captureEvaluation(flags);
-    CK(cudaGraphLaunch(graph[k][par], stream));
+    if (!graph[k]) graph[k] = captureEvaluation(flags);
+    CK(cudaGraphLaunch(graph[k], stream));
+    lists_hold = true;
     ++epoch;
-    ++parity;
-    swapHist();
   }
 
   void init() {
-    sizePairList();
+    sizeLists();
     epoch_t0 = epoch + 1;   // the evaluation at t0 is the next one
     evaluate(kStepStoreFT);
-    ++parity;
-    launch_hist_zero_cumulative(S.hist_old, S.ctl, precision == GDEM_FP64, stream);
+    launch_mem_zero_cumulative(S, precision == GDEM_FP64, stream);
     CK(cudaStreamSynchronize(stream));
-    // size the contact filter's grid for the pair list just built and a
-    // quarter more for growth (the kernel loops over any excess)
-    int np = 0;
-    CK(cudaMemcpy(&np, S.ctl + kCtlPairs, sizeof(int), cudaMemcpyDeviceToHost));
-    S.filter_qblocks = filterBlocks((long long)(1.25 * np), S.nsm);
+    // size the contact filter's grid for the lists just built and a quarter
+    // more for growth (the kernel loops over any excess)
+    int ctl[kCtlWords];
+    CK(cudaMemcpy(ctl, S.ctl, sizeof(ctl), cudaMemcpyDeviceToHost));
+    S.filter_qblocks = filterBlocks((long long)(1.25 * ctl[kCtlPairs]), S.nsm);
+    S.filter_wblocks = (int)((1.25 * ctl[kCtlWallRows]) / 256.) + 1;
     invalidateGraphs();
     collectTimes();
     started = true;
@@ -1141,6 +1189,7 @@ struct System {
   // kick and -- except after the last -- the next opening kick and drift.
   void step(int nsteps) {
     if (nsteps <= 0) return;
+    if (!lists_sized) sizeLists();
     id_order = false;
     CK(cudaEventRecord(ev0, stream));
     timed("move", [&] { launch_move(S, kStepMove, precision == GDEM_FP32_SPLIT, stream); });
@@ -1150,13 +1199,12 @@ struct System {
       const bool is_last = k == nsteps - 1;
       // the pair list's allocation is checked every kCapacityCheck steps
       // within a call (and at its end); it grows before it can run short
-      if (k > 0 && k % kCapacityCheck == 0) checkPairCapacity();
+      if (k > 0 && k % kCapacityCheck == 0) checkCapacity();
       const bool graphs = use_graphs && !diag && !profiling;
       if (graphs) {
         launchEvaluation(is_last ? 1 : 0, is_last ? last : mid);
       } else {
         evaluate(is_last ? last : mid);
-        ++parity;
       }
     }
     CK(cudaEventRecord(ev1, stream));
@@ -1167,7 +1215,7 @@ struct System {
     last_ms = ms;
     collectTimes();
     evaluated = diag ? 1 : 2;
-    checkPairCapacity();
+    checkCapacity();
   }
   int readStatus() {
     int st = 0;
@@ -1418,6 +1466,7 @@ int gdem_pair_counts(gdem_handle h, int64_t* entries, int64_t* contacts) {
     System* s = sys(h);
     if (!s || !s->started) throw std::runtime_error("no force evaluation yet");
     unsigned long long* d = reinterpret_cast<unsigned long long*>(s->d_vstats);
+    s->saveMemory(false);
     launch_pair_counts(s->S, d, s->stream);
     unsigned long long r[2];
     CK(cudaMemcpyAsync(r, d, sizeof(r), cudaMemcpyDeviceToHost, s->stream));
@@ -1529,13 +1578,12 @@ int gdem_upload_history(gdem_handle h, int64_t n, const int* owner, const int* p
     System* s = sys(h);
     if (!s || !s->have_state || n < 0) throw std::runtime_error("upload the state first");
     DevState& S = s->S;
-    HistTable& t = S.hist_old;   // read by the next force evaluation
+    // the table replaces what the lists hold; the next evaluation rebuilds
+    // them and takes the memory from it
+    HistTable& t = S.hist;
     size_t hc = size_t(1) << t.log2cap;
-    // the next evaluation (epoch + 1) looks up tag epoch; the free slots get
-    // tag epoch - 1, which this table's next uses (tags epoch + 2, + 4, ...)
-    // never carry
-    const unsigned tag = (unsigned)s->epoch;
-    const unsigned long long empty = tagged((1ull << kTagShift) - 1, tag - 1u);
+    const unsigned tag = 0;
+    const unsigned long long empty = kEmptyKey;
     std::vector<unsigned long long> keys(hc, empty);
     bool fp64 = s->precision == GDEM_FP64;
     std::vector<double> vd(fp64 ? 9 * hc : 0);
@@ -1564,6 +1612,11 @@ int gdem_upload_history(gdem_handle h, int64_t n, const int* owner, const int* p
     CK(cudaMemcpy(t.keys, keys.data(), hc * sizeof(unsigned long long), cudaMemcpyHostToDevice));
     if (fp64) CK(cudaMemcpy(t.vals, vd.data(), vd.size() * sizeof(double), cudaMemcpyHostToDevice));
     else CK(cudaMemcpy(t.vals, vf.data(), vf.size() * sizeof(float), cudaMemcpyHostToDevice));
+    static const int zero = 0, one = 1;
+    CK(cudaMemcpyAsync(S.ctl + kCtlMemory, &zero, sizeof(int), cudaMemcpyHostToDevice, s->stream));
+    s->lists_hold = false;
+    CK(cudaMemcpyAsync(S.ctl + kCtlNeed, &one, sizeof(int), cudaMemcpyHostToDevice, s->stream));
+    CK(cudaStreamSynchronize(s->stream));
     return GDEM_OK;
   });
 }
@@ -1574,8 +1627,9 @@ int gdem_download_history(gdem_handle h, int64_t capacity, int64_t* count, int* 
     System* s = sys(h);
     if (!s || !s->have_state || !count) throw std::runtime_error("invalid arguments");
     DevState& S = s->S;
+    s->saveMemory(false);
     CK(cudaStreamSynchronize(s->stream));
-    HistTable& t = S.hist_old;   // written by the last force evaluation
+    HistTable& t = S.hist;
     const size_t hc = size_t(1) << t.log2cap;
     std::vector<unsigned long long> keys(hc);
     CK(cudaMemcpy(keys.data(), t.keys, hc * sizeof(unsigned long long), cudaMemcpyDeviceToHost));
@@ -1586,7 +1640,7 @@ int gdem_download_history(gdem_handle h, int64_t capacity, int64_t* count, int* 
     else CK(cudaMemcpy(vf.data(), t.vals, vf.size() * sizeof(float), cudaMemcpyDeviceToHost));
     struct Rec { int a, b; double v[9]; };
     std::vector<Rec> recs;
-    const unsigned tag = (unsigned)s->epoch & kTagMask;
+    const unsigned tag = 0;
     const unsigned idmask = (1u << kMaxIdBits) - 1u;
     const unsigned n = (unsigned)S.n;
     for (size_t k = 0; k < hc; ++k) {
@@ -2008,8 +2062,9 @@ static int writeReloadParticles(gdem_handle h, const char* path, bool hybrid) {
       for (size_t i = 0; i < n; ++i) rotationOf(&q[4 * i], &B[9 * i]);
     }
     auto refId = [&](size_t i) { return s->ref_ids.empty() ? (int)i + 1 : s->ref_ids[i]; };
-    // contact memory of the last evaluation: the table the next one reads
-    HistTable const& t = S.hist_old;
+    // contact memory of the last evaluation
+    s->saveMemory(false);
+    HistTable const& t = S.hist;
     const size_t hc = size_t(1) << t.log2cap;
     std::vector<unsigned long long> keys(hc);
     CK(cudaMemcpy(keys.data(), t.keys, hc * sizeof(unsigned long long), cudaMemcpyDeviceToHost));
@@ -2019,7 +2074,7 @@ static int writeReloadParticles(gdem_handle h, const char* path, bool hybrid) {
     if (fp64) CK(cudaMemcpy(vd.data(), t.vals, vd.size() * sizeof(double), cudaMemcpyDeviceToHost));
     else CK(cudaMemcpy(vf.data(), t.vals, vf.size() * sizeof(float), cudaMemcpyDeviceToHost));
     std::vector<std::vector<MapEntry>> maps(n);
-    const unsigned tag = (unsigned)s->epoch & kTagMask;
+    const unsigned tag = 0;
     const unsigned idmask = (1u << kMaxIdBits) - 1u;
     for (size_t k = 0; k < hc; ++k) {
       if (tagOf(keys[k]) != tag) continue;

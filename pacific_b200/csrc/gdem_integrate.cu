@@ -66,7 +66,6 @@ __global__ void k_decide(DevState S, cudaGraphConditionalHandle h, int use_handl
   S.ctl[kCtlKeptCold] = 0;
   S.ctl[kCtlKept2] = 0;
   S.ctl[kCtlRebuilds] += need ? 1 : 0;
-  if (need) S.ctl[kCtlPairs] = 0;
   if (use_handle) cudaGraphSetConditional(h, need ? 1u : 0u);
 }
 
@@ -91,6 +90,12 @@ __device__ __forceinline__ int buildKey(GridDesc const& bg, d3 x, int* status) {
 __global__ void k_bin(DevState S, const int* gate) {
   if (gatedOff(gate)) return;
   int s = blockIdx.x * blockDim.x + threadIdx.x;
+  // the lists are empty until the pair search and k_wall_rows fill them (their
+  // memory has been saved)
+  if (s == 0) {
+    S.ctl[kCtlPairs] = 0;
+    S.ctl[kCtlWallRows] = 0;
+  }
   if (s >= S.n) return;
   const int key = buildKey(S.bgrids[S.inst[s]], ld3(S.x, S.cap, s), S.status);
   S.skey[s] = key;
@@ -325,10 +330,24 @@ __device__ __forceinline__ void sumShares(DevState const& S, int t, TypeDesc con
       }
     }
     if (na & kNearWall) {
-      const float4* ws = static_cast<const float4*>(S.wshare) + 2 * (size_t)t;
-      const float4 a = ws[0], b = ws[1];
-      fx += a.x; fy += a.y; fz += a.z;
-      tx += b.x; ty += b.y; tz += b.z;
+      // the walls' own sum first, in wall order
+      const float4* ws = static_cast<const float4*>(S.wshare) +
+                         (size_t)kWallShare32 * S.wrow[t] * S.max_walls;
+      float wx = 0.f, wy = 0.f, wz = 0.f, ux = 0.f, uy = 0.f, uz = 0.f;
+      const int nw = S.grids[S.inst[t]].wall_count;
+      for (int k = 0; k < nw; ++k, ws += kWallShare32) {
+        const float4 a = ws[0];
+        if (__float_as_int(a.w) != tag) continue;
+        const float4 b = ws[1];
+        wx += a.x; wy += a.y; wz += a.z;
+        ux += b.x; uy += b.y; uz += b.z;
+        if (b.w != 0.f) {
+          const float4 c = ws[2];
+          ux += c.x; uy += c.y; uz += c.z;
+        }
+      }
+      fx += wx; fy += wy; fz += wz;
+      tx += ux; ty += uy; tz += uz;
     }
     F = mk(tp.weight[0] + (double)fx, tp.weight[1] + (double)fy, tp.weight[2] + (double)fz);
     T = mk((double)tx, (double)ty, (double)tz);
@@ -368,10 +387,23 @@ __device__ __forceinline__ void sumShares(DevState const& S, int t, TypeDesc con
       }
     }
     if (na & kNearWall) {
-      const double2* ws = static_cast<const double2*>(S.wshare) + 3 * (size_t)t;
-      const double2 a = ws[0], b = ws[1], c = ws[2];
-      F = F + mk(a.x, a.y, b.x);
-      T = T + mk(b.y, c.x, c.y);
+      const double2* ws = static_cast<const double2*>(S.wshare) +
+                          (size_t)kWallShare64 * S.wrow[t] * S.max_walls;
+      d3 Fw = mk(0., 0., 0.), Tw = mk(0., 0., 0.);
+      const int nw = S.grids[S.inst[t]].wall_count;
+      for (int k = 0; k < nw; ++k, ws += kWallShare64) {
+        const double2 a = ws[0];
+        if ((int)__double_as_longlong(a.x) != tag) continue;
+        const double2 b = ws[1], c = ws[2], d = ws[3];
+        Fw = Fw + mk(a.y, b.x, b.y);
+        Tw = Tw + mk(c.x, c.y, d.x);
+        if (d.y != 0.) {
+          const double2 e = ws[4], f = ws[5];
+          Tw = Tw + mk(e.x, e.y, f.x);
+        }
+      }
+      F = F + Fw;
+      T = T + Tw;
     }
   }
 }
@@ -459,8 +491,7 @@ __global__ void __launch_bounds__(kMoveBlock<kFast, kBasis>(), kBasis ? 2 : (kFa
 // once, from its lower ID): the FP32 bounding-sphere test, a superset of the
 // contacts; the kept pairs are listed for the pair kernel, which decides each
 // exactly, and both partners marked as candidates.  With walls, the first
-// pblocks blocks take one particle per thread and list (and mark) those near
-// a wall.  A warp tests `rounds` rounds of 32 pairs, then appends all it kept
+// pblocks blocks take the wall list.  A warp tests `rounds` rounds of 32 pairs, then appends all it kept
 // with one atomic: where the last evaluation kept more than an eighth of the
 // pairs (a packed bed, colliding convex bodies) up to kFilterRounds of them,
 // else one, whose append then overlaps the other warps' loads.  A grid-stride
@@ -470,18 +501,6 @@ __global__ void __launch_bounds__(kMoveBlock<kFast, kBasis>(), kBasis ? 2 : (kFa
 // and the appends, which were two atomics per kept pair and one per 32 pairs
 // on a single counter (250,000 packed spheres, 737,000 pairs kept: 32.9 us
 // then, 31.3 with plain marks and 1 round, 22.5 with 8 rounds).
-// Appends idx to list (length *count) for every lane whose pred holds (one
-// atomic per warp); every lane of the warp calls it.
-__device__ __forceinline__ void appendList(int* list, int* count, bool pred, int idx) {
-  const unsigned m = __ballot_sync(0xffffffffu, pred);
-  if (!m) return;
-  const int lane = threadIdx.x & 31;
-  int base = 0;
-  if (lane == 0) base = atomicAdd(count, __popc(m));
-  base = __shfl_sync(0xffffffffu, base, 0);
-  if (pred) list[base + __popc(m & ((1u << lane) - 1u))] = idx;
-}
-
 // Appends the kept pairs of a warp's rounds to a list that grows upwards
 // (dir 1) or downwards (dir -1) from list[0] and marks their partners: lane j
 // holds the ballot of round j in mine (0 beyond the rounds), round j's pairs
@@ -520,31 +539,94 @@ __device__ __forceinline__ void appendRounds(DevState const& S, int* flags, int*
 }
 
 // Whether particle t (posf: its FP32 continuous position) comes within the
-// margin of a wall box of its instance: the wall contacts can only come
-// from such particles.
-__device__ __forceinline__ bool nearWall(DevState const& S, int t) {
-  const int inst = S.inst[t];
-  GridDesc const& g = S.grids[inst];
-  if (!g.wall_count) return false;
-  // the centre wrapped back into the box, against the bounding radius
-  GridDesc const& bg = S.bgrids[inst];
+// margin (plus reach) of wall k of its instance: its contacts with that wall
+// can only come about then.  q: the centre wrapped back into the box.
+struct WallProbe {
+  float q[3], R;
+};
+__device__ __forceinline__ WallProbe wallProbe(DevState const& S, int t, GridDesc const& bg,
+                                               float reach) {
   const float4 pt = S.posf[t];
   const int wt = S.wrap[t];
-  const float q[3] = {pt.x - (float)wrapGet(wt, 0) * bg.Lf[0],
-                      pt.y - (float)wrapGet(wt, 1) * bg.Lf[1],
-                      pt.z - (float)wrapGet(wt, 2) * bg.Lf[2]};
-  for (int w = 0; w < g.wall_count; ++w) {
-    WallDesc const& wd = S.walls[g.wall_begin + w];
-    float d2 = 0.f;
+  return {{pt.x - (float)wrapGet(wt, 0) * bg.Lf[0], pt.y - (float)wrapGet(wt, 1) * bg.Lf[1],
+           pt.z - (float)wrapGet(wt, 2) * bg.Lf[2]},
+          pt.w + bg.filt_margin + reach};
+}
+__device__ __forceinline__ bool nearWall(WallDesc const& wd, WallProbe const& p) {
+  float d2 = 0.f;
 #pragma unroll
-    for (int d = 0; d < 3; ++d) {
-      const float o = fabsf(q[d] - (float)wd.centre[d]) - (float)wd.extent[d];
-      if (o > 0.f) d2 += o * o;
-    }
-    const float R = pt.w + bg.filt_margin;
-    if (d2 <= R * R) return true;
+  for (int d = 0; d < 3; ++d) {
+    const float o = fabsf(p.q[d] - (float)wd.centre[d]) - (float)wd.extent[d];
+    if (o > 0.f) d2 += o * o;
   }
-  return false;
+  return d2 <= p.R * p.R;
+}
+
+// The wall list: particles within the skin of a wall, which no other can
+// reach before the next rebuild (part of a rebuild, after k_copyback).
+__global__ void k_wall_rows(DevState S, const int* gate) {
+  if (gatedOff(gate)) return;
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  bool near = false;
+  if (t < S.n) {
+    const int inst = S.inst[t];
+    GridDesc const& bg = S.bgrids[inst];
+    const WallProbe p = wallProbe(S, t, bg, bg.skin_f);
+    for (int k = 0; k < bg.wall_count && !near; ++k) near = nearWall(S.walls[bg.wall_begin + k], p);
+  }
+  const unsigned m = __ballot_sync(0xffffffffu, near);
+  const int lane = threadIdx.x & 31;
+  int base = 0;
+  if (lane == 0 && m) base = atomicAdd(S.ctl + kCtlWallRows, __popc(m));
+  const int row = __shfl_sync(0xffffffffu, base, 0) + __popc(m & ((1u << lane) - 1u));
+  if (t >= S.n) return;
+  S.wrow[t] = near ? row : -1;
+  if (!near) return;
+  if (row < S.wall_cap) S.wlist[row] = t;
+  else raise(S.status, kErrPairsFull);   // (grown before the next call)
+}
+
+// This evaluation's wall items: for spheres every near (particle, wall) slot
+// of the wall list, else the particles near any wall (their walls are taken in
+// turn: a polyhedron's support vertex runs through them).
+__device__ __forceinline__ void filterWalls(DevState const& S, int* flags, int nblocks) {
+  const unsigned full = 0xffffffffu;
+  const int lane = threadIdx.x & 31;
+  const int nr = listedWalls(S);
+  for (int r0 = (int)(blockIdx.x * blockDim.x + threadIdx.x) & ~31; r0 < nr;
+       r0 += nblocks * blockDim.x) {   // warp-uniform
+    const int row = r0 + lane;
+    int count = 0, t = 0, begin = 0, nw = 0;
+    WallProbe p{};
+    if (row < nr) {
+      t = S.wlist[row];
+      GridDesc const& bg = S.bgrids[S.inst[t]];
+      p = wallProbe(S, t, bg, 0.f);
+      begin = bg.wall_begin;
+      nw = bg.wall_count;
+      for (int k = 0; k < nw; ++k) count += nearWall(S.walls[begin + k], p);
+      if (count) flags[t] = (int)kCandidate;
+      if (S.any_convex) count = min(count, 1);
+    }
+    int incl = count;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int y = __shfl_up_sync(full, incl, o);
+      if (lane >= o) incl += y;
+    }
+    const int total = __shfl_sync(full, incl, 31);
+    if (!total) continue;
+    int at = 0;
+    if (lane == 0) at = atomicAdd(S.ctl + kCtlWork, total);
+    at = __shfl_sync(full, at, 0) + incl - count;
+    if (!count) continue;
+    if (S.any_convex) {
+      S.work[at] = row;
+    } else {
+      for (int k = 0; k < nw; ++k)
+        if (nearWall(S.walls[begin + k], p)) S.work[at++] = row * S.max_walls + k;
+    }
+  }
 }
 
 // kSplit: FP32-split with non-spherical classes (the kept pairs in two lists).
@@ -554,13 +636,10 @@ __global__ void __launch_bounds__(256, 8) k_filter(DevState S, int pblocks) {
   const int lane = threadIdx.x & 31;
   int* flags = contactFlags(S);
   if ((int)blockIdx.x < pblocks) {
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    const bool near = t < S.n && nearWall(S, t);
-    if (near) flags[t] = (int)kCandidate;
-    appendList(S.work, S.ctl + kCtlWork, near, t);
+    filterWalls(S, flags, pblocks);
     return;
   }
-  const int np = S.ctl[kCtlPairs];
+  const int np = listedPairs(S);
   const long long wq = ((long long)((int)blockIdx.x - pblocks) * blockDim.x + threadIdx.x) >> 5;
   const long long nwq = ((long long)(gridDim.x - pblocks) * blockDim.x) >> 5;
   // (all warp-uniform) round j of a warp is the grid's j-th sweep over the list
@@ -630,7 +709,7 @@ __global__ void __launch_bounds__(256, 8) k_filter(DevState S, int pblocks) {
 // known on the device only.
 __global__ void __launch_bounds__(256) k_link(DevState S, const int* gate) {
   if (gatedOff(gate)) return;
-  const int np = S.ctl[kCtlPairs];
+  const int np = listedPairs(S);
   for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < np; k += gridDim.x * blockDim.x) {
     const int2 pr = S.upairs[k];
     const int t = pr.x;
@@ -734,22 +813,114 @@ __global__ void k_coordination_by_id(DevState S, int* out, int id_base) {
   out[i] = c;
 }
 
-// Zeroes the cumulative tangential and rolling memories of every entry of
-// the given evaluation (Component::setContactMapCumulativeFeaturesToZero,
-// Component.cpp:842-851).
-template <typename V>
-__global__ void k_hist_zero_cumulative(HistTable t, const int* ctl) {
-  int s = blockIdx.x * blockDim.x + threadIdx.x;
-  if (s >= (1 << t.log2cap)) return;
-  if (tagOf(t.keys[s]) != ((unsigned)ctl[kCtlEpoch] & kTagMask)) return;
-  V* v = static_cast<V*>(t.vals) + 9 * (size_t)s;
-  v[0] = v[1] = v[2] = 0;
-  v[6] = v[7] = v[8] = 0;
+// Contact memory between the lists and the table.  Entries 0 .. pairs - 1 are
+// the compact pair list's, then come the wall list's slots.
+__device__ __forceinline__ bool memEntry(DevState const& S, int np, long long i, MemView& m,
+                                         long long& at, unsigned long long& key) {
+  if (i < np) {
+    const int2 pr = S.upairs[i];
+    m = S.pmem;
+    at = i;
+    key = pairKey(S.id[pr.x], S.id[(unsigned)pr.y & ((1u << 27) - 1u)]);
+    return true;
+  }
+  m = S.wmem;
+  at = i - np;
+  const int row = (int)(at / S.max_walls), k = (int)(at % S.max_walls);
+  const int t = S.wlist[row];
+  key = wallKey(S.id[t], k);
+  return k < S.grids[S.inst[t]].wall_count;
 }
 
-__global__ void k_fill64(unsigned long long* p, size_t n, unsigned long long value) {
-  size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) p[i] = value;
+// Frees the table's slots before the lists' memory is saved (the plain step).
+__global__ void k_mem_clear(DevState S, const int* gate) {
+  if (gatedOff(gate) || !S.ctl[kCtlMemory]) return;
+  const size_t cap = size_t(1) << S.hist.log2cap;
+  for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < cap;
+       i += (size_t)gridDim.x * blockDim.x)
+    S.hist.keys[i] = kEmptyKey;
+}
+
+// The memory that evaluation now (the counter less back) left in the lists, or
+// any there (the coupled step), into the table.
+template <typename T>
+__global__ void k_mem_save(DevState S, const int* gate, int back) {
+  if (gatedOff(gate) || !S.ctl[kCtlMemory]) return;
+  const int now = S.ctl[kCtlEpoch] - back;
+  const int np = listedPairs(S);
+  const long long ne = np + (long long)listedWalls(S) * S.max_walls;
+  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < ne;
+       i += (long long)gridDim.x * blockDim.x) {
+    MemView m;
+    long long at;
+    unsigned long long key;
+    if (!memEntry(S, np, i, m, at, key)) continue;
+    if (!remembered(S, memEvaluation(m, at, T()), now + 1)) continue;
+    T v[9];
+    memLoad(m, at, v, true);
+    const int s = histInsert(S.hist, key, 0);
+    if (s < 0) { raise(S.status, kErrHashFull); continue; }
+    T* d = static_cast<T*>(S.hist.vals) + 9 * (size_t)s;
+#pragma unroll
+    for (int k = 0; k < 9; ++k) d[k] = v[k];
+  }
+}
+
+// The table's memory into the new lists, as left by the last evaluation; from
+// here on the lists hold it.
+template <typename T>
+__global__ void k_mem_load(DevState S, const int* gate) {
+  if (gatedOff(gate)) return;
+  const int last = S.ctl[kCtlEpoch] - 1;
+  const int np = listedPairs(S);
+  const long long ne = np + (long long)listedWalls(S) * S.max_walls;
+  const long long i0 = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i0 == 0) {
+    S.ctl[kCtlMemory] = 1;
+    S.ctl[kCtlWallRowsMax] = max(S.ctl[kCtlWallRowsMax], S.ctl[kCtlWallRows]);
+  }
+  for (long long i = i0; i < ne; i += (long long)gridDim.x * blockDim.x) {
+    MemView m;
+    long long at;
+    unsigned long long key;
+    const bool used = memEntry(S, np, i, m, at, key);
+    const int s = used ? histFind(S.hist, key, 0) : -1;
+    if (s < 0) { memForget(m, at, T()); continue; }
+    const T* d = static_cast<const T*>(S.hist.vals) + 9 * (size_t)s;
+    T v[9];
+#pragma unroll
+    for (int k = 0; k < 9; ++k) v[k] = d[k];
+    memStore(m, at, v, last, true);
+  }
+}
+
+// Zeroes the cumulative tangential and rolling memories of every contact of
+// the last evaluation (Component::setContactMapCumulativeFeaturesToZero,
+// Component.cpp:842-851), in the lists and, in the coupled step, of the pairs
+// the table keeps.
+template <typename V>
+__global__ void k_mem_zero_cumulative(DevState S) {
+  const long long i0 = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  const long long stride = (long long)gridDim.x * blockDim.x;
+  const int now = S.ctl[kCtlEpoch];
+  const int np = listedPairs(S);
+  const long long ne = np + (long long)listedWalls(S) * S.max_walls;
+  for (long long i = i0; i < ne; i += stride) {
+    MemView m = i < np ? S.pmem : S.wmem;
+    const long long at = i < np ? i : i - np;
+    const int e = memEvaluation(m, at, V());
+    if (!remembered(S, e, now + 1)) continue;
+    V v[9];
+    memLoad(m, at, v, true);
+    v[0] = v[1] = v[2] = v[6] = v[7] = v[8] = 0;
+    memStore(m, at, v, e, true);
+  }
+  if (S.prune) return;
+  for (long long i = i0; i < (1ll << S.hist.log2cap); i += stride) {
+    if (tagOf(S.hist.keys[i]) != 0) continue;
+    V* v = static_cast<V*>(S.hist.vals) + 9 * (size_t)i;
+    v[0] = v[1] = v[2] = v[6] = v[7] = v[8] = 0;
+  }
 }
 
 // Orientation matrix of the quaternion q (x, y, z, w) with the expression
@@ -906,15 +1077,14 @@ __global__ void k_vstats_final(const double* part, int nparts, int n, double* ou
   if (threadIdx.x == 0) { out[0] = smax[0]; out[1] = n > 0 ? ssum[0] / n : 0.; }
 }
 
-// Sum of the pair-list segment lengths and count of the history keys of
-// the last force evaluation.
+// Sum of the pair-list segment lengths and count of the contact-memory table's
+// entries (the host saves the lists into it first).
 __global__ void k_pair_counts(DevState S, unsigned long long* out) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   unsigned long long e = 0, c = 0;
   if (i < S.n) e = (unsigned long long)S.npairs[i];
-  const unsigned tag = (unsigned)S.ctl[kCtlEpoch] & kTagMask;
-  int cap = 1 << S.hist_old.log2cap;
-  for (int k = i; k < cap; k += gridDim.x * blockDim.x) c += tagOf(S.hist_old.keys[k]) == tag;
+  const long long cap = 1ll << S.hist.log2cap;
+  for (long long k = i; k < cap; k += gridDim.x * blockDim.x) c += tagOf(S.hist.keys[k]) == 0;
   for (int o = 16; o > 0; o >>= 1) {
     e += __shfl_down_sync(0xffffffffu, e, o);
     c += __shfl_down_sync(0xffffffffu, c, o);
@@ -953,11 +1123,16 @@ int filterBlocks(long long pairs, int nsm) {
 }
 void launch_filter(DevState const& S, cudaStream_t st) {
   if (!S.n) return;
-  const int pblocks = S.any_walls ? blocks(S.n, 256) : 0;
+  // an eighth of the particles until the leapfrog start has counted the wall list
+  const int pblocks =
+      S.any_walls ? (S.filter_wblocks > 0 ? S.filter_wblocks : blocks(blocks(S.n, 8), 256)) : 0;
   // about 4 pairs per particle until the leapfrog start has counted them
   const int qblocks = S.filter_qblocks > 0 ? S.filter_qblocks : filterBlocks(4ll * S.n, S.nsm);
   if (S.any_convex && !S.pos64) k_filter<true><<<pblocks + qblocks, 256, 0, st>>>(S, pblocks);
   else k_filter<false><<<pblocks + qblocks, 256, 0, st>>>(S, pblocks);
+}
+void launch_wall_rows(DevState const& S, const int* gate, cudaStream_t st) {
+  if (S.n && S.any_walls) k_wall_rows<<<blocks(S.n, 256), 256, 0, st>>>(S, gate);
 }
 void launch_link(DevState const& S, const int* gate, cudaStream_t st) {
   if (S.n) k_link<<<4 * S.nsm, 256, 0, st>>>(S, gate);
@@ -991,8 +1166,20 @@ void launch_move(DevState const& S, int flags, int fast, cudaStream_t st) {
 void launch_append_particle(DevState const& S, NewParticle const& p, cudaStream_t st) {
   k_append_particle<<<1, 32, 0, st>>>(S, p);
 }
-void launch_fill64(unsigned long long* p, size_t n, unsigned long long value, cudaStream_t st) {
-  if (n) k_fill64<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(p, n, value);
+void launch_mem_clear(DevState const& S, const int* gate, cudaStream_t st) {
+  k_mem_clear<<<8 * S.nsm, 256, 0, st>>>(S, gate);
+}
+void launch_mem_save(DevState const& S, const int* gate, int back, int fp64, cudaStream_t st) {
+  if (fp64) k_mem_save<double><<<8 * S.nsm, 256, 0, st>>>(S, gate, back);
+  else k_mem_save<float><<<8 * S.nsm, 256, 0, st>>>(S, gate, back);
+}
+void launch_mem_load(DevState const& S, const int* gate, int fp64, cudaStream_t st) {
+  if (fp64) k_mem_load<double><<<8 * S.nsm, 256, 0, st>>>(S, gate);
+  else k_mem_load<float><<<8 * S.nsm, 256, 0, st>>>(S, gate);
+}
+void launch_mem_zero_cumulative(DevState const& S, int fp64, cudaStream_t st) {
+  if (fp64) k_mem_zero_cumulative<double><<<8 * S.nsm, 256, 0, st>>>(S);
+  else k_mem_zero_cumulative<float><<<8 * S.nsm, 256, 0, st>>>(S);
 }
 void launch_pair_counts(DevState const& S, unsigned long long* out, cudaStream_t st) {
   cudaMemsetAsync(out, 0, 2 * sizeof(unsigned long long), st);
@@ -1024,41 +1211,4 @@ void launch_cells_by_id(DevState const& S, int* ijk, int id_base, cudaStream_t s
 void launch_coordination_by_id(DevState const& S, int* out, int id_base, cudaStream_t st) {
   if (S.n) k_coordination_by_id<<<blocks(S.n, 256), 256, 0, st>>>(S, out, id_base);
 }
-// Contact memory of a step that does not prune it (GrainsCoupledWithFluid::
-// Simulation, Fluid/src/GrainsCoupledWithFluid.cpp:135-205, runs the
-// collision application without Grains::computeParticlesForceAndTorque's
-// setContactMapToFalse / updateContactMap, Component/src/Component.cpp:
-// 567-593): every entry of the previous evaluation's table that this
-// evaluation did not rewrite -- a contact that has ended -- is carried into
-// this evaluation's table unchanged, so that the pair, if it touches again,
-// resumes its tangential spring.  Runs after the pair kernel.
-template <typename T>
-__global__ void k_hist_carry(HistTable old_t, HistTable new_t, const int* ctl, int* status) {
-  const unsigned tag = (unsigned)ctl[kCtlEpoch], tag_old = tag - 1u;
-  const size_t cap = size_t(1) << old_t.log2cap;
-  const T* src = static_cast<const T*>(old_t.vals);
-  T* dst = static_cast<T*>(new_t.vals);
-  for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < cap;
-       i += (size_t)gridDim.x * blockDim.x) {
-    const unsigned long long k = old_t.keys[i];
-    if (tagOf(k) != (tag_old & kTagMask)) continue;
-    const unsigned long long base = k & ((1ull << kTagShift) - 1ull);
-    if (histFind(new_t, base, tag) >= 0) continue;   // rewritten this evaluation
-    const int s = histInsert(new_t, base, tag);
-    if (s < 0) { raise(status, kErrHashFull); continue; }
-#pragma unroll
-    for (int j = 0; j < 9; ++j) dst[(size_t)s * 9 + j] = src[i * 9 + j];
-  }
-}
-void launch_hist_carry(DevState const& S, int fp64, cudaStream_t st) {
-  if (fp64) k_hist_carry<double><<<4 * S.nsm, 256, 0, st>>>(S.hist_old, S.hist_new, S.ctl, S.status);
-  else k_hist_carry<float><<<4 * S.nsm, 256, 0, st>>>(S.hist_old, S.hist_new, S.ctl, S.status);
-}
-
-void launch_hist_zero_cumulative(HistTable const& t, const int* ctl, int fp64, cudaStream_t st) {
-  int cap = 1 << t.log2cap;
-  if (fp64) k_hist_zero_cumulative<double><<<blocks(cap, 256), 256, 0, st>>>(t, ctl);
-  else k_hist_zero_cumulative<float><<<blocks(cap, 256), 256, 0, st>>>(t, ctl);
-}
-
 }  // namespace gdem

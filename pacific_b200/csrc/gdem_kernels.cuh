@@ -61,6 +61,7 @@ void launch_filter(DevState const& S, cudaStream_t st);
 // tested in one round each).
 int filterBlocks(long long pairs, int nsm);
 void launch_link(DevState const& S, const int* gate, cudaStream_t st);
+void launch_wall_rows(DevState const& S, const int* gate, cudaStream_t st);
 void launch_diag_prefill(DevState const& S, cudaStream_t st);
 void launch_place(DevState const& S, const int* gate, cudaStream_t st);
 void launch_cellsort(DevState const& S, const int* gate, cudaStream_t st);
@@ -69,15 +70,18 @@ void launch_copyback(DevState const& S, const int* gate, cudaStream_t st);
 // fast: the FP32-split leapfrog (reciprocals, series; not the reference's
 // operation order)
 void launch_move(DevState const& S, int flags, int fast, cudaStream_t st);
-void launch_fill64(unsigned long long* p, size_t n, unsigned long long value, cudaStream_t st);
 void launch_scatter_by_id(DevState const& S, double* x, double* v, double* w, double* wbf,
                           double* q, double* F, double* T, int id_base, cudaStream_t st);
 void launch_basis_by_id(DevState const& S, double* out, int id_base, cudaStream_t st);
 void launch_cells_by_id(DevState const& S, int* ijk, int id_base, cudaStream_t st);
 // needs the diagnostics records (pair_delta, wall_delta) of the last evaluation
 void launch_coordination_by_id(DevState const& S, int* out, int id_base, cudaStream_t st);
-void launch_hist_zero_cumulative(HistTable const& t, const int* ctl, int fp64, cudaStream_t st);
-void launch_hist_carry(DevState const& S, int fp64, cudaStream_t st);
+// contact memory: the table emptied, the lists' memory (of the evaluation
+// counter less back) saved into it, the new lists loaded from it
+void launch_mem_clear(DevState const& S, const int* gate, cudaStream_t st);
+void launch_mem_save(DevState const& S, const int* gate, int back, int fp64, cudaStream_t st);
+void launch_mem_load(DevState const& S, const int* gate, int fp64, cudaStream_t st);
+void launch_mem_zero_cumulative(DevState const& S, int fp64, cudaStream_t st);
 void launch_load_state(DevState const& S, const double* x, const double* v, const double* w,
                        const double* wbf, const double* q, const double* F, const double* T,
                        const int* type_by_id, const int* inst_by_id, cudaStream_t st);

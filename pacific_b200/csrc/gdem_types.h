@@ -39,6 +39,9 @@ enum CtlWords : int {
   kCtlKeptCold = 9,  // kept pairs not in contact at the last evaluation (listed from the back)
   kCtlKept2 = 10,    // of those, the pairs the first search iteration left undecided (kept2)
   kCtlRounds = 11,   // rounds of 32 pairs per append of this evaluation's contact filter
+  kCtlMemory = 12,   // the pair and wall lists hold the contact memory (else the table does)
+  kCtlWallRows = 13, // particles of the wall list
+  kCtlWallRowsMax = 14,  // most wall-list particles of any rebuild since the last allocation check
   kCtlWords = 16
 };
 
@@ -48,6 +51,7 @@ enum CtlWords : int {
 struct GridDesc {
   double lc_origin[3];   // linked-cell origin (shifted by one cell where periodic)
   double edge[3];        // cell edge lengths
+  double inv_edge[3];    // 1 / edge (reference cells away from cell faces)
   double L[3];           // domain size: the periodic translation vector
   int nb[3];             // cells per direction (incl. the 2 periodic layers)
   int periodic[3];
