@@ -253,11 +253,22 @@ __device__ __forceinline__ void contactLaw32(ModelDesc const& m, double dt, Cont
 
 // Lists a candidate when its bounding spheres are closer than the skin, with
 // a relative margin of 4e-6 that covers the FP32 rounding of the test.
-// kFill = false: returns the row length of slot t.  kFill = true: writes the
-// row (its length known from the counting pass), orders it and returns its
-// number of upper entries.
+// kFill = false: returns the row length of slot t and keeps its first
+// kCandKept entries.  kFill = true: writes the row (its length known from the
+// counting pass) from the kept entries, or by a second search when there were
+// more, orders it and returns its number of upper entries.
 template <bool kFill>
 __device__ __forceinline__ int listPairs32(DevState const& S, int t) {
+  const int cap = S.cap;
+  if (kFill && S.npairs[t] <= kCandKept) {
+    const int len = S.npairs[t];
+    int* row = S.pairs + S.pair_off[t];
+    if (len <= kSortKept)
+      return rankEntriesUpperFirst(row, len, S.id, S.id[t],
+                                   [&](int k) { return S.cand[(size_t)k * cap + t]; });
+    for (int k = 0; k < len; ++k) row[k] = S.cand[(size_t)k * cap + t];
+    return sortEntriesUpperFirst(row, len, S.id, S.id[t]);
+  }
   const int4 cc = S.cellc[t];
   GridDesc const& g = S.bgrids[cc.w];
   const float4 ha = S.offh[t];
@@ -268,7 +279,7 @@ __device__ __forceinline__ int listPairs32(DevState const& S, int t) {
   const float ex = g.edge_f[0], ey = g.edge_f[1], ez = g.edge_f[2];
   forEachCandidate(S.cell_start, g, cc, [&](int u, int dcx, int dj, int dk, int sx, int sy, int sz) {
     if (u == t) return;
-    const float4 hb = offh[u];
+    const float4 hb = __ldg(&offh[u]);
     // lower slot first, so both directions of a pair evaluate the same
     // expression and agree on the (conservative) decision
     const bool lo = t < u;
@@ -279,7 +290,12 @@ __device__ __forceinline__ int listPairs32(DevState const& S, int t) {
     float dz = fmaf(s * (float)dk, ez, h1.z - h0.z);
     float R = (h0.w + h1.w + g.skin_f) * (1.f + 4.e-6f);
     if (dx * dx + dy * dy + dz * dz > R * R) return;
-    if (kFill && cnt < room) out[cnt] = u | (shiftCode(sx, sy, sz) << 27);
+    const int e = u | (shiftCode(sx, sy, sz) << 27);
+    if (kFill) {
+      if (cnt < room) out[cnt] = e;
+    } else if (cnt < kCandKept) {
+      S.cand[(size_t)cnt * cap + t] = e;
+    }
     ++cnt;
   });
   if (!kFill) return cnt;

@@ -34,11 +34,22 @@ namespace {
 // a relative margin of 1e-12, for periodic images whose two orientations
 // round the image translation differently); the pair kernel then decides
 // contact exactly (distance < 0) in lower-ID-first orientation.
-// kFill = false: returns the row length of slot t.  kFill = true: writes the
-// row (its length known from the counting pass), orders it and returns its
-// number of upper entries.
+// kFill = false: returns the row length of slot t and keeps its first
+// kCandKept entries.  kFill = true: writes the row (its length known from the
+// counting pass) from the kept entries, or by a second search when there were
+// more, orders it and returns its number of upper entries.
 template <bool kFill>
 __device__ __forceinline__ int listPairs64(DevState const& S, int t) {
+  const int cap = S.cap;
+  if (kFill && S.npairs[t] <= kCandKept) {
+    const int len = S.npairs[t];
+    int* row = S.pairs + S.pair_off[t];
+    if (len <= kSortKept)
+      return rankEntriesUpperFirst(row, len, S.id, S.id[t],
+                                   [&](int k) { return S.cand[(size_t)k * cap + t]; });
+    for (int k = 0; k < len; ++k) row[k] = S.cand[(size_t)k * cap + t];
+    return sortEntriesUpperFirst(row, len, S.id, S.id[t]);
+  }
   const int4 cc = S.cellc[t];
   GridDesc const& g = S.bgrids[cc.w];
   const double4 pa = S.pos64[t];
@@ -48,13 +59,20 @@ __device__ __forceinline__ int listPairs64(DevState const& S, int t) {
   const double4* __restrict__ pos = S.pos64;
   forEachCandidate(S.cell_start, g, cc, [&](int u, int dcx, int dj, int dk, int sx, int sy, int sz) {
     if (u == t) return;
-    const double4 pb = pos[u];
+    const double2* pu = reinterpret_cast<const double2*>(pos + u);
+    const double2 p0 = __ldg(pu), p1 = __ldg(pu + 1);
+    const double4 pb = make_double4(p0.x, p0.y, p1.x, p1.y);
     d3 shift = mk(sx * g.L[0], sy * g.L[1], sz * g.L[2]);
     d3 d = u > t ? (mk(pb.x, pb.y, pb.z) + shift) - mk(pa.x, pa.y, pa.z)
                  : (mk(pa.x, pa.y, pa.z) + (-shift)) - mk(pb.x, pb.y, pb.z);
     double R = pa.w + pb.w;
     if (norm(d) - R > g.skin + 1.0e-12 * R) return;
-    if (kFill && cnt < room) out[cnt] = u | (shiftCode(sx, sy, sz) << 27);
+    const int e = u | (shiftCode(sx, sy, sz) << 27);
+    if (kFill) {
+      if (cnt < room) out[cnt] = e;
+    } else if (cnt < kCandKept) {
+      S.cand[(size_t)cnt * cap + t] = e;
+    }
     ++cnt;
   });
   if (!kFill) return cnt;

@@ -1,6 +1,7 @@
 // gdem_device.cuh -- device-side state and helpers for the Grains3D DEM step.
 #pragma once
 #include <cuda_runtime.h>
+#include <limits.h>
 #include <stdint.h>
 
 #include "gdem_types.h"
@@ -214,6 +215,9 @@ struct DevState {
   // total of the last rebuild)
   int* pairs; int* npairs; int* pair_off;
   int pair_cap;
+  // candidates found by the counting pass of a rebuild, kCandKept per particle
+  // ([k * cap + t]; the download staging, free during a step)
+  int* cand;
   int* pair_scan_tmp;     // tile sums of the pair-count scan
   double* hydro;          // coupled runs: hydrodynamic force and torque by particle ID (6 each), or null
   int2* upairs;           // compact pair list: (slot, entry) of every upper entry, ctl[kCtlPairs] of them
@@ -409,6 +413,7 @@ __device__ __forceinline__ void forEachCandidate(const int* __restrict__ cs, Gri
       if (!g.periodic[0]) { ilo = max(ilo, 0); ihi = min(ihi, nbx - 1); }
       const int b0 = cs[row + ilo], b1 = cs[row + cc.x], b2 = cs[row + cc.x + 1],
                 b3 = cs[row + ihi + 1];
+#pragma unroll 4
       for (int u = b0; u < b3; ++u) fn(u, u < b1 ? -1 : (u < b2 ? 0 : 1), dj, dk, 0, shy, shz);
       if (g.periodic[0]) {
         const int nin = nbx - 2;
@@ -449,6 +454,43 @@ __device__ __forceinline__ int sortEntriesUpperFirst(int* seg, int cnt, const in
   }
   return nup;
 }
+
+// The same for a row of at most kSortKept entries given by load(k), in
+// registers: each entry goes to its rank.  (The insertion sort above reads IDs
+// and entries from memory at every comparison.)
+constexpr int kSortKept = 12;
+template <typename Load>
+__device__ __forceinline__ int rankEntriesUpperFirst(int* seg, int cnt, const int* id, int idt,
+                                                     Load&& load) {
+  int e[kSortKept], key[kSortKept];
+  int nup = 0;
+#pragma unroll
+  for (int k = 0; k < kSortKept; ++k) {
+    key[k] = INT_MAX;
+    if (k < cnt) e[k] = load(k);
+  }
+#pragma unroll
+  for (int k = 0; k < kSortKept; ++k) {
+    if (k < cnt) {
+      const int idu = id[e[k] & ((1 << 27) - 1)];
+      key[k] = idu > idt ? idu : (1 << 30) | idu;
+      nup += idu > idt ? 1 : 0;
+    }
+  }
+#pragma unroll
+  for (int k = 0; k < kSortKept; ++k) {
+    int rank = 0;
+#pragma unroll
+    for (int j = 0; j < kSortKept; ++j)
+      rank += (key[j] < key[k] || (j < k && key[j] == key[k])) ? 1 : 0;
+    if (k < cnt) seg[rank] = e[k];
+  }
+  return nup;
+}
+
+// Candidates per particle the counting pass keeps for the filling one (of the
+// 44 ints the staging has room for): a longer row is searched again.
+constexpr int kCandKept = 44;
 
 // Row length of a particle with cnt candidates: at most kRowMax (an entry's
 // position in its row is kept in 16 bits); more raises kErrPairsFull.

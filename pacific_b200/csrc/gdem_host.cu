@@ -934,6 +934,7 @@ struct System {
     CK(cudaMemset(S.F, 0, 3 * c * sizeof(double)));
     CK(cudaMemset(S.T, 0, 3 * c * sizeof(double)));
     d_stage = alloc<double>(22 * c);
+    S.cand = reinterpret_cast<int*>(d_stage);
     d_type_id = alloc<int>(c);
     d_inst_id = alloc<int>(c);
     d_vstats = alloc<double>(2 * ((c + 255) / 256) + 2);
@@ -1065,8 +1066,8 @@ struct System {
     launch_scan(S, gate, stream);
     launch_place(S, gate, stream);
     launch_cellsort(S, gate, stream);
-    launch_permute(S, gate, stream);
-    launch_copyback(S, gate, stream);
+    launch_permute(S, gate, 1, stream);
+    launch_copyback(S, gate, 1, stream);
     if (precision == GDEM_FP64) launch_pairs64(S, gate, 0, stream);
     else launch_pairs32(S, gate, 0, stream);
     launch_row_scan(S, gate, stream);
@@ -1119,8 +1120,8 @@ struct System {
     timed("scan", [&] { launch_scan(S, gate, stream); });
     timed("place", [&] { launch_place(S, gate, stream); });
     timed("cellsort", [&] { launch_cellsort(S, gate, stream); });
-    timed("permute", [&] { launch_permute(S, gate, stream); });
-    timed("copyback", [&] { launch_copyback(S, gate, stream); });
+    timed("permute", [&] { launch_permute(S, gate, 0, stream); });
+    timed("copyback", [&] { launch_copyback(S, gate, 0, stream); });
     if (precision == GDEM_FP64) {
       timed("pairs_count64", [&] { launch_pairs64(S, gate, 0, stream); });
       timed("row_scan", [&] { launch_row_scan(S, gate, stream); });

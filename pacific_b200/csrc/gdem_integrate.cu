@@ -215,7 +215,9 @@ __global__ void k_cellsort(DevState S, const int* gate) {
 // Gathers the state into cell order (second buffers) and writes the compact
 // arrays of the pair search: the cell, the FP64 position + radius (FP64
 // mode) or the FP32 offset from the cell's lower corner + radius (FP32-split).
-__global__ void k_permute(DevState S, const int* gate) {
+// forces: F, T too (before the first step of a call; a rebuild inside a call
+// comes between their last use and the last evaluation's, which writes them).
+__global__ void k_permute(DevState S, const int* gate, int forces) {
   if (gatedOff(gate)) return;
   int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= S.n) return;
@@ -228,8 +230,10 @@ __global__ void k_permute(DevState S, const int* gate) {
   st3(S.v2, cap, t, ld3(S.v, cap, s));
   st3(S.w2, cap, t, ld3(S.w, cap, s));
   if (S.wbf_state) st3(S.wbf2, cap, t, ld3(S.wbf, cap, s));
-  st3(S.F2, cap, t, ld3(S.F, cap, s));
-  st3(S.T2, cap, t, ld3(S.T, cap, s));
+  if (forces) {
+    st3(S.F2, cap, t, ld3(S.F, cap, s));
+    st3(S.T2, cap, t, ld3(S.T, cap, s));
+  }
 #pragma unroll
   for (int k = 0; k < 4; ++k) S.q2[k * cap + t] = S.q[k * cap + s];
   if (S.basis) {
@@ -254,7 +258,7 @@ __global__ void k_permute(DevState S, const int* gate) {
 
 // Second buffers back into the current ones; the wraps since the rebuild
 // start again from zero and the FP32 position becomes the rebuild's.
-__global__ void k_copyback(DevState S, const int* gate) {
+__global__ void k_copyback(DevState S, const int* gate, int forces) {
   if (gatedOff(gate)) return;
   int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= S.n) return;
@@ -265,7 +269,7 @@ __global__ void k_copyback(DevState S, const int* gate) {
     const size_t k = (size_t)d * cap + t;
     S.x[k] = S.x2[k]; S.v[k] = S.v2[k]; S.w[k] = S.w2[k];
     if (S.wbf_state) S.wbf[k] = S.wbf2[k];
-    S.F[k] = S.F2[k]; S.T[k] = S.T2[k];
+    if (forces) { S.F[k] = S.F2[k]; S.T[k] = S.T2[k]; }
   }
 #pragma unroll
   for (int k = 0; k < 4; ++k) S.q[k * cap + t] = S.q2[k * cap + t];
@@ -1146,11 +1150,11 @@ void launch_place(DevState const& S, const int* gate, cudaStream_t st) {
 void launch_cellsort(DevState const& S, const int* gate, cudaStream_t st) {
   k_cellsort<<<blocks(S.ncells, 256), 256, 0, st>>>(S, gate);
 }
-void launch_permute(DevState const& S, const int* gate, cudaStream_t st) {
-  if (S.n) k_permute<<<blocks(S.n, 256), 256, 0, st>>>(S, gate);
+void launch_permute(DevState const& S, const int* gate, int forces, cudaStream_t st) {
+  if (S.n) k_permute<<<blocks(S.n, 256), 256, 0, st>>>(S, gate, forces);
 }
-void launch_copyback(DevState const& S, const int* gate, cudaStream_t st) {
-  if (S.n) k_copyback<<<blocks(S.n, 256), 256, 0, st>>>(S, gate);
+void launch_copyback(DevState const& S, const int* gate, int forces, cudaStream_t st) {
+  if (S.n) k_copyback<<<blocks(S.n, 256), 256, 0, st>>>(S, gate, forces);
 }
 void launch_move(DevState const& S, int flags, int fast, cudaStream_t st) {
   if (!S.n) return;

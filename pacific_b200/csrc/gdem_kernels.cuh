@@ -65,8 +65,9 @@ void launch_wall_rows(DevState const& S, const int* gate, cudaStream_t st);
 void launch_diag_prefill(DevState const& S, cudaStream_t st);
 void launch_place(DevState const& S, const int* gate, cudaStream_t st);
 void launch_cellsort(DevState const& S, const int* gate, cudaStream_t st);
-void launch_permute(DevState const& S, const int* gate, cudaStream_t st);
-void launch_copyback(DevState const& S, const int* gate, cudaStream_t st);
+// the state into cell order (forces: F and T too)
+void launch_permute(DevState const& S, const int* gate, int forces, cudaStream_t st);
+void launch_copyback(DevState const& S, const int* gate, int forces, cudaStream_t st);
 // fast: the FP32-split leapfrog (reciprocals, series; not the reference's
 // operation order)
 void launch_move(DevState const& S, int flags, int fast, cudaStream_t st);
