@@ -710,11 +710,12 @@ __global__ void __launch_bounds__(128, kConvex ? 1 : 3) k_pairlaw32(DevState S) 
   const int nh = S.ctl[kCtlKept], n2 = kConvex ? S.ctl[kCtlKept2] : 0, nw = S.ctl[kCtlWork];
   const int nk = nh + n2;
   const int tag = S.ctl[kCtlEpoch];
-  const int stride = gridDim.x * blockDim.x;
+  const int lane = threadIdx.x & 31;
+  const WarpItems w = warpItems(nk + nw);
   int nlaw = 0, nre = 0;   // contacts evaluated / re-evaluated in FP64
   GjkTally gjk;
   StatsTally st;
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < nk + nw; i += stride) {
+  for (int i = w.first + lane; lane < w.lanes && i < nk + nw; i += w.stride) {
     if (i < nh) pairItem32<kConvex>(S, S.kept[i], tag, nlaw, nre, gjk, st);
     else if (i < nk) pairItem32<kConvex>(S, S.kept2[i - nh], tag, nlaw, nre, gjk, st);
     else wallItem32<kConvex>(S, S.work[i - nk], tag, nlaw, nre, gjk, st);

@@ -376,10 +376,11 @@ __global__ void __launch_bounds__(128, kConvex ? 1 : 4) k_pairlaw64(DevState S) 
   pdlTrigger();   // the leapfrog kernel may start; its candidates wait for this kernel
   const int nk = S.ctl[kCtlKept], nw = S.ctl[kCtlWork];
   const int tag = S.ctl[kCtlEpoch];
-  const int stride = gridDim.x * blockDim.x;
+  const int lane = threadIdx.x & 31;
+  const WarpItems w = warpItems(nk + nw);
   GjkTally gjk;
   StatsTally st;
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < nk + nw; i += stride) {
+  for (int i = w.first + lane; lane < w.lanes && i < nk + nw; i += w.stride) {
     if (i < nk) pairItem64<kConvex>(S, S.kept[i], tag, gjk, st);
     else wallItem64<kConvex>(S, S.work[i - nk], tag, gjk, st);
   }

@@ -553,6 +553,24 @@ __device__ __forceinline__ void appendUpperPairs(DevState const& S, int t, const
 __device__ __forceinline__ void pdlWait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdlTrigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
+// Which of n items the lanes of a warp take: `lanes` consecutive ones per warp
+// (lane < lanes), from first on, every stride.  No more items than the grid
+// has warps go one to a warp instead of filling the first few: an item is a
+// chain of dependent latencies, and lanes on different branches of it take
+// turns (200 packed spheres, 680 items: step 43.2 -> 35.5 us).  A few lanes
+// per warp for more items cost more than they gave (7,777 spheres 35.4 ->
+// 39.5 us, the 1M gas's pair kernel 20.9 -> 24.2 us): every warp on every
+// multiprocessor fetches the whole law's instructions.
+struct WarpItems {
+  int lanes, first, stride;
+};
+__device__ __forceinline__ WarpItems warpItems(int n) {
+  const int warps = (int)(gridDim.x * blockDim.x) >> 5;
+  const int warp = (int)(blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const int lanes = n <= warps ? 1 : 32;
+  return {lanes, warp * lanes, warps * lanes};
+}
+
 // Contact-filter flags of the current force evaluation: two buffers used
 // alternately, the filter of one evaluation clearing the other's, so that no
 // kernel needs to clear flags that other warps may still be setting.
