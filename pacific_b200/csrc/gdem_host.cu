@@ -44,6 +44,8 @@ thread_local std::string g_last_error;
 const double PI = 3.14159265358979323846;
 // steps between two checks of the pair list's allocation within a call
 constexpr int kCapacityCheck = 512;
+// Steps of a call's graph, and the call's steps from which it is worth building.
+constexpr int kGraphSteps = 4, kGraphFrom = 16;
 // Particles up to which a system's arrays share allocations and its wall list
 // has room for all of them.
 constexpr int kSmallSystem = 16384;
@@ -611,7 +613,8 @@ struct System {
   bool id_order = false;           // state arrays are in particle-ID order (not yet binned)
   double last_ms = 0.;
   int status_host = 0;
-  cudaGraphExec_t graph[2] = {nullptr, nullptr};   // an evaluation inside a call, and its last
+  // an evaluation inside a call, its last, kGraphSteps inside a call
+  cudaGraphExec_t graph[3] = {nullptr, nullptr, nullptr};
   long epoch = 0;                  // host copy of the evaluation counter
   bool lists_hold = false;         // the lists (not the table) hold the contact memory
   bool lists_sized = false;        // the lists' allocations are checked against this state
@@ -1158,63 +1161,70 @@ struct System {
     ++epoch;
   }
 
-  // The same evaluation as one graph: decide -> conditional node holding the
-  // rebuild -> step kernel.  If the conditional node cannot be built, the
-  // graph holds the gated rebuild instead.
-  cudaGraphExec_t captureEvaluation(int flags) {
+  // `count` evaluations as one graph: each decide -> conditional node holding
+  // the rebuild -> step kernels, after the one before.  If a conditional node
+  // cannot be built, the graph holds the gated rebuild instead.
+  cudaGraphExec_t captureEvaluations(int flags, int count) {
     cudaGraph_t g = nullptr;
     CK(cudaGraphCreate(&g, 0));
     bool conditional = true;
-    cudaGraphConditionalHandle h{};
-    if (cudaGraphConditionalHandleCreate(&h, g, 0, cudaGraphCondAssignDefault) != cudaSuccess) {
-      cudaGetLastError();
-      conditional = false;
-    }
-    CK(cudaStreamBeginCaptureToGraph(stream, g, nullptr, nullptr, 0,
-                                     cudaStreamCaptureModeThreadLocal));
-    launch_decide(S, h, conditional ? 1 : 0, stream);
-    CK(cudaStreamEndCapture(stream, &g));
-    cudaGraphNode_t decide_node = nullptr;
-    size_t nn = 1;
-    CK(cudaGraphGetNodes(g, &decide_node, &nn));
-    cudaGraphNode_t tail = decide_node;
-    if (conditional) {
-      cudaGraphNodeParams cp{};
-      cp.type = cudaGraphNodeTypeConditional;
-      cp.conditional.handle = h;
-      cp.conditional.type = cudaGraphCondTypeIf;
-      cp.conditional.size = 1;
-      cudaGraphNode_t cond = nullptr;
-      if (cudaGraphAddNode(&cond, g, &decide_node, 1, &cp) == cudaSuccess) {
-        cudaGraph_t body = cp.conditional.phGraph_out[0];
-        CK(cudaStreamBeginCaptureToGraph(stream, body, nullptr, nullptr, 0,
-                                         cudaStreamCaptureModeThreadLocal));
-        rebuild(nullptr);
-        CK(cudaStreamEndCapture(stream, &body));
-        tail = cond;
-      } else {
+    cudaGraphNode_t tail = nullptr;   // what the next evaluation comes after
+    // the node that the stream's captured work ended with
+    auto capture = [&](cudaGraph_t into, cudaGraphNode_t after, auto&& work) {
+      CK(cudaStreamBeginCaptureToGraph(stream, into, after ? &after : nullptr, nullptr,
+                                       after ? 1 : 0, cudaStreamCaptureModeThreadLocal));
+      work();
+      cudaStreamCaptureStatus status;
+      const cudaGraphNode_t* deps = nullptr;
+      size_t ndeps = 0;
+      CK(cudaStreamGetCaptureInfo_v2(stream, &status, nullptr, nullptr, &deps, &ndeps));
+      const cudaGraphNode_t last = ndeps ? deps[0] : after;
+      CK(cudaStreamEndCapture(stream, &into));
+      return last;
+    };
+    for (int k = 0; k < count; ++k) {
+      cudaGraphConditionalHandle h{};
+      bool branch = conditional;
+      if (branch && cudaGraphConditionalHandleCreate(&h, g, 0, cudaGraphCondAssignDefault) != cudaSuccess) {
         cudaGetLastError();
-        conditional = false;
+        branch = false;
       }
+      tail = capture(g, tail, [&] { launch_decide(S, h, branch ? 1 : 0, stream); });
+      if (branch) {
+        cudaGraphNodeParams cp{};
+        cp.type = cudaGraphNodeTypeConditional;
+        cp.conditional.handle = h;
+        cp.conditional.type = cudaGraphCondTypeIf;
+        cp.conditional.size = 1;
+        cudaGraphNode_t cond = nullptr;
+        if (cudaGraphAddNode(&cond, g, &tail, 1, &cp) == cudaSuccess) {
+          capture(cp.conditional.phGraph_out[0], nullptr, [&] { rebuild(nullptr); });
+          tail = cond;
+        } else {
+          cudaGetLastError();
+          branch = false;
+        }
+      }
+      conditional = branch;
+      tail = capture(g, tail, [&] {
+        if (!branch) rebuild(S.ctl + kCtlActive);
+        forcesAndMove(flags);
+      });
     }
-    CK(cudaStreamBeginCaptureToGraph(stream, g, &tail, nullptr, 1,
-                                     cudaStreamCaptureModeThreadLocal));
-    if (!conditional) rebuild(S.ctl + kCtlActive);
-    forcesAndMove(flags);
-    CK(cudaStreamEndCapture(stream, &g));
     cudaGraphExec_t ex = nullptr;
     CK(cudaGraphInstantiate(&ex, g, 0));
     CK(cudaGraphDestroy(g));
     graph_conditional = conditional;
     return ex;
   }
-  // Graph of evaluation kind k (0: inside a call, 1: last of a call); built
-  // on first use.
+  // Graph of evaluation kind k (0: inside a call, 1: last of a call, 2:
+  // kGraphSteps inside a call); built on first use.
   void launchEvaluation(int k, int flags) {
-    if (!graph[k]) graph[k] = captureEvaluation(flags);
+    const int count = k == 2 ? kGraphSteps : 1;
+    if (!graph[k]) graph[k] = captureEvaluations(flags, count);
     CK(cudaGraphLaunch(graph[k], stream));
     lists_hold = true;
-    ++epoch;
+    epoch += count;
   }
 
   void init() {
@@ -1251,7 +1261,11 @@ struct System {
       // within a call (and at its end); it grows before it can run short
       if (k > 0 && k % kCapacityCheck == 0) checkCapacity();
       const bool graphs = use_graphs && !diag && !profiling;
-      if (graphs) {
+      if (graphs && nsteps >= kGraphFrom && k + kGraphSteps < nsteps &&
+          k / kCapacityCheck == (k + kGraphSteps - 1) / kCapacityCheck) {
+        launchEvaluation(2, mid);
+        k += kGraphSteps - 1;
+      } else if (graphs) {
         launchEvaluation(is_last ? 1 : 0, is_last ? last : mid);
       } else {
         evaluate(is_last ? last : mid);
