@@ -4,7 +4,7 @@ spheres in a triply periodic box (granular-gas cooling), FP32-split vs FP64.
 
 One step = one kick-drift-kick leapfrog step of the whole system: the force
 evaluation (narrow phase over the skin pair list, Hooke / HookeMemory contact
-force with hashed tangential history, per-particle force/torque reduction)
+force with tangential history, per-particle force/torque reduction)
 fused with the closing kick, the next opening kick and the drift; the pair
 list (counting sort on the cell key + 27-cell search) is rebuilt when a
 particle has moved half the skin.  Inputs: the seeded FCC stand-in of the
@@ -118,7 +118,7 @@ def algorithmic_bytes(kernel, n, entries, contacts, ncells, fp64):
     pairs = entries // 2
     touched = min(n, 2 * contacts)    # particles with a contact
     share = 64 if fp64 else 32        # one side of a contact, per row entry
-    hist = 8 + (72 if fp64 else 36)   # history key + values
+    memory = 64 if fp64 else 32       # a pair's contact memory (without rolling springs)
     if kernel == "filter":
         # per particle its FP32 position; per pair its compact-list word
         # pair; per kept pair its index in the kept list and the two
@@ -126,9 +126,9 @@ def algorithmic_bytes(kernel, n, entries, contacts, ncells, fp64):
         return n * 16 + pairs * 8 + contacts * (4 + 8)
     if kernel in ("pairlaw64", "pairlaw32"):
         # per kept pair: its index, compact-list words and row positions;
-        # both partners' id type wrap x v w and row offsets; the history
-        # read and written; the two shares and the two flags
-        return contacts * (4 + 8 + 4 + 2 * (4 + 4 + 4 + 24 + 2 * vel + 4) + 2 * hist
+        # both partners' id type wrap x v w and row offsets; the contact
+        # memory read and written; the two shares and the two flags
+        return contacts * (4 + 8 + 4 + 2 * (4 + 4 + 4 + 24 + 2 * vel + 4) + 2 * memory
                            + 2 * share + 2 * 4)
     if kernel == "move":
         # state type inst posf0 wrap flags | state wrap posf flags, and
@@ -145,19 +145,22 @@ def algorithmic_bytes(kernel, n, entries, contacts, ncells, fp64):
         return n * 16
     if kernel == "cellsort":     # starts, count reset (per cell); order, id of shared cells
         return ncells * 8 + n * 8
-    if kernel == "permute":      # order skey ids state F T | ids state F T cellc + pos / offset
-        return n * (4 + 4 + 12 + 2 * (state + 48) + 16 + (32 if fp64 else 16))
-    if kernel == "copyback":     # ids state F T | ids state F T wrap posf posf0
-        return n * (12 + 2 * (state + 48) + 12 + 4 + 32)
-    if kernel in ("pairs_count64", "pairs_count32"):   # cellc + own position | row length
-        return n * (16 + (32 if fp64 else 16) + 4) + 4 * ncells
+    if kernel == "permute":      # order skey ids state | ids state cellc + pos / offset
+        return n * (4 + 4 + 12 + 2 * state + 16 + (32 if fp64 else 16))
+    if kernel == "copyback":     # ids state | ids state wrap posf posf0
+        return n * (12 + 2 * state + 12 + 4 + 32)
+    if kernel in ("pairs_count64", "pairs_count32"):
+        # cellc + own position | row length, candidates
+        return n * (16 + (32 if fp64 else 16) + 4) + 4 * ncells + 4 * entries
     if kernel == "row_scan":     # row lengths | row offsets
         return n * 8
     if kernel in ("pairs_fill64", "pairs_fill32"):
-        # cellc + own position + row offset and length | rows, compact list
-        return n * (16 + (32 if fp64 else 16) + 8) + 4 * ncells + 4 * entries + 12 * pairs
+        # row offset and length, ID, candidates | rows, compact list
+        return n * (4 + 8) + 4 * entries + 4 * entries + 12 * pairs
     if kernel == "link":         # compact list, partner's row | row positions
         return pairs * (8 + 4 + 4 + 4)
+    if kernel == "mem_load":     # compact list, both IDs, a table key | the pair's evaluation word
+        return pairs * (8 + 8 + 8 + 4)
     return None
 
 
@@ -695,7 +698,7 @@ def main():
         v64 = world * n * args.steps / (fp64["ms"] * 1e-3)
         # roofline of the dominant kernel of the FP32-split step
         kt = fp32["kt"]
-        dom = max((k for k in kt if k not in ("decide", "hist_fill")), key=lambda k: kt[k][0])
+        dom = max((k for k in kt if k != "decide"), key=lambda k: kt[k][0])
         avg_ms = kt[dom][0] / kt[dom][1]
         ncells = fp32["ncells"]
         ab = algorithmic_bytes(dom, n, fp32["entries"], fp32["contacts"], ncells, False)
@@ -771,13 +774,11 @@ def main():
             "gpu_launches": None,
         }
         # kernels launched in the timed region: the opening move, per step
-        # k_decide, the contact filter, the pair kernel and the move, per
-        # pair-list rebuild its 14 kernels (bin, scan x3, place, cellsort,
-        # permute, copyback, row count, row scan x3, row fill, link), and the
-        # history-table refills (every 512 evaluations per table)
-        e0, e1 = fp32["evals"]
-        fills = sum(1 for e in range(e0 + 1, e1 + 1) if e % 512 < 2)
-        line["gpu_launches"] = 1 + 4 * args.steps + 14 * fp32["rebuilds"] + fills
+        # k_decide, the contact filter, the pair kernel and the move, and per
+        # pair-list rebuild its 17 kernels (table clear, memory save, bin, scan
+        # x3, place, cellsort, permute, copyback, row count, row scan x3, row
+        # fill, link, memory load; the gas has no walls)
+        line["gpu_launches"] = 1 + 4 * args.steps + 17 * fp32["rebuilds"]
         if "fp64" not in res:
             line["fp64"] = None
         line["pair_list"] = {"rebuilds_fp32_split": fp32["rebuilds"],

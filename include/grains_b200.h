@@ -400,8 +400,8 @@ int gdem_use_graphs(gdem_handle h, int on);
  * updateContactMap) or kept, so that a pair that touches again resumes its
  * tangential spring (prune = 0: GrainsCoupledWithFluid::Simulation,
  * Fluid/src/GrainsCoupledWithFluid.cpp:123-228, which never prunes).  Set it
- * before the particles are uploaded or read; with prune = 0 the history
- * tables are four times larger, and a run that fills them raises
+ * before the particles are uploaded or read; with prune = 0 the memory
+ * table is four times larger, and a run that fills it raises
  * GDEM_ST_HASH_FULL. */
 int gdem_set_contact_memory_pruning(gdem_handle h, int prune);
 

@@ -14,9 +14,9 @@
 //               a pair agree.
 //   k_pairlaw64 one thread per pair the contact filter kept: narrow phase
 //               (ClosestPointSPHERESPHERE or GJK), Hooke / HookeMemory force
-//               with the tangential history in the hashed pair table, and the
+//               with the contact memory of the pair's list entry, and the
 //               pair's two shares written into both partners' rows; then one
-//               thread per particle near a wall for its wall contacts
+//               thread per wall item (a particle and a wall it is near)
 //               (SimpleObstacle::InterAction, Component/src/
 //               SimpleObstacle.cpp:222-271).  The leapfrog kernel adds the
 //               shares of each particle in row (partner-ID) order.

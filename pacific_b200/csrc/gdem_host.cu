@@ -9,13 +9,14 @@
 //   k_move (opening kick dt/2 + drift dt with the stored F, T), then per step
 //   k_decide -> [pair-list rebuild, when some particle moved half the skin:
 //                k_bin, scan, k_place, k_cellsort, k_permute, k_copyback,
-//                k_pairs_count, row scan, k_pairs_fill, k_link]
-//   -> k_filter (kept pairs, particles near a wall)
-//   -> k_pairlaw (narrow phase, contact law, history; shares into the rows)
+//                k_pairs_count, row scan, k_pairs_fill, k_link, k_wall_rows,
+//                between k_mem_save and k_mem_load]
+//   -> k_filter (kept pairs, wall items)
+//   -> k_pairlaw (narrow phase, contact law, memory; shares into the rows)
 //   -> k_move (sums of the shares; closing kick, next opening kick + drift)
 //
 // Each step is one captured CUDA graph (the rebuild inside a conditional
-// node); two graphs alternate with the contact-history tables.
+// node); calls of many steps replay graphs of four.
 #include <algorithm>
 #include <array>
 #include <climits>

@@ -11,7 +11,7 @@
 //
 //   k_decide    turns the rebuild request of the previous step into this
 //               step's decision (and the CUDA-graph condition), and counts
-//               the force evaluation (contact-history tag).
+//               the force evaluation (tag of shares and contact memory).
 //   k_bin       pair-list cell of each particle and the cell histogram.
 //   scan/place/cellsort
 //               counting sort of particles on their cell key: a one-digit

@@ -19,7 +19,7 @@ enum StatusBits : int {
   kErrContactOverlap = 1 << 0,   // overlap >= sum of crusts (ContactError)
   kErrMotion = 1 << 1,           // |dx| > crust over one step (MotionError)
   kErrOutOfGrid = 1 << 2,        // particle outside the linked-cell grid (SimulationError)
-  kErrHashFull = 1 << 3,         // contact-history table has no free slot
+  kErrHashFull = 1 << 3,         // the contact-memory table has no free slot
   kErrGjkMaxIter = 1 << 4,       // GJK hit its iteration cap
   kErrTimeout = 1 << 5,          // a bounded device wait gave up
   kErrPairsFull = 1 << 6,        // the pair list outgrew its allocation (or a row kRowMax)
@@ -29,7 +29,7 @@ enum StatusBits : int {
 enum CtlWords : int {
   kCtlNeed = 0,     // set by the step kernels: a particle moved more than skin / 2
   kCtlActive = 1,   // this step rebuilds the pair list (set by k_decide)
-  kCtlEpoch = 2,    // force evaluations so far (tags the contact-history keys)
+  kCtlEpoch = 2,    // force evaluations so far (tags shares and contact memory)
   kCtlRebuilds = 3, // pair-list rebuilds so far
   kCtlWork = 4,     // particles near a wall this evaluation (contact filter)
   kCtlPairs = 5,    // pairs of the compact pair list (set by the rebuild)
