@@ -34,6 +34,7 @@
 #include "../../include/grains_b200.h"
 #include "gdem_kernels.cuh"
 #include "gdem_divide.cuh"
+#include "gdem_memory.h"
 #include "gdem_setup.h"
 #include "xml_reader.hpp"
 
@@ -62,13 +63,14 @@ struct CudaError : std::runtime_error {
       throw CudaError(std::string(#call) + ": " + cudaGetErrorString(e_));           \
   } while (0)
 
-template <typename T>
-T* dalloc(size_t count) {
+// Device memory, or null when there is none.
+void* takeDevice(size_t bytes) {
   void* p = nullptr;
-  if (count == 0) count = 1;
-  CK(cudaMalloc(&p, count * sizeof(T)));
-  return static_cast<T*>(p);
+  if (cudaMalloc(&p, bytes) == cudaSuccess) return p;
+  cudaGetLastError();
+  return nullptr;
 }
+void giveDevice(void* p) { cudaFree(p); }
 
 int nextPow2Log(size_t n) {
   int l = 10;
@@ -621,9 +623,7 @@ struct System {
   bool lists_sized = false;        // the lists' allocations are checked against this state
   long epoch_t0 = 0;               // evaluation counter at the leapfrog's t0 (contact features)
   bool graph_conditional = false;  // the graphs rebuild through a conditional node
-  std::vector<void*> allocs;
-  char* pool = nullptr;            // rest of the last shared block (alloc)
-  size_t pool_left = 0, pool_total = 0;
+  DeviceMemory memory{takeDevice, giveDevice};
   double* d_stage = nullptr;       // AoS staging, ID order (x v w wbf q F T: 22 doubles/particle)
   int* d_type_id = nullptr;        // particle class by ID
   int* d_inst_id = nullptr;        // instance by ID
@@ -640,10 +640,7 @@ struct System {
   ~System() { release(); }
   void release() {
     for (auto& gx : graph) if (gx) { cudaGraphExecDestroy(gx); gx = nullptr; }
-    for (void* p : allocs) cudaFree(p);
-    allocs.clear();
-    pool = nullptr;
-    pool_left = pool_total = 0;
+    memory.release();
     if (d_grids) cudaFree(d_grids);
     if (d_types) cudaFree(d_types);
     if (d_models) cudaFree(d_models);
@@ -663,12 +660,15 @@ struct System {
     if (stream) cudaStreamDestroy(stream);
     stream = nullptr;
   }
+  template <typename T>
+  static T* taken(void* p) {
+    if (!p) throw CudaError(std::string("cudaMalloc: ") + cudaGetErrorString(cudaErrorMemoryAllocation));
+    return static_cast<T*>(p);
+  }
   // An array of its own, which freeAlloc can give back.
   template <typename T>
   T* allocOwn(size_t n) {
-    T* p = dalloc<T>(n);
-    allocs.push_back(p);
-    return p;
+    return taken<T>(memory.own(n * sizeof(T)));
   }
   // An array that lives as long as the system, out of shared blocks: a first
   // one for about 4 KB per particle (all a small system needs), then as much
@@ -678,32 +678,17 @@ struct System {
   // allocation of their own.
   template <typename T>
   T* alloc(size_t n) {
-    const size_t bytes = (std::max<size_t>(n, 1) * sizeof(T) + 255) & ~size_t(255);
+    const size_t bytes = n * sizeof(T);
     if (bytes > (size_t(32) << 20)) return allocOwn<T>(n);
-    if (pool_left < bytes) {
-      size_t block = std::max(bytes, std::min(size_t(64) << 20, std::max(((size_t)S.cap + 64) * 4096, pool_total)));
-      void* p = nullptr;
-      if (cudaMalloc(&p, block) != cudaSuccess) {
-        cudaGetLastError();
-        return allocOwn<T>(n);
-      }
-      allocs.push_back(p);
-      pool = static_cast<char*>(p);
-      pool_left = block;
-      pool_total += block;
-    }
-    T* r = reinterpret_cast<T*>(pool);
-    pool += bytes;
-    pool_left -= bytes;
-    return r;
+    return taken<T>(memory.shared(
+        bytes, std::min(size_t(64) << 20,
+                        std::max(((size_t)S.cap + 64) * 4096, memory.sharedTotal()))));
   }
   void invalidateGraphs() {
     for (auto& gx : graph) if (gx) { cudaGraphExecDestroy(gx); gx = nullptr; }
   }
-  void freeAlloc(void* p) {
-    for (auto& a : allocs)
-      if (a == p) { CK(cudaFree(a)); a = allocs.back(); allocs.pop_back(); return; }
-  }
+  // Gives an array of its own back; one out of a shared block stays there.
+  void freeAlloc(void* p) { memory.giveBack(p); }
 
   // Pair-list skin (a multiple of each instance's largest circumscribed
   // radius; < 0 restores the XML's) and the force kernels' blocks per
@@ -973,8 +958,8 @@ struct System {
     const size_t o_share = part(e * sb), o_mem = part(pc * mb), o_pairs = part(e * sizeof(int)),
                  o_up = part(pc * sizeof(int2)), o_pos = part(pc * sizeof(int)),
                  o_kept = part(pc * sizeof(int)), o_kept2 = part(cold ? pc * sizeof(int) : 0);
-    // (a small system's first lists fit its shared block; they are few MB, so
-    // they may stay there when the lists outgrow them)
+    // (a small system's first lists come out of a shared block; they are few
+    // MB, so they may stay there when the lists outgrow them)
     char* base = kSmallSystem >= S.cap && !S.upairs ? alloc<char>(at) : allocOwn<char>(at);
     S.share = base + o_share;
     S.pmem = MemView{base + o_mem, (long long)pc};
