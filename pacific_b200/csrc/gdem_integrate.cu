@@ -556,18 +556,24 @@ __device__ __forceinline__ WallProbe wallProbe(DevState const& S, int t, GridDes
            pt.z - (float)wrapGet(wt, 2) * bg.Lf[2]},
           pt.w + bg.filt_margin + reach};
 }
-__device__ __forceinline__ bool nearWall(WallDesc const& wd, WallProbe const& p) {
+// images: a wall whose nearest periodic image is near too (the particle can
+// leave through one face of the box and come in at the other).
+__device__ __forceinline__ bool nearWall(GridDesc const& bg, WallDesc const& wd, WallProbe const& p,
+                                         bool images) {
   float d2 = 0.f;
 #pragma unroll
   for (int d = 0; d < 3; ++d) {
-    const float o = fabsf(p.q[d] - (float)wd.centre[d]) - (float)wd.extent[d];
+    float c = p.q[d] - (float)wd.centre[d];
+    if (images && bg.periodic[d]) c -= bg.Lf[d] * rintf(c / bg.Lf[d]);
+    const float o = fabsf(c) - (float)wd.extent[d];
     if (o > 0.f) d2 += o * o;
   }
   return d2 <= p.R * p.R;
 }
 
-// The wall list: particles within the skin of a wall, which no other can
-// reach before the next rebuild (part of a rebuild, after k_copyback).
+// The wall list: particles within the skin of a wall or of a periodic image of
+// one, which no other can reach before the next rebuild (part of a rebuild,
+// after k_copyback).
 __global__ void k_wall_rows(DevState S, const int* gate) {
   if (gatedOff(gate)) return;
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
@@ -576,7 +582,8 @@ __global__ void k_wall_rows(DevState S, const int* gate) {
     const int inst = S.inst[t];
     GridDesc const& bg = S.bgrids[inst];
     const WallProbe p = wallProbe(S, t, bg, bg.skin_f);
-    for (int k = 0; k < bg.wall_count && !near; ++k) near = nearWall(S.walls[bg.wall_begin + k], p);
+    for (int k = 0; k < bg.wall_count && !near; ++k) 
+      near = nearWall(bg, S.walls[bg.wall_begin + k], p, true);
   }
   const unsigned m = __ballot_sync(0xffffffffu, near);
   const int lane = threadIdx.x & 31;
@@ -602,13 +609,14 @@ __device__ __forceinline__ void filterWalls(DevState const& S, int* flags, int n
     const int row = r0 + lane;
     int count = 0, t = 0, begin = 0, nw = 0;
     WallProbe p{};
+    GridDesc const* bg = nullptr;
     if (row < nr) {
       t = S.wlist[row];
-      GridDesc const& bg = S.bgrids[S.inst[t]];
-      p = wallProbe(S, t, bg, 0.f);
-      begin = bg.wall_begin;
-      nw = bg.wall_count;
-      for (int k = 0; k < nw; ++k) count += nearWall(S.walls[begin + k], p);
+      bg = &S.bgrids[S.inst[t]];
+      p = wallProbe(S, t, *bg, 0.f);
+      begin = bg->wall_begin;
+      nw = bg->wall_count;
+      for (int k = 0; k < nw; ++k) count += nearWall(*bg, S.walls[begin + k], p, false);
       if (count) flags[t] = (int)kCandidate;
       if (S.any_convex) count = min(count, 1);
     }
@@ -628,7 +636,7 @@ __device__ __forceinline__ void filterWalls(DevState const& S, int* flags, int n
       S.work[at] = row;
     } else {
       for (int k = 0; k < nw; ++k)
-        if (nearWall(S.walls[begin + k], p)) S.work[at++] = row * S.max_walls + k;
+        if (nearWall(*bg, S.walls[begin + k], p, false)) S.work[at++] = row * S.max_walls + k;
     }
   }
 }
