@@ -620,7 +620,6 @@ struct System {
   cudaGraphExec_t graph[3] = {nullptr, nullptr, nullptr};
   long epoch = 0;                  // host copy of the evaluation counter
   bool lists_hold = false;         // the lists (not the table) hold the contact memory
-  bool lists_sized = false;        // the lists' allocations are checked against this state
   long epoch_t0 = 0;               // evaluation counter at the leapfrog's t0 (contact features)
   bool graph_conditional = false;  // the graphs rebuild through a conditional node
   DeviceMemory memory{takeDevice, giveDevice};
@@ -910,8 +909,8 @@ struct System {
     S.wall_cap = 0;
     S.wrow = alloc<int>(S.any_walls ? c : 1);
     // the wall list: every particle of a small system, a quarter of a large
-    // one's (a wall layer is far thinner; sizeLists grows it before the steps
-    // that follow a new state, checkCapacity during a run)
+    // one's (a wall layer is far thinner; it grows when a rebuild needs more,
+    // and evaluations are put off until it has)
     if (S.any_walls) allocateWalls(c <= kSmallSystem ? (long long)c : (long long)c / 4);
     S.status = alloc<int>(1);
     CK(cudaMemset(S.status, 0, sizeof(int)));
@@ -991,6 +990,8 @@ struct System {
       throw std::runtime_error("wall list too large for 32-bit slots");
     saveMemory(true);
     if (S.wshare) freeAlloc(S.wshare);
+    S.wshare = nullptr;
+    S.wall_cap = 0;
     const bool fp64 = precision == GDEM_FP64;
     const size_t slots = (size_t)rows * S.max_walls;
     // (one allocation; every part a multiple of 16 bytes)
@@ -1014,18 +1015,29 @@ struct System {
   // Grows the pair list (the wall list) when the most entries (particles) a
   // rebuild needed since the last check exceed 80 % of the allocation, to 1.5
   // times that need; the next evaluation rebuilds.  Synchronises the stream.
-  void checkCapacity() {
+  // Returns how many of the evaluations launched so far were put off, because
+  // the wall list had no room for a rebuild: they have to be launched again.
+  int checkCapacity() {
     int ctl[kCtlWords];
     CK(cudaStreamSynchronize(stream));
     CK(cudaMemcpy(ctl, S.ctl, sizeof(ctl), cudaMemcpyDeviceToHost));
     CK(cudaMemsetAsync(S.ctl + kCtlEntriesMax, 0, sizeof(int), stream));
     CK(cudaMemsetAsync(S.ctl + kCtlWallRowsMax, 0, sizeof(int), stream));
+    int off = 0;
+    if (ctl[kCtlNeed] == kPutOff) {
+      static const int one = 1;
+      off = (int)((unsigned)epoch - (unsigned)ctl[kCtlEpoch]);
+      epoch -= off;
+      lists_hold = false;   // (the rebuild left the memory in the table)
+      CK(cudaMemcpyAsync(S.ctl + kCtlNeed, &one, sizeof(int), cudaMemcpyHostToDevice, stream));
+    }
     CK(cudaStreamSynchronize(stream));
     const int hwm = ctl[kCtlEntriesMax], rows = std::max(ctl[kCtlWallRowsMax], ctl[kCtlWallRows]);
     if ((double)hwm > 0.8 * (double)S.pair_cap)
       allocatePairs(std::max((long long)(1.5 * (double)hwm) + 4096, (long long)S.pair_cap));
     if (S.any_walls && S.wall_cap < S.cap && (double)rows > 0.8 * (double)S.wall_cap)
       allocateWalls(std::min((long long)S.cap, (long long)(1.5 * (double)rows) + 4096));
+    return off;
   }
   // The contact memory of the last evaluation from the lists into its table
   // (where the host reads it); with leave the table then holds it and the
@@ -1063,20 +1075,13 @@ struct System {
     launch_wall_rows(S, gate, stream);
     CK(cudaGetLastError());
     id_order = false;
-    int status = 0;   // (too short a wall list is what this finds)
-    CK(cudaStreamSynchronize(stream));
-    CK(cudaMemcpy(&status, S.status, sizeof(int), cudaMemcpyDeviceToHost));
-    status &= ~(int)kErrPairsFull;
-    CK(cudaMemcpy(S.status, &status, sizeof(int), cudaMemcpyHostToDevice));
     checkCapacity();
-    lists_sized = true;
   }
 
   // Host AoS arrays (by ID) -> staging -> SoA state in ID order.
   void loadState(const double* x, const double* v, const double* w, const double* wbf,
                  const double* q, const double* F, const double* T) {
     saveMemory(true);   // (the lists name the particles by slot)
-    lists_sized = !S.any_walls || S.wall_cap == S.cap;
     size_t n = (size_t)S.n;
     double* st = d_stage;
     double *dx = st, *dv = st + 3 * n, *dw = st + 6 * n, *dwb = st + 9 * n, *dq = st + 12 * n,
@@ -1216,7 +1221,7 @@ struct System {
   void init() {
     sizeLists();
     epoch_t0 = epoch + 1;   // the evaluation at t0 is the next one
-    evaluate(kStepStoreFT);
+    evaluate(kStepStoreFT);   // (for the lists just sized)
     launch_mem_zero_cumulative(S, precision == GDEM_FP64, stream);
     CK(cudaStreamSynchronize(stream));
     // size the contact filter's grid for the lists just built and a quarter
@@ -1235,37 +1240,40 @@ struct System {
   // kick and -- except after the last -- the next opening kick and drift.
   void step(int nsteps) {
     if (nsteps <= 0) return;
-    if (!lists_sized) sizeLists();
     id_order = false;
     CK(cudaEventRecord(ev0, stream));
     timed("move", [&] { launch_move(S, kStepMove, precision == GDEM_FP32_SPLIT, stream); });
     const int mid = kStepClose | kStepMove;
     const int last = kStepClose | kStepStoreFT;
-    for (int k = 0; k < nsteps; ++k) {
-      const bool is_last = k == nsteps - 1;
-      // the pair list's allocation is checked every kCapacityCheck steps
-      // within a call (and at its end); it grows before it can run short
-      if (k > 0 && k % kCapacityCheck == 0) checkCapacity();
-      const bool graphs = use_graphs && !diag && !profiling;
-      if (graphs && nsteps >= kGraphFrom && k + kGraphSteps < nsteps &&
-          k / kCapacityCheck == (k + kGraphSteps - 1) / kCapacityCheck) {
-        launchEvaluation(2, mid);
-        k += kGraphSteps - 1;
-      } else if (graphs) {
-        launchEvaluation(is_last ? 1 : 0, is_last ? last : mid);
-      } else {
-        evaluate(is_last ? last : mid);
+    int k = 0;   // evaluations made (or put off: checkCapacity says how many)
+    do {
+      while (k < nsteps) {
+        const bool is_last = k == nsteps - 1;
+        const bool graphs = use_graphs && !diag && !profiling;
+        if (graphs && nsteps >= kGraphFrom && k + kGraphSteps < nsteps &&
+            k / kCapacityCheck == (k + kGraphSteps - 1) / kCapacityCheck) {
+          launchEvaluation(2, mid);
+          k += kGraphSteps;
+        } else {
+          if (graphs) launchEvaluation(is_last ? 1 : 0, is_last ? last : mid);
+          else evaluate(is_last ? last : mid);
+          ++k;
+        }
+        // the lists' allocations are checked every kCapacityCheck steps
+        // within a call (and at its end); the pair list grows before it can
+        // run short
+        if (k < nsteps && k % kCapacityCheck == 0) k -= checkCapacity();
       }
-    }
-    CK(cudaEventRecord(ev1, stream));
-    CK(cudaGetLastError());
-    CK(cudaEventSynchronize(ev1));
+      CK(cudaEventRecord(ev1, stream));
+      CK(cudaGetLastError());
+      CK(cudaEventSynchronize(ev1));
+      k -= checkCapacity();
+    } while (k < nsteps);
     float ms = 0.f;
     CK(cudaEventElapsedTime(&ms, ev0, ev1));
     last_ms = ms;
     collectTimes();
     evaluated = diag ? 1 : 2;
-    checkCapacity();
   }
   int readStatus() {
     int st = 0;

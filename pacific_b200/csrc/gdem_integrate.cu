@@ -443,10 +443,12 @@ __global__ void __launch_bounds__(kMoveBlock<kFast, kBasis>(), kBasis ? 2 : (kFa
     k_move(DevState S, int flags) {
   int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= S.n) return;
+  const int need = S.ctl[kCtlNeed];
   TypeDesc const& tp = S.types[S.type[t]];
   MoveIn m;
   loadMoveIn<kFast, kBasis>(S, t, m);   // nothing the contact kernels write
   const bool sum = (flags & kStepSum) != 0;
+  if (sum && need == kPutOff) return;
   d3 F, T;
   bool candidate = false;
   if (sum) {
@@ -594,7 +596,7 @@ __global__ void k_wall_rows(DevState S, const int* gate) {
   S.wrow[t] = near ? row : -1;
   if (!near) return;
   if (row < S.wall_cap) S.wlist[row] = t;
-  else raise(S.status, kErrPairsFull);   // (grown before the next call)
+  else S.ctl[kCtlNeed] = kPutOff;
 }
 
 // This evaluation's wall items: for spheres every near (particle, wall) slot
@@ -879,18 +881,28 @@ __global__ void k_mem_save(DevState S, const int* gate, int back) {
 }
 
 // The table's memory into the new lists, as left by the last evaluation; from
-// here on the lists hold it.
+// here on the lists hold it.  The last kernel of a rebuild: where the wall list
+// ran short it puts the evaluation off instead (kPutOff).
 template <typename T>
 __global__ void k_mem_load(DevState S, const int* gate) {
   if (gatedOff(gate)) return;
   const int last = S.ctl[kCtlEpoch] - 1;
+  const long long i0 = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  const bool off = S.ctl[kCtlNeed] == kPutOff;
+  if (i0 == 0) {
+    S.ctl[kCtlMemory] = off ? 0 : 1;
+    S.ctl[kCtlWallRowsMax] = max(S.ctl[kCtlWallRowsMax], S.ctl[kCtlWallRows]);
+    if (off) {
+      // (the table keeps the memory)
+      S.ctl[kCtlPairs] = 0;
+      S.ctl[kCtlWallRows] = 0;
+      S.ctl[kCtlEpoch] -= 1;
+      S.ctl[kCtlRebuilds] -= 1;
+    }
+  }
+  if (off) return;
   const int np = listedPairs(S);
   const long long ne = np + (long long)listedWalls(S) * S.max_walls;
-  const long long i0 = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i0 == 0) {
-    S.ctl[kCtlMemory] = 1;
-    S.ctl[kCtlWallRowsMax] = max(S.ctl[kCtlWallRowsMax], S.ctl[kCtlWallRows]);
-  }
   for (long long i = i0; i < ne; i += (long long)gridDim.x * blockDim.x) {
     MemView m;
     long long at;

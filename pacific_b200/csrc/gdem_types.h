@@ -27,7 +27,7 @@ enum StatusBits : int {
 
 // Words of the device control block (DevState::ctl).
 enum CtlWords : int {
-  kCtlNeed = 0,     // set by the step kernels: a particle moved more than skin / 2
+  kCtlNeed = 0,     // set by the step kernels: a particle moved more than skin / 2 (or kPutOff)
   kCtlActive = 1,   // this step rebuilds the pair list (set by k_decide)
   kCtlEpoch = 2,    // force evaluations so far (tags shares and contact memory)
   kCtlRebuilds = 3, // pair-list rebuilds so far
@@ -44,6 +44,12 @@ enum CtlWords : int {
   kCtlWallRowsMax = 14,  // most wall-list particles of any rebuild since the last allocation check
   kCtlWords = 16
 };
+// Value of kCtlNeed where an evaluation is put off: its rebuild found more
+// particles near a wall than the wall list has room for.  That evaluation and
+// those after it (whose rebuilds find the same) leave the state as it is: the
+// lists are empty, the leapfrog moves nothing.  They are not counted; the host
+// makes them once it has enlarged the list, so no wall contact is left out.
+constexpr int kPutOff = 2;
 
 // One independent simulation ("instance").  A single Grains3D system is a
 // batch of one.  Cell numbering follows LinkedCell::getCellNumber
