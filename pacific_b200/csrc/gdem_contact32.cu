@@ -408,13 +408,13 @@ __device__ __forceinline__ void storeShare32(DevState const& S, int64_t entry, i
   sh[1] = make_float4(c.x, c.y, c.z, 0.f);
 }
 
-// Contact of particle t (class ta, row of the wall list) with wall k of its
-// instance: the geometry from the FP64 position, the force law in FP32 (FP64
+// Contact of particle t (class ta) with wall k of its instance (at: its slot of
+// the wall list, or -1): the geometry from the FP64 position, the force law in FP32 (FP64
 // when ill-conditioned).  Returns true for a contact, with its force f, the
 // lever arm's torque c and, with a rolling model (rolling), the rolling
 // torque mr.
 template <bool kConvex>
-__device__ __forceinline__ bool wallContact32(DevState const& S, GridDesc const& g, int row, int t,
+__device__ __forceinline__ bool wallContact32(DevState const& S, GridDesc const& g, int at, int t,
                                               int k, TypeDesc const& ta, d3 xt, d3 vt, d3 wt,
                                               int& curw, bool& walls_gjk, int& nlaw, int& nre,
                                               GjkTally& gjk, StatsTally& st, float3& f, float3& c,
@@ -462,17 +462,16 @@ __device__ __forceinline__ bool wallContact32(DevState const& S, GridDesc const&
   ++nlaw;
   if (m.memory) {
     const int now = S.ctl[kCtlEpoch];
-    const long long at = (long long)row * S.max_walls + k;
     const bool spring = m.rolling != 0;
     float hv[9];
-    const bool existed = remembered(S, memLoad(S.wmem, at, hv, spring), now);
+    const bool existed = at >= 0 && remembered(S, memLoad(S.wmem, at, hv, spring), now);
     if (existed) {
       kd = f3(hv[0], hv[1], hv[2]); pn = f3(hv[3], hv[4], hv[5]);
       sp = f3(hv[6], spring ? hv[7] : 0.f, spring ? hv[8] : 0.f);
     }
     contactLaw32(m, S.dt, ct, b0, b1, existed, kd, pn, sp, f, mr, re);
     const float out[9] = {kd.x, kd.y, kd.z, pn.x, pn.y, pn.z, sp.x, sp.y, sp.z};
-    memStore(S.wmem, at, out, now, spring || !existed);
+    if (at >= 0) memStore(S.wmem, at, out, now, spring || !existed);
   } else {
     contactLaw32(m, S.dt, ct, b0, b1, false, kd, pn, sp, f, mr, re);
   }
@@ -487,14 +486,13 @@ __device__ __forceinline__ bool wallContact32(DevState const& S, GridDesc const&
 }
 
 // One wall item of the evaluation: a (particle, wall) slot of the wall list
-// (spheres), whose contact is its share, or a particle of it, whose walls are
-// taken in order and summed into its first slot's share.  (A sphere in an edge
+// (spheres), whose contact is its share, or a particle of it (its first slot),
+// whose walls are taken in order and summed into that slot's share.  (A sphere in an edge
 // or corner used to take its walls in turn: their laws' latencies added up.)
 template <bool kConvex>
 __device__ __forceinline__ void wallItem32(DevState const& S, int item, int tag, int& nlaw, int& nre,
                                            GjkTally& gjk, StatsTally& st) {
-  const int row = kConvex ? item : item / S.max_walls;
-  const int t = S.wlist[row];
+  const int t = S.wlist[item].x;
   GridDesc const& g = S.grids[S.inst[t]];
   TypeDesc const& ta = S.types[S.type[t]];
   const d3 xt = ld3(S.x, S.cap, t), vt = ld3(S.v, S.cap, t), wt = ld3(S.w, S.cap, t);
@@ -505,8 +503,11 @@ __device__ __forceinline__ void wallItem32(DevState const& S, int item, int tag,
     // the particle's polyhedron vertex runs through its wall calls in order
     curw = startVertex(S, ta, t);
     float3 Fw = f3(0.f, 0.f, 0.f), Tw = f3(0.f, 0.f, 0.f);
-    for (int k = 0; k < g.wall_count; ++k) {
-      if (!wallContact32<kConvex>(S, g, row, t, k, ta, xt, vt, wt, curw, walls_gjk, nlaw, nre, gjk,
+    // (a wall without a slot is out of reach: its search is for the vertex)
+    const int end = item + S.wrow[t].y;
+    for (int k = 0, slot = item; k < g.wall_count; ++k) {
+      const int at = slot < end && S.wlist[slot].y == k ? slot++ : -1;
+      if (!wallContact32<kConvex>(S, g, at, t, k, ta, xt, vt, wt, curw, walls_gjk, nlaw, nre, gjk,
                                   st, f, c, mr, rolling))
         continue;
       Fw = Fw + f;
@@ -518,9 +519,8 @@ __device__ __forceinline__ void wallItem32(DevState const& S, int item, int tag,
     f = Fw;
     c = Tw;
     rolling = false;
-    item = row * S.max_walls;
   } else {
-    any = wallContact32<kConvex>(S, g, row, t, item - row * S.max_walls, ta, xt, vt, wt, curw,
+    any = wallContact32<kConvex>(S, g, item, t, S.wlist[item].y, ta, xt, vt, wt, curw,
                                  walls_gjk, nlaw, nre, gjk, st, f, c, mr, rolling);
   }
   if (!any) return;

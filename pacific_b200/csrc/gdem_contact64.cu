@@ -180,12 +180,12 @@ __device__ __forceinline__ void storeShare64(DevState const& S, int64_t entry, i
   sh[3] = make_double2(c.z, 0.);
 }
 
-// Contact of particle t (class ta, row of the wall list) with wall k of its
-// instance: the particle is p0, the obstacle p1 (mass Component::
+// Contact of particle t (class ta) with wall k of its instance (at: its slot of
+// the wall list, or -1): the particle is p0, the obstacle p1 (mass Component::
 // m_massObstacle).  Returns true for a contact, with its force f, the lever
 // arm's torque c and, with a rolling model (rolling), the rolling torque mr.
 template <bool kConvex>
-__device__ __forceinline__ bool wallContact64(DevState const& S, GridDesc const& g, int row, int t,
+__device__ __forceinline__ bool wallContact64(DevState const& S, GridDesc const& g, int at, int t,
                                               int k, TypeDesc const& ta, d3 xt, d3 vt, d3 wt,
                                               int& curw, bool& walls_gjk, GjkTally& gjk,
                                               StatsTally& st, d3& f, d3& c, d3& mr, bool& rolling) {
@@ -209,10 +209,9 @@ __device__ __forceinline__ bool wallContact64(DevState const& S, GridDesc const&
   const d3 wc = mk(wd.centre[0], wd.centre[1], wd.centre[2]);
   if (m.memory) {
     const int now = S.ctl[kCtlEpoch];
-    const long long at = (long long)row * S.max_walls + k;
     const bool spring = m.rolling != 0;
     double hv[9];
-    const bool existed = remembered(S, memLoad(S.wmem, at, hv, spring), now);
+    const bool existed = at >= 0 && remembered(S, memLoad(S.wmem, at, hv, spring), now);
     d3 kd = zero, pn = zero, sp = zero;
     if (existed) {
       kd = mk(hv[0], hv[1], hv[2]); pn = mk(hv[3], hv[4], hv[5]);
@@ -221,7 +220,7 @@ __device__ __forceinline__ bool wallContact64(DevState const& S, GridDesc const&
     hodc64(m, S.dt, ct.point, ct.overlap, xt, vt, wt, ta.mass, ta.eqrad, wc, zero, zero, 1.e20,
            wd.eqrad, existed, kd, pn, sp, f, mr);
     const double out[9] = {kd.x, kd.y, kd.z, pn.x, pn.y, pn.z, sp.x, sp.y, sp.z};
-    memStore(S.wmem, at, out, now, spring || !existed);
+    if (at >= 0) memStore(S.wmem, at, out, now, spring || !existed);
   } else {
     hooke64(m, ct.point, ct.overlap, xt, vt, wt, ta.mass, ta.eqrad, wc, zero, zero, 1.e20,
             wd.eqrad, f, mr);
@@ -236,13 +235,12 @@ __device__ __forceinline__ bool wallContact64(DevState const& S, GridDesc const&
 }
 
 // One wall item of the evaluation: a (particle, wall) slot of the wall list
-// (spheres), whose contact is its share, or a particle of it, whose walls are
-// taken in order and summed into its first slot's share.
+// (spheres), whose contact is its share, or a particle of it (its first slot),
+// whose walls are taken in order and summed into that slot's share.
 template <bool kConvex>
 __device__ __forceinline__ void wallItem64(DevState const& S, int item, int tag, GjkTally& gjk,
                                            StatsTally& st) {
-  const int row = kConvex ? item : item / S.max_walls;
-  const int t = S.wlist[row];
+  const int t = S.wlist[item].x;
   GridDesc const& g = S.grids[S.inst[t]];
   TypeDesc const& ta = S.types[S.type[t]];
   const d3 xt = ld3(S.x, S.cap, t), vt = ld3(S.v, S.cap, t), wt = ld3(S.w, S.cap, t);
@@ -253,8 +251,11 @@ __device__ __forceinline__ void wallItem64(DevState const& S, int item, int tag,
     // the particle's polyhedron vertex runs through its wall calls in order
     curw = startVertex(S, ta, t);
     d3 Fw = mk(0., 0., 0.), Tw = mk(0., 0., 0.);
-    for (int k = 0; k < g.wall_count; ++k) {
-      if (!wallContact64<kConvex>(S, g, row, t, k, ta, xt, vt, wt, curw, walls_gjk, gjk, st, f, c, mr,
+    // (a wall without a slot is out of reach: its search is for the vertex)
+    const int end = item + S.wrow[t].y;
+    for (int k = 0, slot = item; k < g.wall_count; ++k) {
+      const int at = slot < end && S.wlist[slot].y == k ? slot++ : -1;
+      if (!wallContact64<kConvex>(S, g, at, t, k, ta, xt, vt, wt, curw, walls_gjk, gjk, st, f, c, mr,
                                   rolling))
         continue;
       Fw = Fw + f;
@@ -266,9 +267,8 @@ __device__ __forceinline__ void wallItem64(DevState const& S, int item, int tag,
     f = Fw;
     c = Tw;
     rolling = false;
-    item = row * S.max_walls;
   } else {
-    any = wallContact64<kConvex>(S, g, row, t, item - row * S.max_walls, ta, xt, vt, wt, curw,
+    any = wallContact64<kConvex>(S, g, item, t, S.wlist[item].y, ta, xt, vt, wt, curw,
                                  walls_gjk, gjk, st, f, c, mr, rolling);
   }
   if (!any) return;

@@ -232,17 +232,17 @@ struct DevState {
   // from that pair (written by the pair kernel for a contact, tagged with the
   // evaluation counter), summed in row order by the leapfrog kernel
   void* share;
-  // wall list (rebuilt with the pair list): the particles that can come near a
-  // wall before the next rebuild, and each particle's index in it (or -1);
-  // per listed particle and wall of its instance (max_walls slots) the
-  // contact memory and this evaluation's share
-  int* wlist; int* wrow;
-  int wall_cap;           // listed particles allocated
+  // wall list (rebuilt with the pair list): a slot per (particle, wall) that
+  // can come near one another before the next rebuild, a particle's slots
+  // together and in wall order; each particle's first slot and number of
+  // slots; per slot the contact memory and this evaluation's share
+  int2* wlist; int2* wrow;
+  int wall_cap;           // slots allocated
   void* wshare;           // kWallShare vectors per slot
   int* nact;              // flag words, two buffers of cap (contactFlags)
   float4* posf;           // FP32 continuous position since the last rebuild + circumscribed radius
   // this evaluation's wall items, ctl[kCtlWork]: slots of the wall list
-  // (spheres) or, with non-spherical classes, its particles
+  // (spheres) or, with non-spherical classes, the first slots of its particles
   int* work;
   int nsm;                // multiprocessors of the device (persistent grids)
   int forces_bps;         // blocks per multiprocessor of the pair kernel's persistent grid (0: the default)
@@ -351,7 +351,7 @@ __device__ __forceinline__ int listedPairs(DevState const& S) {
   return (int)min((long long)S.ctl[kCtlPairs], S.pmem.n);
 }
 __device__ __forceinline__ int listedWalls(DevState const& S) {
-  return min(S.ctl[kCtlWallRows], S.wall_cap);
+  return min(S.ctl[kCtlWallSlots], S.wall_cap);
 }
 // Whether memory last written by evaluation e is still the contact's at
 // evaluation now.

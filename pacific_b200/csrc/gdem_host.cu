@@ -48,8 +48,7 @@ const double PI = 3.14159265358979323846;
 constexpr int kCapacityCheck = 512;
 // Steps of a call's graph, and the call's steps from which it is worth building.
 constexpr int kGraphSteps = 4, kGraphFrom = 16;
-// Particles up to which a system's arrays share allocations and its wall list
-// has room for all of them.
+// Particles up to which a system's arrays and first lists share allocations.
 constexpr int kSmallSystem = 16384;
 
 struct CudaError : std::runtime_error {
@@ -907,11 +906,11 @@ struct System {
     S.wlist = nullptr; S.work = nullptr; S.wshare = nullptr;
     S.wmem = MemView{nullptr, 0};
     S.wall_cap = 0;
-    S.wrow = alloc<int>(S.any_walls ? c : 1);
-    // the wall list: every particle of a small system, a quarter of a large
-    // one's (a wall layer is far thinner; it grows when a rebuild needs more,
-    // and evaluations are put off until it has)
-    if (S.any_walls) allocateWalls(c <= kSmallSystem ? (long long)c : (long long)c / 4);
+    S.wrow = alloc<int2>(S.any_walls ? c : 1);
+    // the wall list: two slots per particle of a small system, one per two
+    // particles of a large one (a wall layer is far thinner; it grows when a
+    // rebuild needs more, and evaluations are put off until it has)
+    if (S.any_walls) allocateWalls(c <= kSmallSystem ? 2 * (long long)c + 64 : (long long)c / 2);
     S.status = alloc<int>(1);
     CK(cudaMemset(S.status, 0, sizeof(int)));
     S.law_counts = alloc<unsigned long long>(2);
@@ -982,37 +981,36 @@ struct System {
     CK(cudaStreamSynchronize(stream));
     invalidateGraphs();
   }
-  // The arrays sized by the wall list's particles (rebuilt before the next
+  // The arrays sized by the wall list's slots (rebuilt before the next
   // evaluation): the list, the evaluation's wall items, the slots' memory and
   // shares (tag words all ones: no evaluation's tag).
-  void allocateWalls(long long rows) {
-    if (rows * S.max_walls > (long long)INT_MAX - 64)
+  void allocateWalls(long long slots) {
+    if (slots > (long long)INT_MAX - 64)
       throw std::runtime_error("wall list too large for 32-bit slots");
     saveMemory(true);
     if (S.wshare) freeAlloc(S.wshare);
     S.wshare = nullptr;
     S.wall_cap = 0;
     const bool fp64 = precision == GDEM_FP64;
-    const size_t slots = (size_t)rows * S.max_walls;
     // (one allocation; every part a multiple of 16 bytes)
     auto round16 = [](size_t b) { return (b + 15) & ~size_t(15); };
     const size_t sb = slots * 16 * (fp64 ? kWallShare64 : kWallShare32);
     const size_t mb = round16(slots * (fp64 ? kMemBytes64 : kMemBytes32));
     const size_t wb = round16(slots * sizeof(int));
-    const size_t total = sb + mb + wb + rows * sizeof(int);
+    const size_t total = sb + mb + wb + slots * sizeof(int2);
     char* p = kSmallSystem >= S.cap && !S.wlist ? alloc<char>(total) : allocOwn<char>(total);
-    S.wall_cap = (int)rows;
+    S.wall_cap = (int)slots;
     S.wshare = p;
-    S.wmem = MemView{p + sb, (long long)slots};
+    S.wmem = MemView{p + sb, slots};
     S.work = reinterpret_cast<int*>(p + sb + mb);
-    S.wlist = reinterpret_cast<int*>(p + sb + mb + wb);
+    S.wlist = reinterpret_cast<int2*>(p + sb + mb + wb);
     CK(cudaMemsetAsync(S.wshare, 0xFF, sb, stream));
     static const int one = 1;
     if (S.ctl) CK(cudaMemcpyAsync(S.ctl + kCtlNeed, &one, sizeof(int), cudaMemcpyHostToDevice, stream));
     CK(cudaStreamSynchronize(stream));
     invalidateGraphs();
   }
-  // Grows the pair list (the wall list) when the most entries (particles) a
+  // Grows the pair list (the wall list) when the most entries (slots) a
   // rebuild needed since the last check exceed 80 % of the allocation, to 1.5
   // times that need; the next evaluation rebuilds.  Synchronises the stream.
   // Returns how many of the evaluations launched so far were put off, because
@@ -1022,7 +1020,7 @@ struct System {
     CK(cudaStreamSynchronize(stream));
     CK(cudaMemcpy(ctl, S.ctl, sizeof(ctl), cudaMemcpyDeviceToHost));
     CK(cudaMemsetAsync(S.ctl + kCtlEntriesMax, 0, sizeof(int), stream));
-    CK(cudaMemsetAsync(S.ctl + kCtlWallRowsMax, 0, sizeof(int), stream));
+    CK(cudaMemsetAsync(S.ctl + kCtlWallSlotsMax, 0, sizeof(int), stream));
     int off = 0;
     if (ctl[kCtlNeed] == kPutOff) {
       static const int one = 1;
@@ -1032,11 +1030,12 @@ struct System {
       CK(cudaMemcpyAsync(S.ctl + kCtlNeed, &one, sizeof(int), cudaMemcpyHostToDevice, stream));
     }
     CK(cudaStreamSynchronize(stream));
-    const int hwm = ctl[kCtlEntriesMax], rows = std::max(ctl[kCtlWallRowsMax], ctl[kCtlWallRows]);
+    const int hwm = ctl[kCtlEntriesMax];
+    const int slots = std::max(ctl[kCtlWallSlotsMax], ctl[kCtlWallSlots]);
     if ((double)hwm > 0.8 * (double)S.pair_cap)
       allocatePairs(std::max((long long)(1.5 * (double)hwm) + 4096, (long long)S.pair_cap));
-    if (S.any_walls && S.wall_cap < S.cap && (double)rows > 0.8 * (double)S.wall_cap)
-      allocateWalls(std::min((long long)S.cap, (long long)(1.5 * (double)rows) + 4096));
+    if (S.any_walls && (double)slots > 0.8 * (double)S.wall_cap)
+      allocateWalls((long long)(1.5 * (double)slots) + 4096);
     return off;
   }
   // The contact memory of the last evaluation from the lists into its table
@@ -1229,7 +1228,7 @@ struct System {
     int ctl[kCtlWords];
     CK(cudaMemcpy(ctl, S.ctl, sizeof(ctl), cudaMemcpyDeviceToHost));
     S.filter_qblocks = filterBlocks((long long)(1.25 * ctl[kCtlPairs]), S.nsm);
-    S.filter_wblocks = (int)((1.25 * ctl[kCtlWallRows]) / 256.) + 1;
+    S.filter_wblocks = (int)((1.25 * ctl[kCtlWallSlots]) / 256.) + 1;
     invalidateGraphs();
     collectTimes();
     started = true;

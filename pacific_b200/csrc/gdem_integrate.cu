@@ -94,7 +94,7 @@ __global__ void k_bin(DevState S, const int* gate) {
   // memory has been saved)
   if (s == 0) {
     S.ctl[kCtlPairs] = 0;
-    S.ctl[kCtlWallRows] = 0;
+    S.ctl[kCtlWallSlots] = 0;
   }
   if (s >= S.n) return;
   const int key = buildKey(S.bgrids[S.inst[s]], ld3(S.x, S.cap, s), S.status);
@@ -335,11 +335,11 @@ __device__ __forceinline__ void sumShares(DevState const& S, int t, TypeDesc con
     }
     if (na & kNearWall) {
       // the walls' own sum first, in wall order
+      const int2 row = S.wrow[t];
       const float4* ws = static_cast<const float4*>(S.wshare) +
-                         (size_t)kWallShare32 * S.wrow[t] * S.max_walls;
+                         (size_t)kWallShare32 * row.x;
       float wx = 0.f, wy = 0.f, wz = 0.f, ux = 0.f, uy = 0.f, uz = 0.f;
-      const int nw = S.grids[S.inst[t]].wall_count;
-      for (int k = 0; k < nw; ++k, ws += kWallShare32) {
+      for (int k = 0; k < row.y; ++k, ws += kWallShare32) {
         const float4 a = ws[0];
         if (__float_as_int(a.w) != tag) continue;
         const float4 b = ws[1];
@@ -391,11 +391,11 @@ __device__ __forceinline__ void sumShares(DevState const& S, int t, TypeDesc con
       }
     }
     if (na & kNearWall) {
+      const int2 row = S.wrow[t];
       const double2* ws = static_cast<const double2*>(S.wshare) +
-                          (size_t)kWallShare64 * S.wrow[t] * S.max_walls;
+                          (size_t)kWallShare64 * row.x;
       d3 Fw = mk(0., 0., 0.), Tw = mk(0., 0., 0.);
-      const int nw = S.grids[S.inst[t]].wall_count;
-      for (int k = 0; k < nw; ++k, ws += kWallShare64) {
+      for (int k = 0; k < row.y; ++k, ws += kWallShare64) {
         const double2 a = ws[0];
         if ((int)__double_as_longlong(a.x) != tag) continue;
         const double2 b = ws[1], c = ws[2], d = ws[3];
@@ -573,73 +573,73 @@ __device__ __forceinline__ bool nearWall(GridDesc const& bg, WallDesc const& wd,
   return d2 <= p.R * p.R;
 }
 
-// The wall list: particles within the skin of a wall or of a periodic image of
-// one, which no other can reach before the next rebuild (part of a rebuild,
+// The wall list: the walls, or periodic images of them, within the skin of each
+// particle; it can reach no others before the next rebuild (part of a rebuild,
 // after k_copyback).
 __global__ void k_wall_rows(DevState S, const int* gate) {
   if (gatedOff(gate)) return;
+  const unsigned full = 0xffffffffu;
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  bool near = false;
-  if (t < S.n) {
-    const int inst = S.inst[t];
-    GridDesc const& bg = S.bgrids[inst];
-    const WallProbe p = wallProbe(S, t, bg, bg.skin_f);
-    for (int k = 0; k < bg.wall_count && !near; ++k) 
-      near = nearWall(bg, S.walls[bg.wall_begin + k], p, true);
-  }
-  const unsigned m = __ballot_sync(0xffffffffu, near);
   const int lane = threadIdx.x & 31;
+  int count = 0, begin = 0, nw = 0;
+  WallProbe p{};
+  GridDesc const* bg = nullptr;
+  if (t < S.n) {
+    bg = &S.bgrids[S.inst[t]];
+    begin = bg->wall_begin;
+    nw = bg->wall_count;
+    p = wallProbe(S, t, *bg, bg->skin_f);
+    for (int k = 0; k < nw; ++k) count += nearWall(*bg, S.walls[begin + k], p, true);
+  }
+  int incl = count;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int y = __shfl_up_sync(full, incl, o);
+    if (lane >= o) incl += y;
+  }
   int base = 0;
-  if (lane == 0 && m) base = atomicAdd(S.ctl + kCtlWallRows, __popc(m));
-  const int row = __shfl_sync(0xffffffffu, base, 0) + __popc(m & ((1u << lane) - 1u));
+  if (lane == 31 && incl) base = atomicAdd(S.ctl + kCtlWallSlots, incl);
+  int slot = __shfl_sync(full, base, 31) + incl - count;
   if (t >= S.n) return;
-  S.wrow[t] = near ? row : -1;
-  if (!near) return;
-  if (row < S.wall_cap) S.wlist[row] = t;
-  else S.ctl[kCtlNeed] = kPutOff;
+  S.wrow[t] = make_int2(slot, count);
+  if (!count) return;
+  if (slot > S.wall_cap - count) {
+    S.ctl[kCtlNeed] = kPutOff;
+    return;
+  }
+  for (int k = 0; k < nw; ++k)
+    if (nearWall(*bg, S.walls[begin + k], p, true)) S.wlist[slot++] = make_int2(t, k);
 }
 
-// This evaluation's wall items: for spheres every near (particle, wall) slot
-// of the wall list, else the particles near any wall (their walls are taken in
-// turn: a polyhedron's support vertex runs through them).
+// This evaluation's wall items: for spheres every near slot of the wall list,
+// else the first slots of the particles near any wall (their walls are taken
+// in turn: a polyhedron's support vertex runs through them).
 __device__ __forceinline__ void filterWalls(DevState const& S, int* flags, int nblocks) {
-  const unsigned full = 0xffffffffu;
   const int lane = threadIdx.x & 31;
-  const int nr = listedWalls(S);
-  for (int r0 = (int)(blockIdx.x * blockDim.x + threadIdx.x) & ~31; r0 < nr;
-       r0 += nblocks * blockDim.x) {   // warp-uniform
-    const int row = r0 + lane;
-    int count = 0, t = 0, begin = 0, nw = 0;
-    WallProbe p{};
-    GridDesc const* bg = nullptr;
-    if (row < nr) {
-      t = S.wlist[row];
-      bg = &S.bgrids[S.inst[t]];
-      p = wallProbe(S, t, *bg, 0.f);
-      begin = bg->wall_begin;
-      nw = bg->wall_count;
-      for (int k = 0; k < nw; ++k) count += nearWall(*bg, S.walls[begin + k], p, false);
-      if (count) flags[t] = (int)kCandidate;
-      if (S.any_convex) count = min(count, 1);
+  const int ns = listedWalls(S);
+  for (int s0 = (int)(blockIdx.x * blockDim.x + threadIdx.x) & ~31; s0 < ns;
+       s0 += nblocks * blockDim.x) {   // warp-uniform
+    const int slot = s0 + lane;
+    bool near = false;
+    if (slot < ns) {
+      const int2 e = S.wlist[slot];
+      int last = slot;
+      if (S.any_convex) {
+        const int2 row = S.wrow[e.x];
+        last = row.x == slot ? slot + row.y - 1 : slot - 1;
+      }
+      GridDesc const& bg = S.bgrids[S.inst[e.x]];
+      const WallProbe p = wallProbe(S, e.x, bg, 0.f);
+      for (int s = slot; s <= last && !near; ++s)
+        near = nearWall(bg, S.walls[bg.wall_begin + (s == slot ? e.y : S.wlist[s].y)], p, false);
+      if (near) flags[e.x] = (int)kCandidate;
     }
-    int incl = count;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const int y = __shfl_up_sync(full, incl, o);
-      if (lane >= o) incl += y;
-    }
-    const int total = __shfl_sync(full, incl, 31);
-    if (!total) continue;
+    const unsigned m = __ballot_sync(0xffffffffu, near);
+    if (!m) continue;
     int at = 0;
-    if (lane == 0) at = atomicAdd(S.ctl + kCtlWork, total);
-    at = __shfl_sync(full, at, 0) + incl - count;
-    if (!count) continue;
-    if (S.any_convex) {
-      S.work[at] = row;
-    } else {
-      for (int k = 0; k < nw; ++k)
-        if (nearWall(*bg, S.walls[begin + k], p, false)) S.work[at++] = row * S.max_walls + k;
-    }
+    if (lane == 0) at = atomicAdd(S.ctl + kCtlWork, __popc(m));
+    at = __shfl_sync(0xffffffffu, at, 0) + __popc(m & ((1u << lane) - 1u));
+    if (near) S.work[at] = slot;
   }
 }
 
@@ -828,22 +828,20 @@ __global__ void k_coordination_by_id(DevState S, int* out, int id_base) {
 }
 
 // Contact memory between the lists and the table.  Entries 0 .. pairs - 1 are
-// the compact pair list's, then come the wall list's slots.
-__device__ __forceinline__ bool memEntry(DevState const& S, int np, long long i, MemView& m,
+// the compact pair list's, then come the wall list's.
+__device__ __forceinline__ void memEntry(DevState const& S, int np, long long i, MemView& m,
                                          long long& at, unsigned long long& key) {
   if (i < np) {
     const int2 pr = S.upairs[i];
     m = S.pmem;
     at = i;
     key = pairKey(S.id[pr.x], S.id[(unsigned)pr.y & ((1u << 27) - 1u)]);
-    return true;
+    return;
   }
   m = S.wmem;
   at = i - np;
-  const int row = (int)(at / S.max_walls), k = (int)(at % S.max_walls);
-  const int t = S.wlist[row];
-  key = wallKey(S.id[t], k);
-  return k < S.grids[S.inst[t]].wall_count;
+  const int2 e = S.wlist[at];
+  key = wallKey(S.id[e.x], e.y);
 }
 
 // Frees the table's slots before the lists' memory is saved (the plain step).
@@ -862,13 +860,13 @@ __global__ void k_mem_save(DevState S, const int* gate, int back) {
   if (gatedOff(gate) || !S.ctl[kCtlMemory]) return;
   const int now = S.ctl[kCtlEpoch] - back;
   const int np = listedPairs(S);
-  const long long ne = np + (long long)listedWalls(S) * S.max_walls;
+  const long long ne = np + listedWalls(S);
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < ne;
        i += (long long)gridDim.x * blockDim.x) {
     MemView m;
     long long at;
     unsigned long long key;
-    if (!memEntry(S, np, i, m, at, key)) continue;
+    memEntry(S, np, i, m, at, key);
     if (!remembered(S, memEvaluation(m, at, T()), now + 1)) continue;
     T v[9];
     memLoad(m, at, v, true);
@@ -891,24 +889,24 @@ __global__ void k_mem_load(DevState S, const int* gate) {
   const bool off = S.ctl[kCtlNeed] == kPutOff;
   if (i0 == 0) {
     S.ctl[kCtlMemory] = off ? 0 : 1;
-    S.ctl[kCtlWallRowsMax] = max(S.ctl[kCtlWallRowsMax], S.ctl[kCtlWallRows]);
+    S.ctl[kCtlWallSlotsMax] = max(S.ctl[kCtlWallSlotsMax], S.ctl[kCtlWallSlots]);
     if (off) {
       // (the table keeps the memory)
       S.ctl[kCtlPairs] = 0;
-      S.ctl[kCtlWallRows] = 0;
+      S.ctl[kCtlWallSlots] = 0;
       S.ctl[kCtlEpoch] -= 1;
       S.ctl[kCtlRebuilds] -= 1;
     }
   }
   if (off) return;
   const int np = listedPairs(S);
-  const long long ne = np + (long long)listedWalls(S) * S.max_walls;
+  const long long ne = np + listedWalls(S);
   for (long long i = i0; i < ne; i += (long long)gridDim.x * blockDim.x) {
     MemView m;
     long long at;
     unsigned long long key;
-    const bool used = memEntry(S, np, i, m, at, key);
-    const int s = used ? histFind(S.hist, key, 0) : -1;
+    memEntry(S, np, i, m, at, key);
+    const int s = histFind(S.hist, key, 0);
     if (s < 0) { memForget(m, at, T()); continue; }
     const T* d = static_cast<const T*>(S.hist.vals) + 9 * (size_t)s;
     T v[9];
@@ -928,7 +926,7 @@ __global__ void k_mem_zero_cumulative(DevState S) {
   const long long stride = (long long)gridDim.x * blockDim.x;
   const int now = S.ctl[kCtlEpoch];
   const int np = listedPairs(S);
-  const long long ne = np + (long long)listedWalls(S) * S.max_walls;
+  const long long ne = np + listedWalls(S);
   for (long long i = i0; i < ne; i += stride) {
     MemView m = i < np ? S.pmem : S.wmem;
     const long long at = i < np ? i : i - np;

@@ -31,7 +31,7 @@ enum CtlWords : int {
   kCtlActive = 1,   // this step rebuilds the pair list (set by k_decide)
   kCtlEpoch = 2,    // force evaluations so far (tags shares and contact memory)
   kCtlRebuilds = 3, // pair-list rebuilds so far
-  kCtlWork = 4,     // particles near a wall this evaluation (contact filter)
+  kCtlWork = 4,     // wall items of this evaluation (contact filter)
   kCtlPairs = 5,    // pairs of the compact pair list (set by the rebuild)
   kCtlKept = 6,     // pairs kept by this evaluation's contact filter
   kCtlEntries = 7,  // pair-list entries of the last rebuild
@@ -40,12 +40,12 @@ enum CtlWords : int {
   kCtlKept2 = 10,    // of those, the pairs the first search iteration left undecided (kept2)
   kCtlRounds = 11,   // rounds of 32 pairs per append of this evaluation's contact filter
   kCtlMemory = 12,   // the pair and wall lists hold the contact memory (else the table does)
-  kCtlWallRows = 13, // particles of the wall list
-  kCtlWallRowsMax = 14,  // most wall-list particles of any rebuild since the last allocation check
+  kCtlWallSlots = 13,    // slots of the wall list
+  kCtlWallSlotsMax = 14, // most wall-list slots of any rebuild since the last allocation check
   kCtlWords = 16
 };
 // Value of kCtlNeed where an evaluation is put off: its rebuild found more
-// particles near a wall than the wall list has room for.  That evaluation and
+// (particle, wall) pairs than the wall list has room for.  That evaluation and
 // those after it (whose rebuilds find the same) leave the state as it is: the
 // lists are empty, the leapfrog moves nothing.  They are not counted; the host
 // makes them once it has enlarged the list, so no wall contact is left out.
