@@ -1228,7 +1228,7 @@ struct System {
     int ctl[kCtlWords];
     CK(cudaMemcpy(ctl, S.ctl, sizeof(ctl), cudaMemcpyDeviceToHost));
     S.filter_qblocks = filterBlocks((long long)(1.25 * ctl[kCtlPairs]), S.nsm);
-    S.filter_wblocks = (int)((1.25 * ctl[kCtlWallSlots]) / 256.) + 1;
+    S.filter_wblocks = wallBlocks(ctl[kCtlWallSlots], S.n);
     invalidateGraphs();
     collectTimes();
     started = true;
@@ -1461,6 +1461,7 @@ int gdem_insert_particle(gdem_handle h, int type, const double* x, const double*
     // the contact filter's grid, for about 4 pairs per particle (its kernel
     // loops over any excess)
     S.filter_qblocks = std::max(S.filter_qblocks, filterBlocks(4ll * S.n, S.nsm));
+    S.filter_wblocks = std::max(S.filter_wblocks, wallBlocks(0, S.n));
     s->invalidateGraphs();
     *inserted = 1;
     if (id) *id = p.id;

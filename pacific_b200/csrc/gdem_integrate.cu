@@ -1143,11 +1143,13 @@ int filterBlocks(long long pairs, int nsm) {
   const long long full = (pairs + 2047) / 2048, one = (pairs + 255) / 256;
   return (int)std::max(1ll, std::max(full, std::min(one, 4ll * nsm)));
 }
+int wallBlocks(long long slots, int n) {
+  return std::max(blocks(n, 2048), (int)(5 * slots / 1024) + 1);
+}
 void launch_filter(DevState const& S, cudaStream_t st) {
   if (!S.n) return;
-  // an eighth of the particles until the leapfrog start has counted the wall list
   const int pblocks =
-      S.any_walls ? (S.filter_wblocks > 0 ? S.filter_wblocks : blocks(blocks(S.n, 8), 256)) : 0;
+      S.any_walls ? (S.filter_wblocks > 0 ? S.filter_wblocks : wallBlocks(0, S.n)) : 0;
   // about 4 pairs per particle until the leapfrog start has counted them
   const int qblocks = S.filter_qblocks > 0 ? S.filter_qblocks : filterBlocks(4ll * S.n, S.nsm);
   if (S.any_convex && !S.pos64) k_filter<true><<<pblocks + qblocks, 256, 0, st>>>(S, pblocks);

@@ -60,6 +60,11 @@ void launch_filter(DevState const& S, cudaStream_t st);
 // without four blocks per multiprocessor (a small system's pairs are then
 // tested in one round each).
 int filterBlocks(long long pairs, int nsm);
+// And for the wall list: a slot per thread and a quarter more for growth, and
+// for the time when more particles reach the walls no fewer than one block per
+// 2,048 particles (90,000 spheres that land on a floor after the leapfrog
+// start: FP32-split step 28.4 us, 44.2 with the one block of an empty list).
+int wallBlocks(long long slots, int n);
 void launch_link(DevState const& S, const int* gate, cudaStream_t st);
 void launch_wall_rows(DevState const& S, const int* gate, cudaStream_t st);
 void launch_diag_prefill(DevState const& S, cudaStream_t st);
