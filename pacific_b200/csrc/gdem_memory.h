@@ -26,18 +26,19 @@ class DeviceMemory {
     if (p) own_.push_back(p);
     return p;
   }
-  // block: bytes of a block opened for it.  An array for which no block can
-  // be had gets an allocation of its own.
+  // block: bytes of a block opened for it (a longer array has a block to
+  // itself).  An array for which no block can be had gets an allocation of its
+  // own.
   void* shared(std::size_t bytes, std::size_t block) {
     bytes = (std::max<std::size_t>(bytes, 1) + 255) & ~std::size_t(255);
     if (left_ < bytes) {
-      block = std::max(bytes, block);
-      void* p = take_(block);
+      void* p = take_(std::max(bytes, block));
       if (!p) return own(bytes);
       blocks_.push_back(p);
+      total_ += std::max(bytes, block);
+      if (bytes >= block) return p;
       at_ = static_cast<char*>(p);
       left_ = block;
-      total_ += block;
     }
     void* r = at_;
     at_ += bytes;

@@ -54,7 +54,8 @@ PROGRAM = textwrap.dedent(r"""
             arrays[u] = n;
           };
           auto shared = [&](std::size_t n) {
-            void* p = m.shared(n, std::max((cap + 64) * 4096, m.sharedTotal()));
+            // (small blocks, which some arrays exceed, and large ones)
+            void* p = m.shared(n, cap % 2 ? 1 << 18 : std::max((cap + 64) * 4096, m.sharedTotal()));
             add(p, n);
             return p;
           };
