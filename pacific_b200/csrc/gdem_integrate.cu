@@ -443,12 +443,11 @@ __global__ void __launch_bounds__(kMoveBlock<kFast, kBasis>(), kBasis ? 2 : (kFa
     k_move(DevState S, int flags) {
   int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= S.n) return;
-  const int need = S.ctl[kCtlNeed];
   TypeDesc const& tp = S.types[S.type[t]];
   MoveIn m;
   loadMoveIn<kFast, kBasis>(S, t, m);   // nothing the contact kernels write
   const bool sum = (flags & kStepSum) != 0;
-  if (sum && need == kPutOff) return;
+  if (sum && S.any_walls && S.ctl[kCtlNeed] == kPutOff) return;
   d3 F, T;
   bool candidate = false;
   if (sum) {
