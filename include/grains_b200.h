@@ -202,8 +202,8 @@ int gdem_download_history(gdem_handle h, int64_t capacity, int64_t* count, int* 
  * radius (it sets the pair-list cell size, 2 rmax f + skin, and how often the
  * list is rebuilt; < 0 restores the LinkedCell Skin attribute or 0.25);
  * blocks_per_sm is the force kernels' persistent grid, in blocks per
- * multiprocessor (<= 0: the default, 4, or 3 for spheres in FP32-split).  Results do not depend on
- * either. */
+ * multiprocessor (<= 0: the default, 4; spheres in FP32-split never get more
+ * than the 3 that fit).  Results do not depend on either. */
 int gdem_set_tuning(gdem_handle h, double skin_factor, int blocks_per_sm);
 
 /* Autotuner, before gdem_init: steps copies of the uploaded system for

@@ -746,7 +746,12 @@ void launch_pairsep32(DevState const& S, cudaStream_t st) {
 }
 void launch_pairlaw32(DevState const& S, cudaStream_t st) {
   if (!S.n) return;
-  const int grid = (S.forces_bps > 0 ? S.forces_bps : (S.any_convex ? 4 : 3)) * S.nsm;
+  int bps = S.forces_bps > 0 ? S.forces_bps : 4;
+  // the sphere kernel's three resident blocks at most: a fourth would wait for
+  // one of them to end with its own share of the items (bed of 250,000: step
+  // 151 us, with four 195, with eight 166)
+  if (!S.any_convex) bps = std::min(bps, 3);
+  const int grid = bps * S.nsm;
   if (S.any_convex) launchAfterPrevious(k_pairlaw32<true>, grid, 128, st, S);
   else launchAfterPrevious(k_pairlaw32<false>, grid, 128, st, S);
 }

@@ -1810,7 +1810,7 @@ int gdem_autotune(gdem_handle h, int trial_steps, double* skin_factor, int* bloc
     const double skins[] = {0.1, 0.175, 0.25, 0.4, 0.6};
     const int bpss[] = {2, 4, 8};
     double best = 1.e300, best_sf = 0.25;
-    int best_bps = 4;
+    int best_bps = 4;   // (the default)
     for (double sf : skins) {
       const double ms = trial(sf, 4);
       if (ms < best) { best = ms; best_sf = sf; }
