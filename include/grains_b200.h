@@ -428,7 +428,9 @@ void gdem_destroy(gdem_handle h);
  * with respect to params = (kn, en, muc) (replacing those of every contact
  * model of the XML) and the initial velocities, by a reverse sweep over the
  * steps with the transposed leapfrog and contact-force Jacobians, recomputing
- * states from checkpoints taken every checkpoint_every steps. */
+ * states from checkpoints taken every checkpoint_every steps.  The device
+ * memory that a run works in (blocks of 32 MB or more) is kept for the next
+ * one, up to 1 GiB per handle, until gdem_adjoint_destroy. */
 typedef struct gdem_adjoint* gdem_adjoint_handle;
 int gdem_adjoint_create(const char* xml_path, gdem_adjoint_handle* out);
 /* Particles by index: class, x0, v0 (3 each), w0 (3 each; NULL: zero). */
