@@ -153,10 +153,10 @@ __device__ __forceinline__ int memEvaluation(MemView m, long long i, double) {
   return (int)__double_as_longlong(static_cast<const double2*>(m.p)[m.n + i].y);
 }
 __device__ __forceinline__ void memForget(MemView m, long long i, float) {
-  static_cast<float4*>(m.p)[i].w = __int_as_float(-1);
+  static_cast<float4*>(m.p)[i].w = __int_as_float(kNeverWritten);
 }
 __device__ __forceinline__ void memForget(MemView m, long long i, double) {
-  static_cast<double2*>(m.p)[m.n + i].y = __longlong_as_double(-1ll);
+  static_cast<double2*>(m.p)[m.n + i].y = __longlong_as_double((long long)kNeverWritten);
 }
 
 // Overlap statistics of the contacts over the evaluations since the last
@@ -353,10 +353,8 @@ __device__ __forceinline__ int listedPairs(DevState const& S) {
 __device__ __forceinline__ int listedWalls(DevState const& S) {
   return min(S.ctl[kCtlWallSlots], S.wall_cap);
 }
-// Whether memory last written by evaluation e is still the contact's at
-// evaluation now.
 __device__ __forceinline__ bool remembered(DevState const& S, int e, int now) {
-  return S.prune ? e == now - 1 : e >= 0;
+  return memoryHolds(S.prune, e, now);
 }
 
 // Cell of a neighbour offset (di, dj, dk) around (i, j, k) of grid g, with

@@ -51,6 +51,19 @@ enum CtlWords : int {
 // makes them once it has enlarged the list, so no wall contact is left out.
 constexpr int kPutOff = 2;
 
+// Whether contact memory that evaluation e wrote last (kNeverWritten: none) is
+// the contact's at evaluation now: the evaluation's before with the plain step
+// (prune), any with the coupled one.  Evaluations are counted in 32 bits that
+// wrap (at 35 us a step INT_MAX comes after 21 hours), so no count is too large
+// or negative to be one.
+constexpr int kNeverWritten = -1;
+#ifdef __CUDACC__
+__host__ __device__
+#endif
+inline bool memoryHolds(int prune, int e, int now) {
+  return e != kNeverWritten && (!prune || (unsigned)e == (unsigned)now - 1u);
+}
+
 // One independent simulation ("instance").  A single Grains3D system is a
 // batch of one.  Cell numbering follows LinkedCell::getCellNumber
 // (Base/src/LinkedCell.cpp:1165-1168): j * nbk * nbi + k * nbi + i.
