@@ -9,7 +9,7 @@
 namespace gdem {
 
 // Contact memory.  It lives beside what uses it: per pair of the compact pair
-// list and per wall of each particle in the wall list (MemView), where the
+// list and per (particle, wall) of the wall list (MemView), where the
 // pair kernel's lanes read and write it in list order.  Values are as seen
 // from the lower-ID body (or the particle, for a wall); the other body's view
 // is the negation, as in the reference where p1 holds (-kdelta, -normal,
@@ -28,11 +28,8 @@ namespace gdem {
 // random places of two tables: 1M spheres 5 of the pair kernel's 24 us, a
 // packed bed two thirds of its memory traffic.)
 //
-// Key layout: bits 54-63 a tag (0 for an entry, 1023 for a free slot), bits
-// 27-53 the lower particle ID, bits 0-26 the higher particle ID or, for a
-// wall, 2^27 - 1 - wall index.
-constexpr int kTagShift = 54;
-constexpr unsigned kTagMask = 1023u;
+// Key layout: bits 27-53 the lower particle ID, bits 0-26 the higher particle
+// ID or, for a wall, 2^27 - 1 - wall index; kEmptyKey in a free slot.
 constexpr int kMaxIdBits = 27;
 constexpr unsigned long long kEmptyKey = 0xFFFFFFFFFFFFFFFFull;
 
@@ -49,12 +46,6 @@ __host__ __device__ inline unsigned long long wallKey(int id, int wall) {
   return ((unsigned long long)(uint32_t)id << kMaxIdBits) |
          (uint32_t)((1 << kMaxIdBits) - 1 - wall);
 }
-__host__ __device__ inline unsigned long long tagged(unsigned long long base, unsigned tag) {
-  return ((unsigned long long)(tag & kTagMask) << kTagShift) | base;
-}
-__host__ __device__ inline unsigned tagOf(unsigned long long key) {
-  return (unsigned)(key >> kTagShift);
-}
 __host__ __device__ inline uint32_t hashSlot(unsigned long long k, int log2cap) {
   k ^= k >> 33;
   k *= 0xff51afd7ed558ccdull;
@@ -63,36 +54,27 @@ __host__ __device__ inline uint32_t hashSlot(unsigned long long k, int log2cap) 
   k ^= k >> 33;
   return (uint32_t)(k & ((1ull << log2cap) - 1));
 }
-// Slot holding base with tag, or -1.
-__device__ inline int histFind(HistTable const& t, unsigned long long base, unsigned tag) {
+// Slot holding key, or -1.
+__device__ inline int histFind(HistTable const& t, unsigned long long key) {
   const uint32_t mask = (1u << t.log2cap) - 1;
-  const unsigned long long key = tagged(base, tag);
-  uint32_t s = hashSlot(base, t.log2cap);
+  uint32_t s = hashSlot(key, t.log2cap);
   for (uint32_t probe = 0; probe <= mask; ++probe) {
     const unsigned long long k = t.keys[s];
     if (k == key) return (int)s;
-    if (tagOf(k) != (tag & kTagMask)) return -1;
+    if (k == kEmptyKey) return -1;
     s = (s + 1) & mask;
   }
   return -1;
 }
-// Claims a slot for base with tag (one writer per key at a time); -1
-// when every slot carries the tag already (table full).
-__device__ inline int histInsert(HistTable const& t, unsigned long long base, unsigned tag) {
+// The slot of key, claimed if need be (one writer per key at a time); -1 when
+// the table is full.
+__device__ inline int histInsert(HistTable const& t, unsigned long long key) {
   const uint32_t mask = (1u << t.log2cap) - 1;
-  const unsigned long long key = tagged(base, tag);
-  uint32_t s = hashSlot(base, t.log2cap);
+  uint32_t s = hashSlot(key, t.log2cap);
   for (uint32_t probe = 0; probe <= mask; ++probe) {
     unsigned long long cur = t.keys[s];
-    for (;;) {
-      if (tagOf(cur) == (tag & kTagMask)) {
-        if (cur == key) return (int)s;
-        break;                                   // taken this evaluation
-      }
-      const unsigned long long prev = atomicCAS(&t.keys[s], cur, key);
-      if (prev == cur) return (int)s;
-      cur = prev;                                // raced: look again
-    }
+    if (cur == kEmptyKey) cur = atomicCAS(&t.keys[s], kEmptyKey, key);
+    if (cur == kEmptyKey || cur == key) return (int)s;
     s = (s + 1) & mask;
   }
   return -1;
@@ -570,8 +552,8 @@ __device__ __forceinline__ WarpItems warpItems(int n) {
 }
 
 // Contact-filter flags of the current force evaluation: two buffers used
-// alternately, the filter of one evaluation clearing the other's, so that no
-// kernel needs to clear flags that other warps may still be setting.
+// alternately, the leapfrog kernel of one evaluation clearing the other's, so
+// that no kernel needs to clear flags that other warps may still be setting.
 __device__ __forceinline__ int* contactFlags(DevState const& S, int which = 0) {
   return S.nact + (size_t)(((unsigned)S.ctl[kCtlEpoch] + (unsigned)which) & 1u) * S.cap;
 }

@@ -1646,9 +1646,7 @@ int gdem_upload_history(gdem_handle h, int64_t n, const int* owner, const int* p
     // them and takes the memory from it
     HistTable& t = S.hist;
     size_t hc = size_t(1) << t.log2cap;
-    const unsigned tag = 0;
-    const unsigned long long empty = kEmptyKey;
-    std::vector<unsigned long long> keys(hc, empty);
+    std::vector<unsigned long long> keys(hc, kEmptyKey);
     bool fp64 = s->precision == GDEM_FP64;
     std::vector<double> vd(fp64 ? 9 * hc : 0);
     std::vector<float> vf(fp64 ? 0 : 9 * hc);
@@ -1662,8 +1660,8 @@ int gdem_upload_history(gdem_handle h, int64_t n, const int* owner, const int* p
         key = wallKey(a, -b - 2);
       }
       uint32_t slot = hashSlot(key, t.log2cap);
-      while (keys[slot] != empty) slot = (slot + 1) & (uint32_t)(hc - 1);
-      keys[slot] = tagged(key, tag);
+      while (keys[slot] != kEmptyKey) slot = (slot + 1) & (uint32_t)(hc - 1);
+      keys[slot] = key;
       double vals[9] = {kdelta[3 * e], kdelta[3 * e + 1], kdelta[3 * e + 2],
                         prevn[3 * e], prevn[3 * e + 1], prevn[3 * e + 2],
                         spring ? spring[3 * e] : 0., spring ? spring[3 * e + 1] : 0.,
@@ -1704,11 +1702,10 @@ int gdem_download_history(gdem_handle h, int64_t capacity, int64_t* count, int* 
     else CK(cudaMemcpy(vf.data(), t.vals, vf.size() * sizeof(float), cudaMemcpyDeviceToHost));
     struct Rec { int a, b; double v[9]; };
     std::vector<Rec> recs;
-    const unsigned tag = 0;
     const unsigned idmask = (1u << kMaxIdBits) - 1u;
     const unsigned n = (unsigned)S.n;
     for (size_t k = 0; k < hc; ++k) {
-      if (tagOf(keys[k]) != tag) continue;
+      if (keys[k] == kEmptyKey) continue;
       const unsigned hi = (unsigned)((keys[k] >> kMaxIdBits) & idmask);
       const unsigned lo = (unsigned)(keys[k] & idmask);
       if (hi >= n) continue;
@@ -2138,10 +2135,9 @@ static int writeReloadParticles(gdem_handle h, const char* path, bool hybrid) {
     if (fp64) CK(cudaMemcpy(vd.data(), t.vals, vd.size() * sizeof(double), cudaMemcpyDeviceToHost));
     else CK(cudaMemcpy(vf.data(), t.vals, vf.size() * sizeof(float), cudaMemcpyDeviceToHost));
     std::vector<std::vector<MapEntry>> maps(n);
-    const unsigned tag = 0;
     const unsigned idmask = (1u << kMaxIdBits) - 1u;
     for (size_t k = 0; k < hc; ++k) {
-      if (tagOf(keys[k]) != tag) continue;
+      if (keys[k] == kEmptyKey) continue;
       const unsigned base_hi = (unsigned)((keys[k] >> kMaxIdBits) & idmask);
       const unsigned base_lo = (unsigned)(keys[k] & idmask);
       double val[9];

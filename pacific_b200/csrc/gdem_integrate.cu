@@ -416,14 +416,19 @@ __device__ __forceinline__ void sumShares(DevState const& S, int t, TypeDesc con
 template <bool kFast, bool kBasis>
 constexpr int kMoveBlock() { return kBasis ? 256 : 128; }
 
-// Leapfrog of each particle (128-thread blocks: FP32-split spheres eight per
-// multiprocessor at 64 registers; measured faster at 1M than 256-thread blocks
-// at three, four or five: it is bound by the latency of its loads.  FP64
-// spheres six at 80: 256,000 spheres 22.8 us, 22.1 with five, 22.4 with
-// seven, but a packed bed of 60,000 17.9 us against 16.9 and 18.7).  With an
-// orientation matrix: two 256-thread blocks, an instantiation of its own in
-// both modes (a convex FP64 pour's move 21.5 -> 13.8 us).  With kStepSum the force and torque of this
-// evaluation: the weight for a particle the contact filter did not mark as a
+// Leapfrog of each particle.  Launch bounds, by the whole step: the kernel
+// starts while the pair kernel runs, so its own time is not all that counts.
+// FP32-split spheres: 128-thread blocks, eight per multiprocessor at 64
+// registers (1M: faster than 256-thread blocks at three, four or five; bound by
+// the latency of its loads).  FP64 spheres: six at 80 registers; 256,000 gas
+// spheres step 50.7 us, with five 52.0, with seven 52.7, 60,000 packed 63.9,
+// 65.0 and 66.4, although alone the kernel is as fast or faster with five (23.1
+// and 23.1 us, 18.6 and 17.4).  With an orientation matrix: two 256-thread
+// blocks, an instantiation of its own in both modes (a convex FP64 pour's move
+// 21.5 -> 13.8 us).
+//
+// With kStepSum the force and torque of this evaluation: the weight for a
+// particle the contact filter did not mark as a
 // candidate, else the weight plus its shares (sumShares); without it, the
 // stored F, T (the opening kick of a call continues from the last evaluation
 // of the previous one).  Then the closing kick of the step that ends
@@ -492,20 +497,6 @@ __global__ void __launch_bounds__(kMoveBlock<kFast, kBasis>(), kBasis ? 2 : (kFa
   }
 }
 
-// Contact filter.  One lane per pair of the compact pair list (each pair
-// once, from its lower ID): the FP32 bounding-sphere test, a superset of the
-// contacts; the kept pairs are listed for the pair kernel, which decides each
-// exactly, and both partners marked as candidates.  With walls, the first
-// pblocks blocks take the wall list.  A warp tests `rounds` rounds of 32 pairs, then appends all it kept
-// with one atomic: where the last evaluation kept more than an eighth of the
-// pairs (a packed bed, colliding convex bodies) up to kFilterRounds of them,
-// else one, whose append then overlaps the other warps' loads.  A grid-stride
-// loop covers any count (known on the device only).
-// What bounds it: in a gas (few pairs kept) the latency of the position
-// gathers (1M spheres: 20.9 us with 1 round, 23.1 with 8); in a bed the marks
-// and the appends, which were two atomics per kept pair and one per 32 pairs
-// on a single counter (250,000 packed spheres, 737,000 pairs kept: 32.9 us
-// then, 31.3 with plain marks and 1 round, 22.5 with 8 rounds).
 // Appends the kept pairs of a warp's rounds to a list that grows upwards
 // (dir 1) or downwards (dir -1) from list[0] and marks their partners: lane j
 // holds the ballot of round j in mine (0 beyond the rounds), round j's pairs
@@ -642,6 +633,22 @@ __device__ __forceinline__ void filterWalls(DevState const& S, int* flags, int n
   }
 }
 
+// Contact filter.  One lane per pair of the compact pair list (each pair
+// once, from its lower ID): the FP32 bounding-sphere test, a superset of the
+// contacts; the kept pairs are listed for the pair kernel, which decides each
+// exactly, and both partners marked as candidates.  With walls, the first
+// pblocks blocks take the wall list (filterWalls).  A warp tests `rounds`
+// rounds of 32 pairs, then appends all it kept with one atomic: where the last
+// evaluation kept more than an eighth of the pairs (a packed bed, colliding
+// convex bodies) up to kFilterRounds of them, else one, whose append then
+// overlaps the other warps' loads.  A grid-stride loop covers any count (known
+// on the device only).
+// What bounds it: in a gas (few pairs kept) the latency of the position
+// gathers (1M spheres: 20.9 us with 1 round, 23.1 with 8); in a bed the marks
+// and the appends, which were two atomics per kept pair and one per 32 pairs
+// on a single counter (250,000 packed spheres, 737,000 pairs kept: 32.9 us
+// then, 31.3 with plain marks and 1 round, 22.5 with 8 rounds; 16.7 since the
+// walls are tested for the wall list only).
 // kSplit: FP32-split with non-spherical classes (the kept pairs in two lists).
 template <bool kSplit>
 __global__ void __launch_bounds__(256, 8) k_filter(DevState S, int pblocks) {
@@ -869,7 +876,7 @@ __global__ void k_mem_save(DevState S, const int* gate, int back) {
     if (!remembered(S, memEvaluation(m, at, T()), now + 1)) continue;
     T v[9];
     memLoad(m, at, v, true);
-    const int s = histInsert(S.hist, key, 0);
+    const int s = histInsert(S.hist, key);
     if (s < 0) { raise(S.status, kErrHashFull); continue; }
     T* d = static_cast<T*>(S.hist.vals) + 9 * (size_t)s;
 #pragma unroll
@@ -905,7 +912,7 @@ __global__ void k_mem_load(DevState S, const int* gate) {
     long long at;
     unsigned long long key;
     memEntry(S, np, i, m, at, key);
-    const int s = histFind(S.hist, key, 0);
+    const int s = histFind(S.hist, key);
     if (s < 0) { memForget(m, at, T()); continue; }
     const T* d = static_cast<const T*>(S.hist.vals) + 9 * (size_t)s;
     T v[9];
@@ -938,7 +945,7 @@ __global__ void k_mem_zero_cumulative(DevState S) {
   }
   if (S.prune) return;
   for (long long i = i0; i < (1ll << S.hist.log2cap); i += stride) {
-    if (tagOf(S.hist.keys[i]) != 0) continue;
+    if (S.hist.keys[i] == kEmptyKey) continue;
     V* v = static_cast<V*>(S.hist.vals) + 9 * (size_t)i;
     v[0] = v[1] = v[2] = v[6] = v[7] = v[8] = 0;
   }
@@ -1105,7 +1112,7 @@ __global__ void k_pair_counts(DevState S, unsigned long long* out) {
   unsigned long long e = 0, c = 0;
   if (i < S.n) e = (unsigned long long)S.npairs[i];
   const long long cap = 1ll << S.hist.log2cap;
-  for (long long k = i; k < cap; k += gridDim.x * blockDim.x) c += tagOf(S.hist.keys[k]) == 0;
+  for (long long k = i; k < cap; k += gridDim.x * blockDim.x) c += S.hist.keys[k] != kEmptyKey;
   for (int o = 16; o > 0; o >>= 1) {
     e += __shfl_down_sync(0xffffffffu, e, o);
     c += __shfl_down_sync(0xffffffffu, c, o);

@@ -1,8 +1,9 @@
 """The wall list and the contact memory beside the lists at sizes where their
 allocations and launches change: a packed slab two layers high, whose spheres
 all touch a wall and their neighbours, just below and above the particle count
-up to which the wall list has room for everybody (16,384; above, the list has
-to grow before the first step), one evaluation per warp lane and several.
+up to which the wall list starts with two slots per particle (16,384; above, a
+slot per two particles, so that it has to grow before or, started from forces,
+at the first evaluation), one evaluation per warp lane and several.
 
 Against the CPU FP64 restatement over three steps (the memory of the first is
 used by the next two), started by the leapfrog start and from uploaded forces
