@@ -48,7 +48,7 @@ typedef struct gdem_system* gdem_handle;
 #define GDEM_ST_HASH_FULL 0x08        /* contact-history table full */
 #define GDEM_ST_GJK_MAXITER 0x10      /* GJK iteration cap reached */
 #define GDEM_ST_TIMEOUT 0x20          /* a bounded device wait gave up */
-#define GDEM_ST_PAIRS_FULL 0x40       /* the pair list's allocation was too small at a rebuild (rows emptied; grown before the next call) */
+#define GDEM_ST_PAIRS_FULL 0x40       /* a particle has more than 65,535 partners within the skin (the others are left out) */
 
 /* Builds a system from a Grains3D XML input (Construction: LinkedCell,
  * Origin, Periodicity, Particles, Obstacles, ContactForceModels; Forces:

@@ -92,7 +92,7 @@ __global__ void __launch_bounds__(256) k_pairs_fill64(DevState S, const int* gat
   const bool valid = t < S.n && rowFits(S, t);
   const int nu = valid ? listPairs64<true>(S, t) : 0;
   // each pair once, from its lower ID, into the compact list of the filter
-  appendUpperPairs(S, t, valid ? S.pairs + S.pair_off[t] : S.pairs, nu, S.status);
+  appendUpperPairs(S, t, valid ? S.pairs + S.pair_off[t] : S.pairs, nu);
 }
 
 // One pair in the canonical orientation -- p0 (slot s0, the lower ID) at its

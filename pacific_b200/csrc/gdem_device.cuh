@@ -482,22 +482,20 @@ __device__ __forceinline__ int rowLength(DevState const& S, int cnt) {
   return cnt;
 }
 // Whether slot t's row, placed by the scan of the row lengths, lies inside
-// the allocation of the pair list; a row that does not is emptied (its
-// particle then sees no partner) and kErrPairsFull raised -- the host grows
-// the allocation before the next call.
+// the allocation of the pair list; with one that does not the evaluation is
+// put off until the host has enlarged it.
 __device__ __forceinline__ bool rowFits(DevState const& S, int t) {
   const int off = S.pair_off[t];   // negative when the scan's total overflowed
   if (off >= 0 && (long long)off + S.npairs[t] <= (long long)S.pair_cap) return true;
   S.npairs[t] = 0;
-  raise(S.status, kErrPairsFull);
+  S.ctl[kCtlNeed] = kPutOff;
   return false;
 }
 
 // Appends the first nu entries of slot t's row (seg) to the compact pair
 // list (one atomic per warp), with each entry's position in the row.  Every
 // lane of the warp calls it; valid lanes only contribute.
-__device__ __forceinline__ void appendUpperPairs(DevState const& S, int t, const int* seg, int nu,
-                                                 int* status) {
+__device__ __forceinline__ void appendUpperPairs(DevState const& S, int t, const int* seg, int nu) {
   const unsigned full = 0xffffffffu;
   const int lane = threadIdx.x & 31;
   int incl = nu;
@@ -513,7 +511,7 @@ __device__ __forceinline__ void appendUpperPairs(DevState const& S, int t, const
   base = __shfl_sync(full, base, 31);
   const long long cap = (long long)S.pair_cap / 2 + 1;
   if (base + (long long)total > cap) {
-    if (lane == 0) raise(status, kErrPairsFull);
+    if (lane == 0) S.ctl[kCtlNeed] = kPutOff;
     return;
   }
   const int first = base + incl - nu;

@@ -1020,7 +1020,7 @@ struct System {
   // rebuild needed since the last check exceed 80 % of the allocation, to 1.5
   // times that need; the next evaluation rebuilds.  Synchronises the stream.
   // Returns how many of the evaluations launched so far were put off, because
-  // the wall list had no room for a rebuild: they have to be launched again.
+  // a list had no room for a rebuild: they have to be launched again.
   int checkCapacity() {
     int ctl[kCtlWords];
     CK(cudaStreamSynchronize(stream));
@@ -1038,10 +1038,14 @@ struct System {
     CK(cudaStreamSynchronize(stream));
     const int hwm = ctl[kCtlEntriesMax];
     const int slots = std::max(ctl[kCtlWallSlotsMax], ctl[kCtlWallSlots]);
-    if ((double)hwm > 0.8 * (double)S.pair_cap)
+    const bool pairs = (double)hwm > 0.8 * (double)S.pair_cap;
+    const bool walls = S.any_walls && (double)slots > 0.8 * (double)S.wall_cap;
+    if (off) started = false;   // (in the middle of a step, should there be no memory)
+    if (off && !pairs && !walls) throw std::runtime_error("a contact list has no room, but asks for none");
+    if (pairs)
       allocatePairs(std::max((long long)(1.5 * (double)hwm) + 4096, (long long)S.pair_cap));
-    if (S.any_walls && (double)slots > 0.8 * (double)S.wall_cap)
-      allocateWalls((long long)(1.5 * (double)slots) + 4096);
+    if (walls) allocateWalls((long long)(1.5 * (double)slots) + 4096);
+    if (off) started = true;
     return off;
   }
   // The contact memory of the last evaluation from the lists into its table
@@ -1265,8 +1269,7 @@ struct System {
           ++k;
         }
         // the lists' allocations are checked every kCapacityCheck steps
-        // within a call (and at its end); the pair list grows before it can
-        // run short
+        // within a call (and at its end)
         if (k < nsteps && k % kCapacityCheck == 0) k -= checkCapacity();
       }
       CK(cudaEventRecord(ev1, stream));

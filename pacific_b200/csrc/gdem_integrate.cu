@@ -448,11 +448,12 @@ __global__ void __launch_bounds__(kMoveBlock<kFast, kBasis>(), kBasis ? 2 : (kFa
     k_move(DevState S, int flags) {
   int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= S.n) return;
+  const int need = S.ctl[kCtlNeed];
   TypeDesc const& tp = S.types[S.type[t]];
   MoveIn m;
   loadMoveIn<kFast, kBasis>(S, t, m);   // nothing the contact kernels write
   const bool sum = (flags & kStepSum) != 0;
-  if (sum && S.any_walls && S.ctl[kCtlNeed] == kPutOff) return;
+  if (sum && need == kPutOff) return;
   d3 F, T;
   bool candidate = false;
   if (sum) {
@@ -725,10 +726,10 @@ __global__ void __launch_bounds__(256, 8) k_filter(DevState S, int pblocks) {
 // Where each pair of the compact list sits in its partner's row: the entry of
 // the lower-ID slot t in the row of u (rows are symmetric: the pair search
 // decides both directions with the same expression).  0xFFFF when absent (a
-// row emptied for lack of room).  Grid-stride over the pairs, whose count is
-// known on the device only.
+// row cut off at kRowMax).  Grid-stride over the pairs, whose count is known on
+// the device only; not where the list is incomplete for lack of room.
 __global__ void __launch_bounds__(256) k_link(DevState S, const int* gate) {
-  if (gatedOff(gate)) return;
+  if (gatedOff(gate) || S.ctl[kCtlNeed] == kPutOff) return;
   const int np = listedPairs(S);
   for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < np; k += gridDim.x * blockDim.x) {
     const int2 pr = S.upairs[k];
@@ -885,8 +886,8 @@ __global__ void k_mem_save(DevState S, const int* gate, int back) {
 }
 
 // The table's memory into the new lists, as left by the last evaluation; from
-// here on the lists hold it.  The last kernel of a rebuild: where the wall list
-// ran short it puts the evaluation off instead (kPutOff).
+// here on the lists hold it.  The last kernel of a rebuild: where a list ran
+// short it puts the evaluation off instead (kPutOff).
 template <typename T>
 __global__ void k_mem_load(DevState S, const int* gate) {
   if (gatedOff(gate)) return;

@@ -22,7 +22,7 @@ enum StatusBits : int {
   kErrHashFull = 1 << 3,         // the contact-memory table has no free slot
   kErrGjkMaxIter = 1 << 4,       // GJK hit its iteration cap
   kErrTimeout = 1 << 5,          // a bounded device wait gave up
-  kErrPairsFull = 1 << 6,        // the pair list outgrew its allocation (or a row kRowMax)
+  kErrPairsFull = 1 << 6,        // a row of the pair list outgrew kRowMax
 };
 
 // Words of the device control block (DevState::ctl).
@@ -45,10 +45,11 @@ enum CtlWords : int {
   kCtlWords = 16
 };
 // Value of kCtlNeed where an evaluation is put off: its rebuild found more
-// (particle, wall) pairs than the wall list has room for.  That evaluation and
-// those after it (whose rebuilds find the same) leave the state as it is: the
-// lists are empty, the leapfrog moves nothing.  They are not counted; the host
-// makes them once it has enlarged the list, so no wall contact is left out.
+// pairs than the pair list, or more (particle, wall) pairs than the wall list,
+// has room for.  That evaluation and those after it (whose rebuilds find the
+// same) leave the state as it is: the lists are empty, the leapfrog moves
+// nothing.  They are not counted; the host makes them once it has enlarged the
+// list, so no contact is left out.
 constexpr int kPutOff = 2;
 
 // Whether contact memory that evaluation e wrote last (kNeverWritten: none) is
