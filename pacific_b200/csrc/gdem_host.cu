@@ -672,20 +672,24 @@ struct System {
   // arrays have an allocation of their own).  What costs time is memory mapped
   // anew, 0.31 ms to take and 0.26 ms to give back per 2 MB piece or larger
   // allocation; requests of at most 1 MB come out of pieces that are mapped
-  // already.  A system has some 50 arrays of about 5 KB per particle in all.
-  // Up to 4 MB of them go into blocks of 256 KB, with next to nothing mapped
-  // (200 spheres, FP64: upload 0.54 -> 0.16 ms, close 0.85 -> 0.55), above
-  // that into one block for them all (1,000 spheres: upload 0.95 -> 0.50 ms,
-  // close 1.23 -> 0.81), above 64 MB into blocks of that size (60,000: upload
-  // 2.0 ms, 10 with an allocation per array).
+  // already.  A system has some 50 arrays of about 5 KB per particle in all,
+  // half of that where the lists are on their own.  Up to 4 MB of them go into
+  // blocks of 256 KB, with next to nothing mapped (200 spheres, FP64: upload
+  // 0.54 -> 0.16 ms, close 0.85 -> 0.55), above that into one block for them
+  // all (1,000 spheres: upload 0.95 -> 0.50 ms, close 1.23 -> 0.81), above 128
+  // MB into blocks of that size (60,000: upload 2.0 ms, 10 with an allocation
+  // per array).  Where a state about fills the L2, how it lies in memory shows:
+  // a gas of 256,000 FP64 spheres takes 44.7 us a step with blocks of 64 MB,
+  // 42.9 to 43.6 with 96 to 512; beds and pours differ by less than 1 %.
   template <typename T>
   T* alloc(size_t n) {
     const size_t bytes = n * sizeof(T);
     if (bytes > (size_t(32) << 20)) return allocOwn<T>(n);
-    const size_t all = (size_t)S.cap * 5120 + (size_t(512) << 10);
+    const size_t all =
+        (size_t)S.cap * (S.cap <= kSmallSystem ? 5120 : 2560) + (size_t(512) << 10);
     const size_t block = all <= (size_t(4) << 20)
                              ? size_t(256) << 10
-                             : std::min(size_t(64) << 20, std::max(all, memory.sharedTotal()));
+                             : std::min(size_t(128) << 20, std::max(all, memory.sharedTotal()));
     return taken<T>(memory.shared(bytes, block));
   }
   void invalidateGraphs() {
