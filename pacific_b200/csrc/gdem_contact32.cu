@@ -690,10 +690,10 @@ __global__ void __launch_bounds__(128) k_pairsep32(DevState S) {
 }
 
 // The pair kernel of an evaluation, one thread per item over a persistent
-// grid: first the pairs the contact filter kept, then the particles near a
-// wall.  Its trigger comes after its wait, so the leapfrog kernel, which
+// grid: first the pairs the contact filter kept, then the wall items.  Its
+// trigger comes after its wait, so the leapfrog kernel, which
 // starts at the trigger, sees the filter's candidate marks complete.
-// What bounds the sphere kernel is latency: about 1,350 instructions per
+// What bounds the sphere kernel is latency: about 1,470 instructions per
 // contact in chains of divisions and square roots at 10 to 12 warps per
 // multiprocessor (issue slots 23 % busy, DRAM 5 % on a packed bed).  With the
 // memory in the pair list instead of a hash table and the wall slots as items
@@ -706,7 +706,7 @@ __global__ void __launch_bounds__(128, kConvex ? 1 : 3) k_pairlaw32(DevState S) 
   pdlTrigger();   // the leapfrog kernel may start; its candidates wait for this kernel
   // the pairs in contact at the last evaluation (all kept pairs, without
   // non-spherical classes), then those k_pairsep32 left undecided, then the
-  // particles near a wall
+  // wall items
   const int nh = S.ctl[kCtlKept], n2 = kConvex ? S.ctl[kCtlKept2] : 0, nw = S.ctl[kCtlWork];
   const int nk = nh + n2;
   const int tag = S.ctl[kCtlEpoch];

@@ -362,14 +362,14 @@ __device__ __forceinline__ void pairItem64(DevState const& S, int c, int tag, Gj
 }
 
 // The pair kernel of an evaluation, one thread per item over a persistent
-// grid: first the pairs the contact filter kept, then the particles near a
-// wall.  Its trigger comes after its wait, so the leapfrog kernel, which
+// grid: first the pairs the contact filter kept, then the wall items.  Its
+// trigger comes after its wait, so the leapfrog kernel, which
 // starts at the trigger, sees the filter's candidate marks complete.
-// The sphere kernel is bound by latency like the FP32-split one; four blocks
-// per multiprocessor (128 registers, some spilled) beat two and three where
-// there is work for them: packed beds of 60,000 and 250,000 spheres 39.6 and
-// 120.8 us, with three 40.5 and 126.6, with two 37.2 and 159.9 (before: 79.8
-// and 307.7, with the memory in a hash table and a particle's walls in turn).
+// The sphere kernel is bound by latency like the FP32-split one.  Four blocks
+// per multiprocessor (128 registers, some spilled), for the large beds: 250,000
+// packed spheres 120.8 us, with three 126.6, with two 159.9; 60,000 39.6, 40.5
+// and 37.2 (before: 307.7 and 79.8, with the memory in a hash table and a
+// particle's walls in turn).
 template <bool kConvex>
 __global__ void __launch_bounds__(128, kConvex ? 1 : 4) k_pairlaw64(DevState S) {
   pdlWait();      // the contact filter's lists
