@@ -121,3 +121,18 @@ def test_spheres_inserted_on_the_floor(tmp_path, lib, precision):
     assert len(F) == keep + 6000
     assert (F[keep:, 2] > 0.0).all() and (F[:keep, 2] <= 0.0).all()
     g.close()
+
+
+@pytest.mark.parametrize("precision", [FP64, FP32_SPLIT], ids=["fp64", "fp32split"])
+def test_convex_layer_lands_within_a_call(tmp_path, lib, precision):
+    """17,161 cubes, tetrahedra and cylinders (walls of a particle in turn, support
+    vertices carried on) thrown onto the floor."""
+    tet = scenarios.write_tetrahedron(tmp_path / "tet.insert")
+    sc = scenarios.convex_pour(n=131 * 131, seed=4, poly_path=tet, box=(0.4915, 0.4915, 0.02),
+                               cylinders=True)
+    sc.x[:, 2] += 0.6e-3                                # out of the floor's reach
+    sc.v[:, 2] = -5.0
+    xml = str(sc.write_xml(tmp_path / "convex.xml"))
+    got = _run(xml, sc, precision, (110,))
+    assert (got[1]["partner"] == -6).sum() > 1000
+    _same(got, _run(xml, sc, precision, (110,), room=4 * sc.n))
