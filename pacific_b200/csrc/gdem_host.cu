@@ -939,6 +939,11 @@ struct System {
     CK(cudaDeviceSynchronize());
   }
 
+  // The next evaluation rebuilds the lists.
+  void askRebuild() {
+    static const int one = 1;
+    if (S.ctl) CK(cudaMemcpyAsync(S.ctl + kCtlNeed, &one, sizeof(int), cudaMemcpyHostToDevice, stream));
+  }
   // The arrays sized by the pair list's entries: the rows, the compact pair
   // list with the pairs' positions in their rows, the contact filter's kept
   // list, the shares (tag words all ones: no evaluation's tag) and, when on,
@@ -948,10 +953,17 @@ struct System {
     if (entries > (long long)INT_MAX - 64)
       throw std::runtime_error("pair list too large for 32-bit row offsets");
     saveMemory(true);
+    askRebuild();
+    invalidateGraphs();
     for (void* p : {S.share, (void*)S.pair_delta, (void*)S.pair_force})
       if (p) freeAlloc(p);
+    // (no room at all until there is new memory: should there be none, the
+    // next evaluation is put off)
+    S.share = nullptr;
+    S.pair_delta = S.pair_force = nullptr;
+    S.pair_cap = 0;
+    S.pmem = MemView{nullptr, 0};
     const size_t e = (size_t)entries, pc = e / 2 + 1;
-    S.pair_cap = (int)entries;
     const size_t mb = precision == GDEM_FP64 ? kMemBytes64 : kMemBytes32;
     const size_t sb = precision == GDEM_FP64 ? 64 : 32;
     // the cold pairs' first pass (FP32-split, non-spherical classes)
@@ -969,6 +981,11 @@ struct System {
     // (a small system's first lists come out of a shared block; they are few
     // MB, so they may stay there when the lists outgrow them)
     char* base = kSmallSystem >= S.cap && !S.upairs ? alloc<char>(at) : allocOwn<char>(at);
+    if (S.wall_delta) {
+      S.pair_delta = allocOwn<double>(e);
+      S.pair_force = allocOwn<double>(3 * e);
+    }
+    S.pair_cap = (int)entries;
     S.share = base + o_share;
     S.pmem = MemView{base + o_mem, (long long)pc};
     S.pairs = reinterpret_cast<int*>(base + o_pairs);
@@ -979,17 +996,7 @@ struct System {
     // (on the library's stream, which does not synchronise with the legacy
     // default stream)
     CK(cudaMemsetAsync(S.share, 0xFF, e * sb, stream));
-    if (S.wall_delta) {
-      S.pair_delta = allocOwn<double>(e);
-      S.pair_force = allocOwn<double>(3 * e);
-    } else {
-      S.pair_delta = nullptr;
-      S.pair_force = nullptr;
-    }
-    static const int one = 1;
-    if (S.ctl) CK(cudaMemcpyAsync(S.ctl + kCtlNeed, &one, sizeof(int), cudaMemcpyHostToDevice, stream));
     CK(cudaStreamSynchronize(stream));
-    invalidateGraphs();
   }
   // The arrays sized by the wall list's slots (rebuilt before the next
   // evaluation): the list, the evaluation's wall items, the slots' memory and
@@ -998,6 +1005,8 @@ struct System {
     if (slots > (long long)INT_MAX - 64)
       throw std::runtime_error("wall list too large for 32-bit slots");
     saveMemory(true);
+    askRebuild();
+    invalidateGraphs();
     if (S.wshare) freeAlloc(S.wshare);
     S.wshare = nullptr;
     S.wall_cap = 0;
@@ -1015,10 +1024,7 @@ struct System {
     S.work = reinterpret_cast<int*>(p + sb + mb);
     S.wlist = reinterpret_cast<int2*>(p + sb + mb + wb);
     CK(cudaMemsetAsync(S.wshare, 0xFF, sb, stream));
-    static const int one = 1;
-    if (S.ctl) CK(cudaMemcpyAsync(S.ctl + kCtlNeed, &one, sizeof(int), cudaMemcpyHostToDevice, stream));
     CK(cudaStreamSynchronize(stream));
-    invalidateGraphs();
   }
   // Grows the pair list (the wall list) when the most entries (slots) a
   // rebuild needed since the last check exceed 80 % of the allocation, to 1.5
@@ -1033,11 +1039,10 @@ struct System {
     CK(cudaMemsetAsync(S.ctl + kCtlWallSlotsMax, 0, sizeof(int), stream));
     int off = 0;
     if (ctl[kCtlNeed] == kPutOff) {
-      static const int one = 1;
       off = (int)((unsigned)epoch - (unsigned)ctl[kCtlEpoch]);
       epoch -= off;
       lists_hold = false;   // (the rebuild left the memory in the table)
-      CK(cudaMemcpyAsync(S.ctl + kCtlNeed, &one, sizeof(int), cudaMemcpyHostToDevice, stream));
+      askRebuild();
     }
     CK(cudaStreamSynchronize(stream));
     const int hwm = ctl[kCtlEntriesMax];
