@@ -24,10 +24,13 @@
 //   k_pairs_*   (gdem_contact64/32.cu) the rows of the skin pair list:
 //               counted, placed by a scan of the counts, written; k_link
 //               then records where each pair of the compact list sits in
-//               its partner's row.
+//               its partner's row, and k_wall_rows lists the (particle, wall)
+//               pairs within the skin.
+//   k_mem_*     the contact memory from the old lists through its table into
+//               the new ones.
 //   k_filter    lists the pairs of the skin list whose bounding spheres
-//               overlap now, and the particles near a wall, and marks them
-//               as candidates; the pair kernel (gdem_contact64/32.cu)
+//               overlap now, and the wall-list slots that are near, and marks
+//               their particles as candidates; the pair kernel (gdem_contact64/32.cu)
 //               evaluates them exactly and writes each contact's two shares
 //               into the partners' rows.
 //   k_move      the leapfrog of each particle in place: its force and torque
